@@ -17,7 +17,7 @@
 //        - dX/dt written once; each block stores its max |dX/dt| in its
 //          own slot (plain store).
 //      Variants (autotuned, all computing the same values): tile shapes,
-//      a split form (k_chem64 writes mu/M once per point, the tile kernel
+//      a split form (k_chem writes mu/M once per point, the tile kernel
 //      reads them back), table-cell sort, shared table window, per-point
 //      faces.
 //   5. k_dt_finish (one block): max over the slots, the adaptive dt rule,
@@ -39,6 +39,7 @@
 #include "pf5d_device.cuh"
 #include "pf5d_fft.h"
 #include "pf5d_fp32c.h"
+#include "pf5d_gather.cuh"
 #include "pf5d_tiles.cuh"
 #include "pf5d_window.cuh"
 #include "pf5d_diag.cuh"
@@ -95,14 +96,6 @@ __device__ __forceinline__ void chem_point(const RateParams &P, const double x[S
 constexpr int kWin64 = 3;                       // window nodes per axis (2 cells)
 constexpr int kWinNodes64 = kWin64 * kWin64 * kWin64 * kWin64;
 constexpr int kNodeV64 = 5;                     // double2 per 10-double table node
-
-// Table cell of x exactly as the reference computes it (interpolation.py:103-121).
-__device__ __forceinline__ bool cell64(const Table &T, const double x[S], int ii[S], double tt[S]) {
-  if (!linear_region(T, x)) return false;
-#pragma unroll
-  for (int a = 0; a < S; ++a) axis_coord(x[a] * T.inv_step, T.n, ii[a], tt[a]);
-  return true;
-}
 
 // The 16-corner sum of interp_linear<true> from node-strided double2 data
 // (global table or shared window); identical arithmetic and order.
@@ -354,7 +347,7 @@ __device__ __forceinline__ void mu_plane64(const RateParams &P, const double *Xm
 }
 
 // mu/M of one plane (tile + 1-cell halo, or tile only) read from the split
-// buffer P.mm (written by k_chem64) into dst, in mu_plane64's layout.
+// buffer P.mm (written by k_chem) into dst, in mu_plane64's layout.
 template <int TX, int TY, int NTH = TX * TY>
 __device__ __forceinline__ void load_mu_plane(const RateParams &P, int64_t zoff, const int *wx,
                                               const int *wy, bool interior_only, double *dst,
@@ -371,448 +364,116 @@ __device__ __forceinline__ void load_mu_plane(const RateParams &P, int64_t zoff,
 }
 
 // Split rate evaluation, first kernel: chemical potential and mobility at
-// every point of a 2D/3D field into P.mm, one point per thread, a 32 x 8
-// tile of a plane per block.  Same arithmetic as mu_plane64: Laplacian
-// neighbour order (operators.py:49-76) +axis0, -axis0, +axis1, -axis1
-// (, +axis2, -axis2), then mu = v - lap*kappa (+ s' * l).
+// every point of a field into P.mm (SoA rows), each point once.  The table
+// values come first (pf5d_gather.cuh), then each thread takes its own points
+// in order: Laplacian (operators.py:49-76: +axis0, -axis0, +axis1, ...), then
+// mu = v - lap*kappa (+ s' * l).  A block's points are 512 in a row (1D), 32
+// columns by 16 rows (2D), or 32 columns by 4 rows by 4 planes (3D), and a
+// thread's four are consecutive along y (2D) or z (3D), so it loads each point
+// of that axis once.
 //
-// Before interpolating, the block orders its points by table cell
-// (counting sort on cell_hash), so the lanes of a warp gather the same
-// table nodes: a warp-wide corner load then touches one or two cache lines
-// instead of one per lane.  Every point is evaluated exactly once (no halo)
-// and the order only changes which thread evaluates a point.
-template <int DIM, bool VEC, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_chem64(RateParams P) {
-  constexpr int NT = 256;
-  __shared__ double io[2 * S + 1][NT];   // inputs of each point: x, lap, s'
-  __shared__ int hist[NT];
-  __shared__ int wsum[NT / 32 + 1];
-  __shared__ unsigned short order[NT];
-  pdl_wait();
-  if (P.st->halt) return;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  const int x = blockIdx.x * 32 + threadIdx.x;
-  const int y = blockIdx.y * 8 + threadIdx.y;
-  const int z = blockIdx.z;
-  const bool valid = x < P.nx && y < P.ny;
-  const int64_t plane = (int64_t)P.ny * P.nx;
-  const int64_t zo = (int64_t)z * plane;
-  const int64_t g = zo + (int64_t)y * P.nx + x;
-  hist[tid] = 0;
-  int key = 0, rank = 0;
-  __syncthreads();
-  if (valid) {
-    auto ld = [&](int64_t gi, double v[S]) {
-      const double2 a = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi));
-      const double2 b = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi) + 1);
-      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-    };
-    const int xp = x + 1 == P.nx ? 0 : x + 1, xm = x == 0 ? P.nx - 1 : x - 1;
-    const int yp = y + 1 == P.ny ? 0 : y + 1, ym = y == 0 ? P.ny - 1 : y - 1;
-    double xc[S], lap[S], n0[S], n1[S];
-    ld(g, xc);
-    if (DIM == 1) {
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = 0.0;
-    } else if (DIM == 3) {
-      const int zp = z + 1 == P.nz ? 0 : z + 1, zm = z == 0 ? P.nz - 1 : z - 1;
-      ld((int64_t)zp * plane + (int64_t)y * P.nx + x, n0);
-      ld((int64_t)zm * plane + (int64_t)y * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = n0[c] + n1[c];
-      ld(zo + (int64_t)yp * P.nx + x, n0);
-      ld(zo + (int64_t)ym * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = (lap[c] + n0[c]) + n1[c];
-    } else {
-      ld(zo + (int64_t)yp * P.nx + x, n0);
-      ld(zo + (int64_t)ym * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = n0[c] + n1[c];
-    }
-    ld(zo + (int64_t)y * P.nx + xp, n0);
-    ld(zo + (int64_t)y * P.nx + xm, n1);
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      if (DIM == 1)
-        lap[c] = ((n0[c] + n1[c]) - 2.0 * xc[c]) * P.inv_dx2;
-      else
-        lap[c] = (((lap[c] + n0[c]) + n1[c]) - (DIM == 3 ? 6.0 : 4.0) * xc[c]) * P.inv_dx2;
-      io[c][tid] = xc[c];
-      io[S + c][tid] = lap[c];
-    }
-    io[2 * S][tid] = P.sp ? __ldg(P.sp + g) : 0.0;
-    key = cell_hash(xc, (float)P.T.inv_step);
-    rank = atomicAdd(&hist[key], 1);
-  }
-  __syncthreads();
-  const int count = block_exclusive_scan<NT, NT>(hist, wsum, tid);
-  if (valid) order[hist[key] + rank] = (unsigned short)tid;
-  __syncthreads();
-  unsigned flags = 0;
-  double v[NP];
-  if (tid < count) {
-    const int q = order[tid];
-    double xq[S], lq[S];
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      xq[c] = io[c][q];
-      lq[c] = io[S + c][q];
-    }
-    const double spv = io[2 * S][q];
-    const int o[S] = {0, 0, 0, 0};
-    interp_win64<VEC>(P.T, xq, nullptr, o, v, &flags);
-    // point q of the tile: row q / 32, column q % 32
-    const int64_t gq = zo + (int64_t)(blockIdx.y * 8 + (q >> 5)) * P.nx + blockIdx.x * 32 + (q & 31);
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      const double lk = lq[c] * P.kappa.v[c];
-      double m = v[c] - lk;
-      if (P.sp) m = m + spv * P.lvec.v[c];
-      P.mm[c * P.npts + gq] = m;
-    }
-#pragma unroll
-    for (int c = 0; c < NM; ++c) P.mm[(S + c) * P.npts + gq] = v[S + c];
-  }
-  raise_rate_flags(P.st, flags);
-}
+// Bound by the L1 data path (67% of its wavefronts' rate at 128x256x256, FP64
+// pipe 38%).  One point per thread (1.21 ms at 256^3, on-node composition)
+// moved every node into registers once per point; with K = 3 points of a cell
+// per load it is 0.99 ms.  K = 4 needs 168 registers, and the 12 warps per SM
+// that leaves lose more (1.18) than the fewer loads give; K = 2 with the same
+// 16 warps is 1.01.  512 points per block keep a cell's run longer than K in
+// fields that spread over many cells: with 256 points 1.05, 1.24 against 1.05
+// ms in a field of two phases.
+constexpr int kChemNT = 128, kChemPer = 4, kChemK = 3, kChemMinB = 4;
+using ChemSmem = GatherSmem<kChemNT, kChemPer, kChemK>;
 
-// Split rate evaluation, first kernel, staged form (VEC tables, 2D/3D): the
-// values of k_chem64 bit for bit, with each thread's results put back in
-// the shared input rows at its point's tile position, so the mu/M rows of
-// P.mm are written in tile order (coalesced) rather than in the table-cell
-// order the gathers run in.
-template <int DIM, int MINB>
-__global__ void __launch_bounds__(256, MINB) k_chem64s(RateParams P) {
-  constexpr int NT = 256;
-  static_assert(DIM >= 2, "plane tiles");
-  __shared__ double io[2 * S + 1][NT];   // inputs of each point (x, lap, s'), then its mu/M
-  __shared__ int hist[NT];
-  __shared__ int wsum[NT / 32 + 1];
-  __shared__ unsigned short order[NT];
-  pdl_wait();
-  if (P.st->halt) return;
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  const int x = blockIdx.x * 32 + threadIdx.x;
-  const int y = blockIdx.y * 8 + threadIdx.y;
-  const int z = blockIdx.z;
-  const bool valid = x < P.nx && y < P.ny;
-  const int64_t plane = (int64_t)P.ny * P.nx;
-  const int64_t zo = (int64_t)z * plane;
-  const int64_t g = zo + (int64_t)y * P.nx + x;
-  hist[tid] = 0;
-  int key = 0, rank = 0;
-  __syncthreads();
-  if (valid) {
-    auto ld = [&](int64_t gi, double v[S]) {
-      const double2 a = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi));
-      const double2 b = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi) + 1);
-      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-    };
-    const int xp = x + 1 == P.nx ? 0 : x + 1, xm = x == 0 ? P.nx - 1 : x - 1;
-    const int yp = y + 1 == P.ny ? 0 : y + 1, ym = y == 0 ? P.ny - 1 : y - 1;
-    double xc[S], lap[S], n0[S], n1[S];
-    ld(g, xc);
-    if (DIM == 3) {
-      const int zp = z + 1 == P.nz ? 0 : z + 1, zm = z == 0 ? P.nz - 1 : z - 1;
-      ld((int64_t)zp * plane + (int64_t)y * P.nx + x, n0);
-      ld((int64_t)zm * plane + (int64_t)y * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = n0[c] + n1[c];
-      ld(zo + (int64_t)yp * P.nx + x, n0);
-      ld(zo + (int64_t)ym * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = (lap[c] + n0[c]) + n1[c];
-    } else {
-      ld(zo + (int64_t)yp * P.nx + x, n0);
-      ld(zo + (int64_t)ym * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = n0[c] + n1[c];
-    }
-    ld(zo + (int64_t)y * P.nx + xp, n0);
-    ld(zo + (int64_t)y * P.nx + xm, n1);
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      lap[c] = (((lap[c] + n0[c]) + n1[c]) - (DIM == 3 ? 6.0 : 4.0) * xc[c]) * P.inv_dx2;
-      io[c][tid] = xc[c];
-      io[S + c][tid] = lap[c];
-    }
-    io[2 * S][tid] = P.sp ? __ldg(P.sp + g) : 0.0;
-    key = cell_hash(xc, (float)P.T.inv_step);
-    rank = atomicAdd(&hist[key], 1);
-  }
-  __syncthreads();
-  const int count = block_exclusive_scan<NT, NT>(hist, wsum, tid);
-  if (valid) order[hist[key] + rank] = (unsigned short)tid;
-  __syncthreads();
-  unsigned flags = 0;
-  if (tid < count) {
-    const int q = order[tid];
-    double xq[S], lq[S], v[NP];
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      xq[c] = io[c][q];
-      lq[c] = io[S + c][q];
-    }
-    const double spv = io[2 * S][q];
-    const int o[S] = {0, 0, 0, 0};
-    interp_win64<true>(P.T, xq, nullptr, o, v, &flags);
-    // column q is this thread's alone: its inputs are read, now its results
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      const double lk = lq[c] * P.kappa.v[c];
-      double m = v[c] - lk;
-      if (P.sp) m = m + spv * P.lvec.v[c];
-      io[c][q] = m;
-    }
-#pragma unroll
-    for (int c = 0; c < NM; ++c) io[S + c][q] = v[S + c];
-  }
-  raise_rate_flags(P.st, flags);
-  __syncthreads();
-  if (valid) {
-#pragma unroll
-    for (int r = 0; r < NP; ++r) P.mm[r * P.npts + g] = io[r][tid];
-  }
-}
-
-// Split rate evaluation, first kernel, shared-gather form: the same values
-// as k_chem64 (bit for bit), with the table gathers of up to K points of one
-// table cell shared.  A block of 256 threads takes a brick of 256 K points
-// (32 x 8 x K in 3D, 32 x 8K in 2D, 256K in 1D):
-//   1. per point: x, the Laplacian (k_chem64's order) and s', the table
-//      cell (axis_coord of interpolation.py:110-121) or "nearest row";
-//   2. counting sort of the points by a hash of their cell (bin 255: points
-//      outside the linear region);
-//   3. each linear bin's run is cut into work items of up to K points;
-//   4. a thread evaluates an item: each corner node is loaded once and its
-//      term w * v accumulated into every point of the item, each point with
-//      its own weight ((w0 w1) w2) w3 and the reference's left-to-right
-//      16-term sum, so every value is the one k_chem64 computes.  Points
-//      whose cell differs from the item's first (hash collisions) are set
-//      aside;
-//   5. the points set aside and the nearest-row points, one per thread;
-//   6. coalesced stores of the SoA rows.
-constexpr int kChem64Threads = 256;
-// Doubles per point of k_chem64i's shared staging, point-major (80 bytes, so
-// a point's values move as 16-byte vectors without bank conflicts between
-// neighbouring points): x (4), lap (4), s' -- overwritten by mu (4), M (5).
-constexpr int kIo64 = 10;
-
-template <int DIM, int K>
-struct Chem64Geom {
-  static constexpr int NPB = kChem64Threads * K;
-  static constexpr int BX = DIM == 1 ? NPB : 32;
-  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? 8 * K : 8);
-  static constexpr int BZ = DIM == 3 ? K : 1;
-  static constexpr int NITEMS = NPB / K + 256;
-  // io[kIo64 * NPB] doubles (point-major), cell[NPB] int, items[NITEMS] u32,
-  // order/prank/left [NPB] u16, skey/pkey [NPB] u8, hist/cnt/ibase [256] int,
-  // wsum + nleft
-  static constexpr size_t smem = (size_t)10 * NPB * 8 + NPB * 4 + NITEMS * 4 + 3 * NPB * 2 +
-                                 2 * NPB + 3 * 256 * 4 + 16 * 4;
+template <int DIM>
+struct ChemTile {
+  static constexpr int BX = DIM == 1 ? kChemNT * kChemPer : 32;
+  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? kChemNT / 32 * kChemPer : kChemNT / 32);
+  static constexpr int BZ = DIM == 3 ? kChemPer : 1;
 };
 
-template <int DIM, bool VEC, int K, int MINB>
-__global__ void __launch_bounds__(kChem64Threads, MINB) k_chem64i(RateParams P) {
-  using G = Chem64Geom<DIM, K>;
-  constexpr int NT = kChem64Threads, NPB = G::NPB;
-  extern __shared__ double2 smd[];
-  double *io = reinterpret_cast<double *>(smd);             // kIo64 per point, point-major
-  int *cellv = reinterpret_cast<int *>(io + kIo64 * NPB);
-  unsigned *items = reinterpret_cast<unsigned *>(cellv + NPB);
-  unsigned short *order = reinterpret_cast<unsigned short *>(items + G::NITEMS);
-  unsigned short *prank = order + NPB;
-  unsigned short *left = prank + NPB;
-  unsigned char *skey = reinterpret_cast<unsigned char *>(left + NPB);
-  unsigned char *pkey = skey + NPB;
-  int *hist = reinterpret_cast<int *>(pkey + NPB);
-  int *cnt = hist + 256;
-  int *ibase = cnt + 256;
-  int *wsum = ibase + 256;
-  int *nleft = wsum + 12;
+template <int DIM, bool VEC>
+__global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
+  using G = ChemTile<DIM>;
+  constexpr int NT = kChemNT, PER = kChemPer;
+  __shared__ ChemSmem g;
   pdl_wait();
   if (P.st->halt) return;
-  const int tid = threadIdx.x;
-  const Table &T = P.T;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int bx = blockIdx.x * G::BX, by = blockIdx.y * G::BY, bz = blockIdx.z * G::BZ;
   const int64_t plane = (int64_t)P.ny * P.nx;
-  hist[tid] = 0;
-  if (tid == 0) *nleft = 0;
+  const bool wide = ((uintptr_t)P.X & 31) == 0;
+  // the point in slot q = j * NT + w * 32 + lane
+  auto px = [&](int j, int l, int v) { return DIM == 1 ? bx + j * NT + v * 32 + l : bx + l; };
+  auto py = [&](int j, int v) { return DIM == 1 ? 0 : (DIM == 2 ? by + PER * v + j : by + v); };
+  auto pz = [&](int j) { return DIM == 3 ? bz + j : 0; };
+  gather_begin(g, tid);
   __syncthreads();
-  // 1. per-point inputs
-#pragma unroll 1
-  for (int j = 0; j < K; ++j) {
-    const int q = tid + j * NT;
-    const int qx = q % G::BX, qy = (q / G::BX) % G::BY, qz = q / (G::BX * G::BY);
-    const int x = blockIdx.x * G::BX + qx, y = blockIdx.y * G::BY + qy, z = blockIdx.z * G::BZ + qz;
-    prank[q] = kNoRank;
-    if (x >= P.nx || y >= P.ny || z >= P.nz) continue;
-    const int64_t zo = (int64_t)z * plane, g = zo + (int64_t)y * P.nx + x;
-    auto ld = [&](int64_t gi, double v[S]) {
-      const double2 a = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi));
-      const double2 b = __ldg(reinterpret_cast<const double2 *>(P.X + 4 * gi) + 1);
-      v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
-    };
-    const int xp = x + 1 == P.nx ? 0 : x + 1, xm = x == 0 ? P.nx - 1 : x - 1;
-    double xc[S], lap[S], n0[S], n1[S];
-    ld(g, xc);
+  int kr[PER];
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    const int x = px(j, lane, w), y = py(j, w), z = pz(j);
+    const bool valid = x < P.nx && y < P.ny && z < P.nz;
+    double xc[S] = {0.0, 0.0, 0.0, 0.0};
+    if (valid) load_comp4(P.X + 4 * (z * plane + (int64_t)y * P.nx + x), wide, xc);
+    kr[j] = gather_add(g, P.T, valid, xc, j * NT + tid);
+  }
+  const int nitems = gather_sort(g, kr, tid);
+  gather_values<VEC>(g, P.T, nitems, tid);
+  unsigned flags = 0;
+  gather_rest<VEC>(g, P.T, tid, &flags, [&](int q, double x[S]) {
+    const int j = q / NT, v = (q / 32) % (NT / 32);
+    load_comp4(P.X + 4 * (pz(j) * plane + (int64_t)py(j, v) * P.nx + px(j, q & 31, v)), wide, x);
+  });
+  raise_rate_flags(P.st, flags);
+  if (kr[0] == kNoKey) return;                  // none of this thread's points is in the field
+  double below[S], xc[S], above[S];             // along the marching axis (y in 2D, z in 3D)
+  const int x0 = px(0, lane, w), y0 = py(0, w), z0 = pz(0);
+  auto at = [&](int z, int y, int x) { return P.X + 4 * (z * plane + (int64_t)y * P.nx + x); };
+  if (DIM == 2) load_comp4(at(0, y0 == 0 ? P.ny - 1 : y0 - 1, x0), wide, below);
+  if (DIM == 3) load_comp4(at(z0 == 0 ? P.nz - 1 : z0 - 1, y0, x0), wide, below);
+  load_comp4(at(z0, y0, x0), wide, xc);
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if (kr[j] == kNoKey) break;
+    const int x = px(j, lane, w), y = py(j, w), z = pz(j);
+    double lap[S], n0[S], n1[S];
+    if (DIM == 1) {
+      if (j > 0) load_comp4(at(0, 0, x), wide, xc);
+    } else {
+      const int yp = y + 1 == P.ny ? 0 : y + 1, zp = z + 1 == P.nz ? 0 : z + 1;
+      load_comp4(DIM == 2 ? at(0, yp, x) : at(zp, y, x), wide, above);
+#pragma unroll
+      for (int c = 0; c < S; ++c) lap[c] = above[c] + below[c];
+    }
     if (DIM == 3) {
-      const int zp = z + 1 == P.nz ? 0 : z + 1, zm = z == 0 ? P.nz - 1 : z - 1;
-      ld((int64_t)zp * plane + (int64_t)y * P.nx + x, n0);
-      ld((int64_t)zm * plane + (int64_t)y * P.nx + x, n1);
+      load_comp4(at(z, y + 1 == P.ny ? 0 : y + 1, x), wide, n0);
+      load_comp4(at(z, y == 0 ? P.ny - 1 : y - 1, x), wide, n1);
 #pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = n0[c] + n1[c];
+      for (int c = 0; c < S; ++c) lap[c] = (lap[c] + n0[c]) + n1[c];
     }
-    if (DIM >= 2) {
-      const int yp = y + 1 == P.ny ? 0 : y + 1, ym = y == 0 ? P.ny - 1 : y - 1;
-      ld(zo + (int64_t)yp * P.nx + x, n0);
-      ld(zo + (int64_t)ym * P.nx + x, n1);
-#pragma unroll
-      for (int c = 0; c < S; ++c) lap[c] = DIM == 3 ? (lap[c] + n0[c]) + n1[c] : n0[c] + n1[c];
-    }
-    ld(zo + (int64_t)y * P.nx + xp, n0);
-    ld(zo + (int64_t)y * P.nx + xm, n1);
+    load_comp4(at(z, y, x + 1 == P.nx ? 0 : x + 1), wide, n0);
+    load_comp4(at(z, y, x == 0 ? P.nx - 1 : x - 1), wide, n1);
+    const int64_t gi = z * plane + (int64_t)y * P.nx + x;
+    const double spv = P.sp ? __ldg(P.sp + gi) : 0.0;
+    double v[NP];
+    gather_get(g, j * NT + tid, v);
 #pragma unroll
     for (int c = 0; c < S; ++c) {
-      if (DIM == 1)
-        lap[c] = ((n0[c] + n1[c]) - 2.0 * xc[c]) * P.inv_dx2;
-      else
-        lap[c] = (((lap[c] + n0[c]) + n1[c]) - (DIM == 3 ? 6.0 : 4.0) * xc[c]) * P.inv_dx2;
-      io[q * kIo64 + c] = xc[c];
-      io[q * kIo64 + S + c] = lap[c];
-    }
-    io[q * kIo64 + 8] = P.sp ? __ldg(P.sp + g) : 0.0;
-    int ii[S];
-    double tt[S];
-    int cell = -1, key = 255;
-    if (cell64(T, xc, ii, tt)) {
-      cell = ((ii[0] * T.n + ii[1]) * T.n + ii[2]) * T.n + ii[3];
-      key = (int)((unsigned)(41 * ii[0] + 13 * ii[1] + 5 * ii[2] + ii[3]) % 255u);
-    }
-    cellv[q] = cell;
-    pkey[q] = (unsigned char)key;
-    prank[q] = (unsigned short)atomicAdd(&hist[key], 1);
-  }
-  __syncthreads();
-  // 2. counting sort by cell key
-  cnt[tid] = hist[tid];
-  const int nvalid = block_exclusive_scan<256, NT>(hist, wsum, tid);
-  for (int q = tid; q < NPB; q += NT) {
-    if (prank[q] == kNoRank) continue;
-    const int b = pkey[q], s = hist[b] + prank[q];
-    order[s] = (unsigned short)q;
-    skey[s] = (unsigned char)b;
-  }
-  // 3. work items of up to K points of one linear bin
-  ibase[tid] = tid == 255 ? 0 : (cnt[tid] + K - 1) / K;
-  const int nitems = block_exclusive_scan<256, NT>(ibase, wsum, tid);
-  const int lin_end = nvalid - cnt[255];
-  for (int s = tid; s < lin_end; s += NT) {
-    const int b = skey[s], r = s - hist[b];
-    if (r % K == 0) items[ibase[b] + r / K] = (unsigned)s | ((unsigned)min(K, cnt[b] - r) << 16);
-  }
-  __syncthreads();
-  // 4. the work items
-  const int64_t s3 = T.stride, s2 = (int64_t)T.n * s3, s1 = (int64_t)T.n * s2,
-                s0 = (int64_t)T.n * s1;
-  for (int it = tid; it < nitems; it += NT) {
-    const unsigned e = items[it];
-    const int s = (int)(e & 0xFFFFu), m = (int)(e >> 16);
-    int q[K];
-    bool use[K];
-    double tt[K][S], qq[K][S];
-    int cell0 = 0;
-#pragma unroll
-    for (int j = 0; j < K; ++j) {
-      q[j] = j < m ? (int)order[s + j] : 0;
-      const int cj = cellv[q[j]];
-      if (j == 0) cell0 = cj;
-      use[j] = j < m && cj == cell0;
-      if (j < m && !use[j]) left[atomicAdd(nleft, 1)] = (unsigned short)q[j];
-#pragma unroll
-      for (int a = 0; a < S; ++a) {
-        int i;
-        axis_coord(io[q[j] * kIo64 + a] * T.inv_step, T.n, i, tt[j][a]);
-        qq[j][a] = 1.0 - tt[j][a];
-      }
-    }
-    double acc[K][NP];
-    const double *base = T.grid + (int64_t)cell0 * s3;
-#pragma unroll
-    for (int c = 0; c < 16; ++c) {
-      const int b0 = (c >> 3) & 1, b1 = (c >> 2) & 1, b2 = (c >> 1) & 1, b3 = c & 1;
-      const double *node = base + b0 * s0 + b1 * s1 + b2 * s2 + b3 * s3;
-      double v[NP + 1];
-      if (VEC) {
-        const double2 *n2 = reinterpret_cast<const double2 *>(node);
-#pragma unroll
-        for (int k = 0; k < (NP + 1) / 2; ++k) {
-          const double2 a = __ldg(n2 + k);
-          v[2 * k] = a.x;
-          v[2 * k + 1] = a.y;
-        }
-      } else {
-#pragma unroll
-        for (int p = 0; p < NP; ++p) v[p] = __ldg(node + p);
-      }
-#pragma unroll
-      for (int j = 0; j < K; ++j) {
-        const double w = (b0 ? tt[j][0] : qq[j][0]) * (b1 ? tt[j][1] : qq[j][1]) *
-                         (b2 ? tt[j][2] : qq[j][2]) * (b3 ? tt[j][3] : qq[j][3]);
-#pragma unroll
-        for (int p = 0; p < NP; ++p) {
-          const double term = w * v[p];
-          acc[j][p] = (c == 0) ? term : acc[j][p] + term;
-        }
-      }
+      if (DIM == 1) lap[c] = ((n0[c] + n1[c]) - 2.0 * xc[c]) * P.inv_dx2;
+      else lap[c] = (((lap[c] + n0[c]) + n1[c]) - (DIM == 3 ? 6.0 : 4.0) * xc[c]) * P.inv_dx2;
+      const double lk = lap[c] * P.kappa.v[c];
+      double m = v[c] - lk;
+      if (P.sp) m = m + spv * P.lvec.v[c];
+      P.mm[c * P.npts + gi] = m;
     }
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      if (!use[j]) continue;
+    for (int c = 0; c < NM; ++c) P.mm[(S + c) * P.npts + gi] = v[S + c];
+    if (DIM != 1) {
 #pragma unroll
       for (int c = 0; c < S; ++c) {
-        const double lk = io[q[j] * kIo64 + S + c] * P.kappa.v[c];
-        double mu = acc[j][c] - lk;
-        if (P.sp) mu = mu + io[q[j] * kIo64 + 8] * P.lvec.v[c];
-        io[q[j] * kIo64 + c] = mu;
+        below[c] = xc[c];
+        xc[c] = above[c];
       }
-#pragma unroll
-      for (int c = 0; c < NM; ++c) io[q[j] * kIo64 + S + c] = acc[j][S + c];
     }
-  }
-  __syncthreads();
-  // 5. points set aside and points outside the linear region, one per thread
-  unsigned flags = 0;
-  const int nnn = cnt[255], nl = nnn + *nleft;
-  for (int l = tid; l < nl; l += NT) {
-    const int q = l < nnn ? (int)order[lin_end + l] : (int)left[l - nnn];
-    double xq[S], v[NP];
-#pragma unroll
-    for (int c = 0; c < S; ++c) xq[c] = io[q * kIo64 + c];
-    const int o[S] = {0, 0, 0, 0};
-    interp_win64<VEC>(T, xq, nullptr, o, v, &flags);
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      const double lk = io[q * kIo64 + S + c] * P.kappa.v[c];
-      double mu = v[c] - lk;
-      if (P.sp) mu = mu + io[q * kIo64 + 8] * P.lvec.v[c];
-      io[q * kIo64 + c] = mu;
-    }
-#pragma unroll
-    for (int c = 0; c < NM; ++c) io[q * kIo64 + S + c] = v[S + c];
-  }
-  raise_rate_flags(P.st, flags);
-  __syncthreads();
-  // 6. coalesced stores of the SoA rows
-#pragma unroll 1
-  for (int j = 0; j < K; ++j) {
-    const int q = tid + j * NT;
-    const int qx = q % G::BX, qy = (q / G::BX) % G::BY, qz = q / (G::BX * G::BY);
-    const int x = blockIdx.x * G::BX + qx, y = blockIdx.y * G::BY + qy, z = blockIdx.z * G::BZ + qz;
-    if (x >= P.nx || y >= P.ny || z >= P.nz) continue;
-    const int64_t g = (int64_t)z * plane + (int64_t)y * P.nx + x;
-#pragma unroll
-    for (int c = 0; c < NP; ++c) P.mm[c * P.npts + g] = io[q * kIo64 + c];
   }
 }
 
@@ -1072,8 +733,7 @@ struct March64Geom {
   static constexpr int NFMAX = G::NFX > G::NFY ? G::NFX : G::NFY;
 };
 
-template <int TX, int TY, int MINB, bool VEC, bool WIN, bool SPLIT = false, int SORT = 0,
-          bool PERPOINT = false>
+template <int TX, int TY, int MINB, bool VEC, bool WIN, int SORT = 0, bool PERPOINT = false>
 __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, int zc) {
   using G = PlaneGeom<TX, TY>;
   pdl_wait();
@@ -1113,36 +773,25 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
     load_plane<TX, TY>(P.X, (int64_t)wrap_any(z, P.nz) * plane, wx, wy, P.nx, xplane(z), tid);
   };
   auto compute_mu = [&](int z, bool interior_only) {
-    if constexpr (SPLIT)
-      load_mu_plane<TX, TY>(P, (int64_t)wrap_any(z, P.nz) * plane, wx, wy, interior_only,
-                            mplane(z), tid);
-    else
-      mu_plane64<TX, TY, 3, VEC, WIN, TX * TY, SORT>(P, xplane(z - 1), xplane(z), xplane(z + 1),
-                                                     mplane(z), (int64_t)wrap_any(z, P.nz) * plane,
-                                                     wx, wy, interior_only, win, win_lo, &flags,
-                                                     tid, ss);
+    mu_plane64<TX, TY, 3, VEC, WIN, TX * TY, SORT>(P, xplane(z - 1), xplane(z), xplane(z + 1),
+                                                   mplane(z), (int64_t)wrap_any(z, P.nz) * plane,
+                                                   wx, wy, interior_only, win, win_lo, &flags, tid,
+                                                   ss);
   };
   const int pX = (ty + 2) * G::HX + (tx + 2);
   const int pM = (ty + 1) * G::MX + (tx + 1);
   const bool in_tile = (x0 + tx < P.nx) && (y0 + ty < P.ny);
 
   __syncthreads();
-  if constexpr (SPLIT) {          // faces need X and mu/M of planes z and z+1 only
-    load_x(zb - 1);
-    load_x(zb);
-    compute_mu(zb - 1, true);
-    compute_mu(zb, false);
-  } else {
-    load_x(zb - 2);
-    load_x(zb - 1);
-    load_x(zb);
-    __syncthreads();
-    compute_mu(zb - 1, true);
-    __syncthreads();
-    load_x(zb + 1);
-    __syncthreads();
-    compute_mu(zb, false);
-  }
+  load_x(zb - 2);
+  load_x(zb - 1);
+  load_x(zb);
+  __syncthreads();
+  compute_mu(zb - 1, true);
+  __syncthreads();
+  load_x(zb + 1);
+  __syncthreads();
+  compute_mu(zb, false);
   __syncthreads();
   double Jm[S];
   face_between<G::PX, G::PM>(xplane(zb - 1), mplane(zb - 1), pX, pM, xplane(zb), mplane(zb), pX,
@@ -1150,14 +799,9 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
   double vmax = 0.0;
   for (int z = zb; z < ze; ++z) {
     __syncthreads();
-    if constexpr (SPLIT) {
-      load_x(z + 1);
-      compute_mu(z + 1, false);
-    } else {
-      load_x(z + 2);
-      __syncthreads();
-      compute_mu(z + 1, false);
-    }
+    load_x(z + 2);
+    __syncthreads();
+    compute_mu(z + 1, false);
     __syncthreads();
     double a[S];
     face_between<G::PX, G::PM>(xplane(z), mplane(z), pX, pM, xplane(z + 1), mplane(z + 1), pX,
@@ -1228,7 +872,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
 // ------------------------------------------------------------------------
 // Split rate evaluation, second kernel in 3D: faces and divergence of a
 // TY x TX plane tile marching along axis 0, from X and the mu/M rows that
-// k_chem64 wrote.  The X and mu/M of each plane (tile + 1-cell halo) go
+// k_chem wrote.  The X and mu/M of each plane (tile + 1-cell halo) go
 // through a three-plane ring in shared memory that cp.async fills two
 // planes ahead, so the loads of plane z+2 run under the faces of plane z.
 // Faces and the divergence sum in k_rate_march3d's order (fluxes.py:352-395:
@@ -1693,15 +1337,13 @@ constexpr int kGraphSteps = 50;      // steps per captured graph
 
 // Rate-kernel variants the autotuner chooses from: plane tile (TX x TY
 // threads) and the minimum resident blocks per SM (which caps registers);
-// fused (one kernel) or split (k_chem64 over all points, then the tile
-// kernel reading mu/M back).  All variants compute every value the same way.
+// fused (one kernel) or split (k_chem over all points, then the kernels that
+// read mu/M back).  All variants compute every value the same way.
 struct RateVariant {
   int tx, ty, minb;
   int nth;          // threads of a 2D block (1D block; >= tx * ty)
   bool win;
   bool split;
-  bool only3d = false;   // 2D runs another variant's kernels: not tuned there
-  bool only2d = false;   // 3D runs another variant's kernels: not tuned there
   size_t smem2d, smem3d;
   void (*set_attrs)(bool vec);
   void (*launch2d)(bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P);
@@ -1729,10 +1371,10 @@ RateVariant make_variant() {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (vec) {
       cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, true, WIN, false, NTH, SORT, PP>, a, s2);
-      cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, true, WIN, false, SORT, PP>, a, s3);
+      cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, true, WIN, SORT, PP>, a, s3);
     } else {
       cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, false, WIN, false, NTH, SORT, PP>, a, s2);
-      cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, false, WIN, false, SORT, PP>, a, s3);
+      cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, false, WIN, SORT, PP>, a, s3);
     }
   };
   v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
@@ -1741,44 +1383,29 @@ RateVariant make_variant() {
   };
   v.launch3d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P,
                   int zc) {
-    if (vec) launch_pdl(k_rate_march3d<TX, TY, MINB, true, WIN, false, SORT, PP>, g, b, sm, s, P, zc);
-    else launch_pdl(k_rate_march3d<TX, TY, MINB, false, WIN, false, SORT, PP>, g, b, sm, s, P, zc);
+    if (vec) launch_pdl(k_rate_march3d<TX, TY, MINB, true, WIN, SORT, PP>, g, b, sm, s, P, zc);
+    else launch_pdl(k_rate_march3d<TX, TY, MINB, false, WIN, SORT, PP>, g, b, sm, s, P, zc);
   };
   v.kernels = [](bool vec, int dim) {
     if (dim == 2) return kname("k_rate_tile2d", {TX, TY, MINB, vec, WIN, 0, NTH, SORT, PP});
-    return kname("k_rate_march3d", {TX, TY, MINB, vec, WIN, 0, SORT, PP});
+    return kname("k_rate_march3d", {TX, TY, MINB, vec, WIN, SORT, PP});
   };
   return v;
 }
 
-// The split form's mu/M kernel: k_chem64 (K = 1) or its shared-gather form
-// k_chem64i with K points per work item.
-template <int DIM, int KMINB, int K = 1>
+// The split form's mu/M kernel.
+template <int DIM>
 void launch_chem(bool vec, cudaStream_t s, const RateParams &P) {
-  if constexpr (K == 1) {
-    const dim3 b(32, 8), g((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + 7) / 8),
-                           (unsigned)P.nz);
-    if (vec) launch_pdl(k_chem64<DIM, true, KMINB>, g, b, 0, s, P);
-    else launch_pdl(k_chem64<DIM, false, KMINB>, g, b, 0, s, P);
-  } else {
-    using G = Chem64Geom<DIM, K>;
-    const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
-                 (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-    if (vec) launch_pdl(k_chem64i<DIM, true, K, KMINB>, g, dim3(kChem64Threads), G::smem, s, P);
-    else launch_pdl(k_chem64i<DIM, false, K, KMINB>, g, dim3(kChem64Threads), G::smem, s, P);
-  }
+  using G = ChemTile<DIM>;
+  const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
+               (unsigned)((P.nz + G::BZ - 1) / G::BZ));
+  if (vec) launch_pdl(k_chem<DIM, true>, g, dim3(kChemNT), 0, s, P);
+  else launch_pdl(k_chem<DIM, false>, g, dim3(kChemNT), 0, s, P);
 }
 
-template <int DIM, int KMINB, int K>
-void chem_attrs() {
-  if constexpr (K > 1) {
-    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k_chem64i<DIM, true, K, KMINB>, a, (int)Chem64Geom<DIM, K>::smem);
-    cudaFuncSetAttribute(k_chem64i<DIM, false, K, KMINB>, a, (int)Chem64Geom<DIM, K>::smem);
-  }
-}
-
-template <int TX, int TY, int MINB, int KMINB, bool PP = false, int K = 1>
+// Split variant: k_chem, then faces and divergence by the tile kernel in 2D
+// and by the cp.async marching kernel (PP: per-point faces) in 3D.
+template <int TX, int TY, int MINB, bool PP>
 RateVariant make_split_variant() {
   RateVariant v;
   v.tx = TX;
@@ -1788,72 +1415,6 @@ RateVariant make_split_variant() {
   v.win = false;
   v.split = true;
   v.smem2d = tile2d_smem<TX, TY>();
-  v.smem3d = march3d_smem<TX, TY>();
-  v.set_attrs = [](bool) {
-    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, true, false, true>, a,
-                         (int)tile2d_smem<TX, TY>());
-    cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, true, false, true, false, PP>, a,
-                         (int)march3d_smem<TX, TY>());
-    chem_attrs<2, KMINB, K>();
-    chem_attrs<3, KMINB, K>();
-  };
-  v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
-    launch_chem<2, KMINB, K>(vec, s, P);
-    launch_pdl(k_rate_tile2d<TX, TY, MINB, true, false, true>, g, b, sm, s, P);
-  };
-  v.launch3d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P,
-                  int zc) {
-    launch_chem<3, KMINB, K>(vec, s, P);
-    launch_pdl(k_rate_march3d<TX, TY, MINB, true, false, true, false, PP>, g, b, sm, s, P, zc);
-  };
-  v.kernels = [](bool vec, int dim) {
-    const std::string chem = (K == 1 ? kname("k_chem64", {dim, vec, KMINB})
-                                     : kname("k_chem64i", {dim, vec, K, KMINB})) + " + ";
-    if (dim == 2) return chem + kname("k_rate_tile2d", {TX, TY, MINB, 1, 0, 1, TX * TY, 0, 0});
-    return chem + kname("k_rate_march3d", {TX, TY, MINB, 1, 0, 1, 0, PP});
-  };
-  return v;
-}
-
-// Split variant for 3D with the cp.async marching flux kernel k_flux3_64
-// (PP: per-point faces) after the mu/M kernel CHEM (0: k_chem64, 1:
-// k_chem64s; k_chem64 for tables that are not double2-aligned); in 2D it
-// runs make_split_variant's kernels.
-template <int DIM, int KMINB, int CHEM>
-void launch_chem3(bool vec, cudaStream_t s, const RateParams &P) {
-  if (CHEM == 0 || !vec) {
-    launch_chem<DIM, KMINB, 1>(vec, s, P);
-    return;
-  }
-  const dim3 b(32, 8), g((unsigned)((P.nx + 31) / 32), (unsigned)((P.ny + 7) / 8), (unsigned)P.nz);
-  launch_pdl(k_chem64s<DIM, KMINB>, g, b, 0, s, P);
-}
-
-// Split variant for 2D with k_chem64s (coalesced mu/M rows) before the
-// split tile kernel; in 3D it runs make_split_variant's kernels.
-template <int TX, int TY, int MINB, int KMINB>
-RateVariant make_split2s_variant() {
-  RateVariant v = make_split_variant<TX, TY, MINB, KMINB>();
-  v.only2d = true;
-  v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
-    launch_chem3<2, KMINB, 1>(vec, s, P);
-    launch_pdl(k_rate_tile2d<TX, TY, MINB, true, false, true>, g, b, sm, s, P);
-  };
-  v.kernels = [](bool vec, int dim) {
-    if (dim == 2)
-      return (vec ? kname("k_chem64s", {2, KMINB}) : kname("k_chem64", {2, vec, KMINB})) + " + " +
-             kname("k_rate_tile2d", {TX, TY, MINB, 1, 0, 1, TX * TY, 0, 0});
-    return kname("k_chem64", {dim, vec, KMINB}) + " + " +
-           kname("k_rate_march3d", {TX, TY, MINB, 1, 0, 1, 0, 0});
-  };
-  return v;
-}
-
-template <int TX, int TY, int MINB, int KMINB, bool PP, int CHEM = 0>
-RateVariant make_split3_variant() {
-  RateVariant v = make_split_variant<TX, TY, MINB, KMINB>();
-  v.only3d = true;
   v.smem3d = Flux3Geom64<TX, TY>::smem(PP);
   v.set_attrs = [](bool) {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
@@ -1861,15 +1422,17 @@ RateVariant make_split3_variant() {
                          (int)tile2d_smem<TX, TY>());
     cudaFuncSetAttribute(k_flux3_64<TX, TY, MINB, PP>, a, (int)Flux3Geom64<TX, TY>::smem(PP));
   };
+  v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
+    launch_chem<2>(vec, s, P);
+    launch_pdl(k_rate_tile2d<TX, TY, MINB, true, false, true>, g, b, sm, s, P);
+  };
   v.launch3d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P,
                   int zc) {
-    launch_chem3<3, KMINB, CHEM>(vec, s, P);
+    launch_chem<3>(vec, s, P);
     launch_pdl(k_flux3_64<TX, TY, MINB, PP>, g, b, sm, s, P, zc);
   };
   v.kernels = [](bool vec, int dim) {
-    const std::string chem =
-        (CHEM == 0 || !vec ? kname("k_chem64", {dim, vec, KMINB})
-                           : kname("k_chem64s", {dim, KMINB})) + " + ";
+    const std::string chem = kname("k_chem", {dim, vec}) + " + ";
     if (dim == 2) return chem + kname("k_rate_tile2d", {TX, TY, MINB, 1, 0, 1, TX * TY, 0, 0});
     return chem + kname("k_flux3_64", {TX, TY, MINB, PP});
   };
@@ -1881,9 +1444,6 @@ const std::vector<RateVariant> &rate_variants() {
       make_variant<32, 8, 2>(), make_variant<32, 8, 3>(), make_variant<32, 4, 4>(),
       make_variant<16, 8, 4>(), make_variant<64, 4, 2>(), make_variant<32, 4, 6>(),
       make_variant<32, 8, 2, false>(), make_variant<32, 8, 3, false>(),
-      make_split_variant<32, 8, 3, 2>(), make_split_variant<32, 8, 3, 3>(),
-      make_split_variant<32, 4, 4, 2>(), make_split_variant<32, 4, 4, 3>(),
-      make_split_variant<32, 8, 3, 4>(), make_split_variant<32, 4, 4, 4>(),
       make_variant<32, 8, 2, true, 352, true>(), make_variant<32, 8, 2, false, 352, true>(),
       make_variant<32, 8, 2, true, 352, false>(), make_variant<32, 4, 4, true, 224, true>(),
       make_variant<32, 4, 4, false, 224, true>(), make_variant<32, 16, 1, false, 608, true>(),
@@ -1891,15 +1451,10 @@ const std::vector<RateVariant> &rate_variants() {
       make_variant<32, 8, 2, false, 256, 2, true>(), make_variant<32, 8, 2, false, 256, 2, false>(),
       make_variant<32, 4, 4, false, 128, 2, true>(),
       make_variant<32, 8, 3, false, 256, false, true>(), make_variant<64, 4, 2, true, 256, false, true>(),
-      make_split_variant<32, 8, 3, 3, true>(), make_split_variant<32, 4, 4, 3, true>(),
-      make_split_variant<32, 8, 3, 2, false, 2>(), make_split_variant<32, 4, 4, 2, false, 2>(),
-      make_split_variant<32, 8, 3, 2, true, 2>(), make_split_variant<32, 4, 4, 2, true, 2>(),
-      make_split3_variant<32, 4, 3, 3, true>(), make_split3_variant<32, 4, 3, 3, false>(),
-      make_split3_variant<32, 8, 2, 3, true>(), make_split3_variant<32, 8, 2, 3, false>(),
-      make_split3_variant<64, 4, 1, 3, true>(), make_split3_variant<32, 4, 2, 3, true>(),
-      make_split3_variant<32, 4, 3, 3, true, 1>(), make_split3_variant<32, 4, 3, 4, true, 1>(),
-      make_split3_variant<32, 4, 2, 3, true, 1>(),
-      make_split2s_variant<32, 8, 3, 4>()};
+      make_split_variant<32, 4, 3, true>(), make_split_variant<32, 4, 3, false>(),
+      make_split_variant<32, 8, 2, true>(), make_split_variant<32, 8, 2, false>(),
+      make_split_variant<64, 4, 1, true>(), make_split_variant<32, 4, 2, true>(),
+      make_split_variant<32, 8, 3, true>()};
   return v;
 }
 
@@ -2003,8 +1558,6 @@ pf5d_status autotune_rate(pf5d_stepper *h, cudaStream_t s, float *best_ms) {
   const int reps = 5;
   std::vector<std::pair<float, int>> rate_t;
   for (int v = 0; v < (int)rate_variants().size(); ++v) {
-    if (rate_variants()[v].only3d && h->d.dim != 3) continue;
-    if (rate_variants()[v].only2d && h->d.dim != 2) continue;
     pf5d_status st = configure_rate(h, v);
     if (st != PF5D_OK) continue;
     if (launch_rate(h, s) != PF5D_OK) {           // warm-up (e.g. too much smem)
@@ -2429,9 +1982,9 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
     if ((st = launch_rate(h, s)) != PF5D_OK) return st;
     // mu and M of this step at every point, then the "before" reductions
     switch (dim) {
-      case 1: launch_chem<1, 3>(h->vec, s, h->rp); break;
-      case 2: launch_chem<2, 3>(h->vec, s, h->rp); break;
-      default: launch_chem<3, 3>(h->vec, s, h->rp);
+      case 1: launch_chem<1>(h->vec, s, h->rp); break;
+      case 2: launch_chem<2>(h->vec, s, h->rp); break;
+      default: launch_chem<3>(h->vec, s, h->rp);
     }
     PF5D_LAUNCHED();
     Xpre = h->X;
