@@ -54,6 +54,8 @@ typedef enum {
 #define PF5D_FLAG_NN_USED      0x20u  /* some point took the nearest-row fallback   */
 #define PF5D_FLAG_HALTED       0x40u  /* step loop stopped (OOB check or an NN error) */
 #define PF5D_FLAG_NN_NONFINITE 0x80u  /* a fallback point had a NaN/inf component   */
+#define PF5D_FLAG_STALLED      0x100u /* the 1D step loop's blocks lost each other: a
+                                         wait gave up; halted, field as before the call */
 /* The nearest-row search is exact for every finite point (it widens its
  * window until the nearest present node is proven).  NN_FAR, NN_TRUNCATED and
  * NN_NONFINITE are errors where the reference raises (RuntimeError for the
@@ -275,7 +277,7 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
  * pf5d_stepper_set_variant are 0 .. count-1); 0 for a null stepper. */
 int32_t pf5d_stepper_variant_count(const pf5d_stepper *h);
 /* Kernels of this library that one step launches with the current variant
- * (rate kernel(s), dt controller, update, and when elasticity is on the B(k)
+ * (a 1D solve advanced by the step loop: one, for up to 2000 steps; otherwise rate kernel(s), dt controller, update, and when elasticity is on the B(k)
  * multiply -- the column kernel in 2D with a power-of-two axis 0, the
  * closed-form kernel in 1D; cuFFT's own kernels not counted); 0 for a null
  * stepper. */

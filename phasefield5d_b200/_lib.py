@@ -30,6 +30,7 @@ FLAG_NN_TRUNCATED = 0x10
 FLAG_NN_USED = 0x20
 FLAG_HALTED = 0x40
 FLAG_NN_NONFINITE = 0x80
+FLAG_STALLED = 0x100
 
 STAGE_RATE, STAGE_UPDATE, STAGE_FFT_FWD, STAGE_BMUL, STAGE_FFT_INV = 0, 1, 2, 3, 4
 PRECISION_FP64, PRECISION_FP32C = 0, 1

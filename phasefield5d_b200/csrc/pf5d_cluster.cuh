@@ -1,0 +1,148 @@
+// pf5d_cluster.cuh -- what the 1D step loops share (one thread-block cluster
+// advances a whole solve, many steps per launch): the split of the points over
+// the cluster's blocks, the sum behind the closed-form elastic term, and the
+// launch.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+#include <cooperative_groups.h>
+
+#include "pf5d_host.h"
+
+namespace pf5d {
+
+constexpr int64_t kLoop1dMax = 16384;        // points of a 1D solve that a cluster advances
+constexpr int kLoop1dThreads = 512;          // most threads of a block (128 registers each)
+constexpr int kLoop1dBlocks = 16;            // most blocks of a cluster
+constexpr int kLoop1dSteps = 2000;           // most steps of a launch
+constexpr int kLoop1dGroups = (int)(kLoop1dMax / 32);
+
+// Sum of n values in groups of 32 consecutive ones: a fixed tree within each
+// group (group_sum); then each lane adds every 32nd group's sum in order and a
+// tree adds the lanes (sum_groups).  The result does not depend on how the
+// groups are spread over warps and blocks.  Called by whole warps.
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = v + __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ double sum_groups(const double *sums, int n) {
+  double v = 0.0;
+  for (int g = threadIdx.x & 31; g < n; g += 32) v = v + sums[g];
+  return group_sum(v);
+}
+
+// ------------------------------------------------------------------------
+// Messages between the blocks of a cluster: 16 bytes into another block's
+// shared memory that also count towards an mbarrier there.  A block waits on
+// its own mbarrier for the bytes it expects, so it meets the others without a
+// cluster barrier -- whose acquire at cluster scope empties the L1, and with it
+// the table nodes that the next step reads again.
+// ------------------------------------------------------------------------
+__device__ __forceinline__ unsigned shared_addr(const void *p) {
+  return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ unsigned rank_addr(unsigned addr, int rank) {
+  unsigned r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void send2(unsigned dst, unsigned bar, unsigned long long a,
+                                      unsigned long long b) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];"
+               :: "r"(dst), "l"(a), "l"(b), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void mbar_init(unsigned bar) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+}
+// One thread per phase: the phase ends when `bytes` have come in.
+__device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+}
+constexpr int kMbarTries = 1 << 22;          // then the wait gives up
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+  for (int i = 0; i < kMbarTries; ++i) {
+    unsigned ok;
+    asm volatile("{\n.reg .pred p;\n"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 "selp.b32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+
+// Max over the warp of non-negative values, none NaN: their bits are ordered
+// as the values are, so two 32-bit reductions replace five rounds of shuffles.
+__device__ __forceinline__ double warp_max_nonneg(double v) {
+  const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+  const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
+  return __hiloint2double((int)mh, (int)ml);
+}
+
+// Blocks of the cluster, points per block (a multiple of 32) and threads per
+// block for n points.  A block evaluates mu/M at its points and one halo
+// position on each side: all warps but the last (which sums the misfit
+// meanwhile) cover chunk + 2 positions in as few passes as kLoop1dThreads
+// allows.
+struct Loop1dShape {
+  int blocks, chunk, threads;
+};
+inline Loop1dShape loop1d_shape(int64_t n, int max_blocks) {
+  Loop1dShape L;
+  const int groups = (int)((n + 31) / 32);
+  L.blocks = 1;
+  while (L.blocks < max_blocks && L.blocks < groups) L.blocks *= 2;
+  L.chunk = 32 * ((groups + L.blocks - 1) / L.blocks);
+  const int most = kLoop1dThreads - 32;
+  const int passes = (L.chunk + 2 + most - 1) / most;
+  L.threads = 32 + 32 * (((L.chunk + 2 + passes - 1) / passes + 31) / 32);
+  return L;
+}
+
+// One cluster of L.blocks blocks.
+template <typename... KArgs, typename... Args>
+cudaError_t launch_cluster(void (*kernel)(KArgs...), const Loop1dShape &L, size_t smem,
+                           cudaStream_t s, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L.blocks);
+  cfg.blockDim = dim3(L.threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = L.blocks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// Whether this device can hold the cluster (once per solve, at its creation).
+template <typename... KArgs>
+bool cluster_fits(void (*kernel)(KArgs...), const Loop1dShape &L, size_t smem) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(L.blocks);
+  cfg.blockDim = dim3(L.threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = L.blocks;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  const cudaError_t e = cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+  cudaGetLastError();
+  return e == cudaSuccess && n > 0;
+}
+
+}  // namespace pf5d

@@ -36,6 +36,7 @@
 
 #include <cuda_pipeline_primitives.h>
 
+#include "pf5d_cluster.cuh"
 #include "pf5d_device.cuh"
 #include "pf5d_fft.h"
 #include "pf5d_fp32c.h"
@@ -1273,26 +1274,374 @@ namespace pf5d {
 // s' = bn (s - mean s) + b0 mean s, where bn is B(k) for every k != 0 and
 // b0 is B(0).  That is irfft(B rfft(s)) (elastic.py:250-263) exactly, for a
 // B(k) that depends on k only through its sign, as every 1D B(k) does.  One
-// block: per-thread sums over a fixed stride, then a fixed tree, so the
-// mean has the same bits on every run.
+// block; the mean is summed in the order of pf5d_cluster.cuh, as k_loop1d
+// sums it, so a step has the same bits either way.
 constexpr int kElastic1dThreads = 1024;
-constexpr int64_t kElastic1dMax = 16384;     // points of a 1D solve that use it
+constexpr int64_t kElastic1dMax = kLoop1dMax;     // points of a 1D solve that use it
 __global__ void __launch_bounds__(kElastic1dThreads)
     k_elastic1d(double *s, int64_t n, double bn, double b0, const unsigned *halt) {
-  __shared__ double red[kElastic1dThreads / 32];
+  __shared__ double sums[kLoop1dGroups];
   pdl_wait();
   if (*halt) return;
-  const int t = threadIdx.x;
-  double acc = 0.0;
-  for (int64_t i = t; i < n; i += kElastic1dThreads) acc = acc + s[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((t & 31) == 0) red[t >> 5] = acc;
+  const int t = threadIdx.x, ng = (int)((n + 31) / 32);
+  for (int g = t >> 5; g < ng; g += kElastic1dThreads / 32) {
+    const int64_t i = 32 * (int64_t)g + (t & 31);
+    const double v = group_sum(i < n ? s[i] : 0.0);
+    if ((t & 31) == 0) sums[g] = v;
+  }
   __syncthreads();
-  double tot = red[0];
-  for (int w = 1; w < kElastic1dThreads / 32; ++w) tot = tot + red[w];
-  const double mean = tot / (double)n;
+  const double mean = sum_groups(sums, ng) / (double)n;
   for (int64_t i = t; i < n; i += kElastic1dThreads) s[i] = bn * (s[i] - mean) + b0 * mean;
+}
+
+// ------------------------------------------------------------------------
+// 1D step loop: one cluster advances the whole solve, many steps per launch.
+// ------------------------------------------------------------------------
+// A 1D step is a few microseconds of work, and as four kernels (elastic term,
+// rate, dt, update) most of its time went to launches and to their cold
+// caches.  Here each block of the cluster keeps its chunk of points in shared
+// memory for all steps of the launch, and the blocks exchange two rounds of
+// messages per step (pf5d_cluster.cuh):
+//   before A: mu/M at the chunk and one halo position on each side, without
+//     the elastic term (the last warp sums the misfit meanwhile), then mu and
+//     the faces, dX/dt;
+//   A, each warp to every block: its max |dX/dt| and nearest-row flags.  Every
+//     thread then forms the same dt; update and clamp;
+//   B, to every block: each 32 points' misfit sum and out-of-bounds flags; to
+//     the neighbours: the points of their halos.
+// One copy of each message is enough: a block sends A of a step only when it
+// has all of B of the step before, and every warp has read that by then; it
+// sends B only when it has all of A, and B leaves after the block's barrier
+// that follows the reads of A.
+// Values are formed as k_elastic1d, k_rate_1d, k_dt_finish and k_update_step
+// form them.  The positions are taken in the order of their table cells, so
+// that the lanes of a warp read few nodes; the cells hardly change from step to
+// step, so the order is renewed every kLoop1dResort steps (it decides which
+// thread evaluates a position, never a value).
+//
+// Bound by the latency of a step's dependent phases, in large solves by the
+// table loads of 16 SMs.  Steps of a long run, on-node composition, four
+// kernels -> here: 203 points 14.4 -> 3.3 us, 1280 14.7 -> 3.6, 4112 16.1 ->
+// 5.7, 16384 18.0 -> 14.1 -- so every solve with the closed-form elastic term
+// (or none) takes it.  With cluster barriers in place of the messages a step
+// of 1280 points was 6.0 us, without the cell order 5.0.
+struct Loop1dSmem {
+  ulonglong2 sums[kLoop1dGroups];        // B: misfit sum (bits) and flags of every group
+  ulonglong2 max[kLoop1dBlocks * (kLoop1dThreads / 32)];   // A: max |dX/dt| (bits), flags
+  ulonglong2 halo[4][2];                 // B: positions -2, -1, m, m + 1
+  double own[kLoop1dGroups];             // this block's groups, before they are sent
+  unsigned own_flags[kLoop1dGroups];
+  double mean, pad;
+  unsigned long long bar_a, bar_b;
+  int bins[256];                         // of the cell sort
+};
+// then X [S][chunk + 4], mu/M and the misfit [NP + 1][chunk + 2],
+// faces [S][chunk + 1], dX/dt [S][chunk], order [chunk + 2] (16 bit)
+inline size_t loop1d_smem(int chunk) {
+  return sizeof(Loop1dSmem) + sizeof(double) * ((size_t)S * (chunk + 4) + (NP + 1) * (chunk + 2) +
+                                                S * (chunk + 1) + S * chunk) +
+         sizeof(unsigned short) * (chunk + 2);
+}
+constexpr int kLoop1dResort = 128;
+
+template <bool VEC, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k_loop1d(RateParams P, UpdateParams U, double bn, double b0, int chunk, int nsteps) {
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  extern __shared__ __align__(16) unsigned char lraw[];
+  Loop1dSmem &sm = *reinterpret_cast<Loop1dSmem *>(lraw);
+  const int HX = chunk + 4, MX = chunk + 2, FX = chunk + 1;
+  double *Xs = reinterpret_cast<double *>(lraw + sizeof(Loop1dSmem));
+  double *Ms = Xs + S * HX, *Qs = Ms + NP * MX, *Fs = Qs + MX, *Ds = Fs + S * FX;
+  unsigned short *order = reinterpret_cast<unsigned short *>(Ds + S * chunk);
+  StepState *st = P.st;
+  if (st->halt) return;
+  const int n = P.nx, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nw = (int)blockDim.x >> 5, nt = (int)blockDim.x - 32;   // the last warp sums
+  const bool worker = t < nt;
+  const int rank = (int)cluster.block_rank(), nb = (int)cluster.num_blocks();
+  const int i0 = rank * chunk, m = max(0, min(chunk, n - i0));
+  const int ng = (n + 31) / 32;
+  const unsigned bar_a = shared_addr(&sm.bar_a), bar_b = shared_addr(&sm.bar_b);
+  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + (m > 0 ? sizeof(sm.halo) : 0u);
+  double dt = st->dt, time = st->time, xdotmax = st->xdotmax;
+  long long step = st->step;
+  // steps until the next out-of-bounds test (the one after which step is a multiple)
+  int to_check = U.oob_interval > 0 ? U.oob_interval - (int)(step % U.oob_interval) : -1;
+  unsigned flags = 0;
+  bool halt = false, stalled = false, checked = false;
+
+  auto misfit = [&](const double x[S]) {
+    double acc = 0.0;
+#pragma unroll
+    for (int c = 0; c < S; ++c) acc = acc + (x[c] - U.x0.v[c]) * U.lvec.v[c];
+    return acc;
+  };
+  // The halo entry this thread keeps current: entry h of block b holds the
+  // point at Xs index hsrc of this block (none: hsrc < 0).  4 * nb <= threads.
+  int hsrc = -1;
+  unsigned hdst = 0, hbar = 0;
+  {
+    const int b = t >> 2, h = t & 3;
+    const int bm = b < nb ? max(0, min(chunk, n - b * chunk)) : 0;
+    if (bm > 0 && m > 0) {
+      const int src = wrap_any(b * chunk + (h < 2 ? h - 2 : bm + h - 2), n) - i0;
+      if (src >= 0 && src < m) {
+        hsrc = src + 2;
+        hdst = rank_addr(shared_addr(sm.halo[h]), b);
+        hbar = rank_addr(bar_b, b);
+      }
+    }
+  }
+  // B: the chunk's groups and the halo entries, from what the block holds now
+  auto send_b = [&]() {
+    for (int g = warp; 32 * g < m; g += nw)
+      if (lane < nb)
+        send2(rank_addr(shared_addr(&sm.sums[i0 / 32 + g]), lane), rank_addr(bar_b, lane),
+              (unsigned long long)__double_as_longlong(sm.own[g]), sm.own_flags[g]);
+    if (hsrc >= 0)
+#pragma unroll
+      for (int c = 0; c < S; c += 2)
+        send2(hdst + 8 * c, hbar, (unsigned long long)__double_as_longlong(Xs[c * HX + hsrc]),
+              (unsigned long long)__double_as_longlong(Xs[(c + 1) * HX + hsrc]));
+  };
+  // 32 points from p0 (x: this lane's): their misfit sum and flags
+  auto keep_group = [&](const double x[S], int p0, unsigned f) {
+    const double v = P.sp ? group_sum(p0 + lane < m ? misfit(x) : 0.0) : 0.0;
+    const unsigned any = __reduce_or_sync(0xffffffffu, f);
+    if (lane == 0) {
+      sm.own[p0 >> 5] = v;
+      sm.own_flags[p0 >> 5] = any;
+    }
+  };
+
+  // positions in the order of their cells (a counting sort over cell_hash)
+  auto sort_cells = [&]() {
+    for (int b = t; b < 256; b += (int)blockDim.x) sm.bins[b] = 0;
+    __syncthreads();
+    auto key = [&](int pos) {
+      double x[S];
+#pragma unroll
+      for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + pos + 1];
+      return cell_hash(x, (float)P.T.inv_step);
+    };
+    for (int pos = t; pos < m + 2; pos += (int)blockDim.x) atomicAdd(&sm.bins[key(pos)], 1);
+    __syncthreads();
+    if (warp == 0) {
+      int v[8], sum = 0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        v[j] = sum;
+        sum += sm.bins[8 * lane + j];
+      }
+      int before = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += u;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sm.bins[8 * lane + j] = before - sum + v[j];
+    }
+    __syncthreads();
+    for (int pos = t; pos < m + 2; pos += (int)blockDim.x)
+      order[atomicAdd(&sm.bins[key(pos)], 1)] = (unsigned short)pos;
+    __syncthreads();
+  };
+
+  if (t == 0) {
+    mbar_init(bar_a);
+    mbar_init(bar_b);
+  }
+  for (int p = t; p < m; p += (int)blockDim.x) {
+    const double2 a = reinterpret_cast<const double2 *>(P.X + 4 * (int64_t)(i0 + p))[0];
+    const double2 b = reinterpret_cast<const double2 *>(P.X + 4 * (int64_t)(i0 + p))[1];
+    Xs[p + 2] = a.x;
+    Xs[HX + p + 2] = a.y;
+    Xs[2 * HX + p + 2] = b.x;
+    Xs[3 * HX + p + 2] = b.y;
+  }
+  __syncthreads();
+  for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+    double x[S];
+#pragma unroll
+    for (int c = 0; c < S; ++c) x[c] = p0 + lane < m ? Xs[c * HX + p0 + lane + 2] : 0.0;
+    keep_group(x, p0, 0);
+  }
+  cluster.sync();                        // every block has started and set up its barriers
+  if (t == 0) mbar_expect(bar_b, bytes_b);
+  send_b();
+
+  for (int k = 0; k <= nsteps; ++k) {
+    // B of the step before (k = 0: the state at the launch)
+    stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
+    if (t < 8 && m > 0) {                // halo entries into the chunk's rows
+      const int h = t >> 1, c = 2 * (t & 1), p = h < 2 ? h : m + h;
+      const ulonglong2 v = sm.halo[h][t & 1];
+      Xs[c * HX + p] = __longlong_as_double((long long)v.x);
+      Xs[(c + 1) * HX + p] = __longlong_as_double((long long)v.y);
+    }
+    if (checked) {
+      unsigned f = 0;
+      for (int g = lane; g < ng; g += 32) f |= (unsigned)sm.sums[g].y;
+      f = __reduce_or_sync(0xffffffffu, f);
+      flags |= f;
+      if (f & (PF5D_FLAG_NONFINITE | PF5D_FLAG_OOB_HARD)) halt = true;
+    }
+    if (__syncthreads_or(stalled)) stalled = true;
+    if (halt || stalled || k == nsteps) break;
+    if (m > 0 && k % kLoop1dResort == 0) sort_cells();
+    unsigned nn = 0;
+    if (worker) {
+      if (m > 0)
+        for (int w = t; w < m + 2; w += nt) {
+          const int pos = order[w];
+          double x[S], v[NP];
+#pragma unroll
+          for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + pos + 1];
+          interp_point<VEC>(P.T, x, v, &nn);
+#pragma unroll
+          for (int c = 0; c < S; ++c) {
+            const double *q = Xs + c * HX + pos + 1;
+            const double lap = (q[1] + q[-1] - 2.0 * x[c]) * P.inv_dx2;
+            const double lk = lap * P.kappa.v[c];
+            Ms[c * MX + pos] = v[c] - lk;
+          }
+#pragma unroll
+          for (int c = 0; c < NM; ++c) Ms[(S + c) * MX + pos] = v[S + c];
+          if (P.sp) Qs[pos] = misfit(x);
+        }
+    } else {
+      if (lane == 0) {
+        mbar_expect(bar_a, bytes_a);
+        mbar_expect(bar_b, bytes_b);
+      }
+      if (P.sp) {
+        double total = 0.0;
+        for (int g = lane; g < ng; g += 32)
+          total = total + __longlong_as_double((long long)sm.sums[g].x);
+        total = group_sum(total);
+        if (lane == 0) sm.mean = total / (double)n;
+      }
+    }
+    __syncthreads();
+    // face i lies between mu/M positions i and i+1 (X positions i+1, i+2)
+    if (m > 0) {
+      const double mean = sm.mean;
+      for (int i = t; i < m + 1; i += (int)blockDim.x) {
+        double Xc[S], Xn[S], Mc[NM], Mn[NM], g[S], J[S];
+        const double sc = P.sp ? bn * (Qs[i] - mean) + b0 * mean : 0.0;
+        const double sn = P.sp ? bn * (Qs[i + 1] - mean) + b0 * mean : 0.0;
+#pragma unroll
+        for (int c = 0; c < S; ++c) {
+          Xc[c] = Xs[c * HX + i + 1];
+          Xn[c] = Xs[c * HX + i + 2];
+          double muc = Ms[c * MX + i], mun = Ms[c * MX + i + 1];
+          if (P.sp) {
+            muc = muc + sc * P.lvec.v[c];
+            mun = mun + sn * P.lvec.v[c];
+          }
+          g[c] = (mun - muc) * P.inv_dx;
+        }
+#pragma unroll
+        for (int c = 0; c < NM; ++c) {
+          Mc[c] = Ms[(S + c) * MX + i];
+          Mn[c] = Ms[(S + c) * MX + i + 1];
+        }
+        face_flux(Xc, Mc, Xn, Mn, g, J);
+#pragma unroll
+        for (int c = 0; c < S; ++c) Fs[c * FX + i] = J[c];
+      }
+    }
+    __syncthreads();
+    double vmax = 0.0;
+    for (int p = t; p < m; p += (int)blockDim.x)
+#pragma unroll
+      for (int c = 0; c < S; ++c) {
+        const double d = (Fs[c * FX + p + 1] - Fs[c * FX + p]) * P.inv_dx;
+        Ds[c * chunk + p] = d;
+        const double v = fabs(d);
+        if (v > vmax) vmax = v;
+      }
+    vmax = warp_max_nonneg(vmax);
+    nn = __reduce_or_sync(0xffffffffu, nn);
+    if (lane < nb)
+      send2(rank_addr(shared_addr(&sm.max[rank * nw + warp]), lane), rank_addr(bar_a, lane),
+            (unsigned long long)__double_as_longlong(vmax), nn);
+    stalled = stalled || !mbar_wait(bar_a, (unsigned)k & 1u);       // A
+    double gmax = 0.0;
+    nn = 0;
+    for (int i = lane; i < nb * nw; i += 32) {
+      gmax = fmax(gmax, __longlong_as_double((long long)sm.max[i].x));
+      nn |= (unsigned)sm.max[i].y;
+    }
+    gmax = warp_max_nonneg(gmax);
+    nn = __reduce_or_sync(0xffffffffu, nn);
+    flags |= nn;
+    if (nn & kNNErrorFlags) {            // the same in every block: stop before the update
+      halt = true;
+      break;
+    }
+    if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
+    time = time + dt;
+    xdotmax = gmax;
+    step = step + 1;
+    checked = --to_check == 0;
+    if (checked) to_check = U.oob_interval;
+    for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+      const int p = p0 + lane;
+      double x[S] = {0.0, 0.0, 0.0, 0.0};
+      unsigned fo = 0;
+      if (p < m) {
+#pragma unroll
+        for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + p + 2] + Ds[c * chunk + p] * dt;
+        double sum = 0.0;
+#pragma unroll
+        for (int c = 0; c < S; ++c) sum = sum + x[c];
+        if (sum > 1.0) {
+          const double inv = 1.0 / sum;
+#pragma unroll
+          for (int c = 0; c < S; ++c) x[c] = x[c] * inv;
+        }
+#pragma unroll
+        for (int c = 0; c < S; ++c) Xs[c * HX + p + 2] = x[c];
+        if (checked) fo = oob_flags(x);
+      }
+      keep_group(x, p0, fo);
+    }
+    __syncthreads();
+    send_b();
+  }
+
+  if (!stalled)
+    for (int p = t; p < m; p += (int)blockDim.x) {
+      double x[S], d[S];
+#pragma unroll
+      for (int c = 0; c < S; ++c) {
+        x[c] = Xs[c * HX + p + 2];
+        d[c] = Ds[c * chunk + p];
+      }
+      const int64_t g = i0 + p;
+      double2 *xo = reinterpret_cast<double2 *>(U.X + 4 * g);
+      double2 *o = reinterpret_cast<double2 *>(P.dX + 4 * g);
+      xo[0] = make_double2(x[0], x[1]);
+      xo[1] = make_double2(x[2], x[3]);
+      o[0] = make_double2(d[0], d[1]);
+      o[1] = make_double2(d[2], d[3]);
+      if (U.s) U.s[g] = misfit(x);
+    }
+  if (stalled && t == 0) {
+    atomicOr(&st->flags, PF5D_FLAG_STALLED);
+    atomicExch(&st->halt, 1u);
+  } else if (rank == 0 && t == 0) {
+    st->dt = dt;
+    st->time = time;
+    st->xdotmax = xdotmax;
+    st->step = step;
+    if (flags) atomicOr(&st->flags, flags);
+    if (halt) atomicExch(&st->halt, 1u);
+  }
+  cluster.sync();                        // no block leaves while another may still send to it
 }
 
 }  // namespace pf5d
@@ -1326,6 +1675,8 @@ struct pf5d_stepper {
   ColPass2D colp;                // 2D elastic term: row transforms + one column kernel
   bool use_colpass = false;
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
+  bool use_loop1d = false;       // 1D steps by k_loop1d
+  Loop1dShape loop;
   double *save_x = nullptr;      // FP32C save steps: FP64 field, dX/dt, mu/M
   std::string kernels;           // text returned by pf5d_stepper_rate_kernels
 };
@@ -1655,6 +2006,15 @@ pf5d_status enqueue_step(pf5d_stepper *h, cudaStream_t s) {
   return PF5D_OK;
 }
 
+// The step loop of a 1D solve.  Blocks of up to 256 threads may take 255
+// registers each, which lets the table loads run ahead of the sums.
+using Loop1dKernel = void (*)(RateParams, UpdateParams, double, double, int, int);
+Loop1dKernel loop1d_kernel(const pf5d_stepper *h) {
+  const bool few = h->loop.threads <= kLoop1dThreads / 2;
+  if (h->vec) return few ? k_loop1d<true, kLoop1dThreads / 2> : k_loop1d<true, kLoop1dThreads>;
+  return few ? k_loop1d<false, kLoop1dThreads / 2> : k_loop1d<false, kLoop1dThreads>;
+}
+
 pf5d_status graph_for(pf5d_stepper *h, int64_t nsteps, cudaGraphExec_t *out) {
   auto it = h->graphs.find(nsteps);
   if (it != h->graphs.end()) {
@@ -1818,6 +2178,12 @@ pf5d_status pf5d_stepper_create(const pf5d_stepper_desc *desc, double *X, void *
   U.s = desc->elastic ? h->s : nullptr;
   U.oob_interval = desc->oob_interval;
   if ((st = configure_rate(h, 0)) != PF5D_OK) return fail(st);
+  if (desc->dim == 1 && npts <= kLoop1dMax && (!desc->elastic || h->closed1d))
+    for (int blocks = kLoop1dBlocks; blocks >= 8 && !h->use_loop1d; blocks /= 2) {
+      h->loop = loop1d_shape(npts, blocks);
+      const size_t sm = loop1d_smem(h->loop.chunk);
+      h->use_loop1d = cluster_fits(loop1d_kernel(h), h->loop, sm);
+    }
   if ((st = pf5d_stepper_reset(h, desc->dt0, 0.0, stream)) != PF5D_OK) return fail(st);
   (void)s;
   *out = h;
@@ -1853,6 +2219,15 @@ pf5d_status pf5d_stepper_advance(pf5d_stepper *h, int64_t nsteps, void *stream) 
   PF5D_REQUIRE(h && nsteps >= 0, PF5D_ERR_ARG, "bad arguments");
   if (h->s32) return s32_advance(h->s32, nsteps, stream);
   cudaStream_t s = as_stream(stream);
+  if (h->use_loop1d) {
+    const size_t sm = loop1d_smem(h->loop.chunk);
+    for (; nsteps > 0; nsteps -= kLoop1dSteps) {
+      const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);
+      PF5D_CUDA(launch_cluster(loop1d_kernel(h), h->loop, sm, s, h->rp, h->up, h->bn, h->b0,
+                               h->loop.chunk, n));
+    }
+    return PF5D_OK;
+  }
   while (nsteps > 0) {
     const int64_t n = nsteps < kGraphSteps ? nsteps : kGraphSteps;
     cudaGraphExec_t g = nullptr;
@@ -2052,6 +2427,7 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
 int32_t pf5d_stepper_launches_per_step(const pf5d_stepper *h) {
   if (!h) return 0;
   if (h->s32) return s32_launches_per_step(h->s32);
+  if (h->use_loop1d) return 1;
   const bool split = h->d.dim >= 2 && rate_variants()[h->variant].split;
   return (split ? 2 : 1) + 2 + (h->d.elastic ? 1 : 0);   // rate (+chem), dt, update, bmul
 }
