@@ -34,6 +34,24 @@ __device__ __forceinline__ double sum_groups(const double *sums, int n) {
   return group_sum(v);
 }
 
+// Exclusive prefix sum of 256 shared counters by one warp.
+__device__ __forceinline__ void scan_bins256(int *bins, int lane) {
+  int v[8], sum = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    v[j] = sum;
+    sum += bins[8 * lane + j];
+  }
+  int upto = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, upto, o);
+    if (lane >= o) upto += u;
+  }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) bins[8 * lane + j] = upto - sum + v[j];
+}
+
 // ------------------------------------------------------------------------
 // Messages between the blocks of a cluster: 16 bytes into another block's
 // shared memory that also count towards an mbarrier there.  A block waits on

@@ -28,6 +28,7 @@
 #include <cuda_pipeline_primitives.h>
 #include <cufft.h>
 
+#include "pf5d_cluster.cuh"
 #include "pf5d_device.cuh"
 #include "pf5d_fft.h"
 #include "pf5d_fp32c.h"
@@ -226,6 +227,31 @@ struct Update32 {
   int oob_interval;
 };
 
+// One point's compensated update and clamp: (h, l) += dtf * r, the simplex
+// clamp on X = X0 + D in FP64; dd is the new D in FP64.
+__device__ __forceinline__ void update_point32(const Update32 &U, float dtf, const float r[S],
+                                               float h[S], float l[S], double dd[S]) {
+#pragma unroll
+  for (int c = 0; c < S; ++c) comp_add(h[c], l[c], __fmul_rn(dtf, r[c]));
+  double dsum = 0.0;
+#pragma unroll
+  for (int c = 0; c < S; ++c) {
+    dd[c] = (double)h[c] + (double)l[c];
+    dsum = dsum + dd[c];
+  }
+  const double total = U.sum_x0 + dsum;
+  if (total > 1.0) {
+    const double inv = 1.0 / total;
+#pragma unroll
+    for (int c = 0; c < S; ++c) {
+      const double dn = (U.x0[c] + dd[c]) * inv - U.x0[c];
+      h[c] = (float)dn;
+      l[c] = (float)(dn - (double)h[c]);
+      dd[c] = (double)h[c] + (double)l[c];
+    }
+  }
+}
+
 __global__ void k32_update(Update32 U) {
   pdl_wait();
   StepState32 *st = U.st;
@@ -238,25 +264,8 @@ __global__ void k32_update(Update32 U) {
     const float4 H = U.hi[p], L = U.lo[p], R = U.dX[p];
     float h[S] = {H.x, H.y, H.z, H.w}, l[S] = {L.x, L.y, L.z, L.w};
     const float r[S] = {R.x, R.y, R.z, R.w};
-#pragma unroll
-    for (int c = 0; c < S; ++c) comp_add(h[c], l[c], __fmul_rn(dtf, r[c]));
-    double dd[S], dsum = 0.0;
-#pragma unroll
-    for (int c = 0; c < S; ++c) {
-      dd[c] = (double)h[c] + (double)l[c];
-      dsum = dsum + dd[c];
-    }
-    const double total = U.sum_x0 + dsum;
-    if (total > 1.0) {                 // clamp_simplex on X = X0 + D, in FP64
-      const double inv = 1.0 / total;
-#pragma unroll
-      for (int c = 0; c < S; ++c) {
-        const double dn = (U.x0[c] + dd[c]) * inv - U.x0[c];
-        h[c] = (float)dn;
-        l[c] = (float)(dn - (double)h[c]);
-        dd[c] = (double)h[c] + (double)l[c];
-      }
-    }
+    double dd[S];
+    update_point32(U, dtf, r, h, l, dd);
     U.hi[p] = make_float4(h[0], h[1], h[2], h[3]);
     U.lo[p] = make_float4(l[0], l[1], l[2], l[3]);
     if (U.s) {
@@ -742,26 +751,323 @@ __global__ void __launch_bounds__(kDt32Threads) k32_dt(Rate32 P, int nparts) {
 // The 1D elastic term in closed form, in place: s -> s' = bn (s - mean s) +
 // b0 mean s (bn: B(k) for every k != 0, b0: B(0)), i.e. irfft(B rfft(s))
 // exactly (elastic.py:250-263); the mean and the product in FP64, s' rounded
-// once to FP32.  One block, a fixed summation order.
+// once to FP32.  One block; the mean is summed in the order of
+// pf5d_cluster.cuh, as k32_loop1d sums it.
 constexpr int kElastic1dThreads32 = 1024;
-constexpr int64_t kElastic1dMax32 = 16384;
+constexpr int64_t kElastic1dMax32 = kLoop1dMax;
 __global__ void __launch_bounds__(kElastic1dThreads32)
     k32_elastic1d(float *s, int64_t n, double bn, double b0, const unsigned *halt) {
-  __shared__ double red[kElastic1dThreads32 / 32];
+  __shared__ double sums[kLoop1dGroups];
   pdl_wait();
   if (*halt) return;
-  const int t = threadIdx.x;
-  double acc = 0.0;
-  for (int64_t i = t; i < n; i += kElastic1dThreads32) acc = acc + (double)s[i];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) acc = acc + __shfl_xor_sync(0xffffffffu, acc, o);
-  if ((t & 31) == 0) red[t >> 5] = acc;
+  const int t = threadIdx.x, ng = (int)((n + 31) / 32);
+  for (int g = t >> 5; g < ng; g += kElastic1dThreads32 / 32) {
+    const int64_t i = 32 * (int64_t)g + (t & 31);
+    const double v = group_sum(i < n ? (double)s[i] : 0.0);
+    if ((t & 31) == 0) sums[g] = v;
+  }
   __syncthreads();
-  double tot = red[0];
-  for (int w = 1; w < kElastic1dThreads32 / 32; ++w) tot = tot + red[w];
-  const double mean = tot / (double)n;
+  const double mean = sum_groups(sums, ng) / (double)n;
   for (int64_t i = t; i < n; i += kElastic1dThreads32)
     s[i] = (float)(bn * ((double)s[i] - mean) + b0 * mean);
+}
+
+// ------------------------------------------------------------------------
+// 1D step loop of the precision form: the FP64 form's k_loop1d (same blocks,
+// messages and order of the phases) on the FP32 pair.  A halo entry brings the
+// neighbour point's hi part and its misfit.  Values are formed as
+// k32_elastic1d, k32_rate_1d, k32_dt and k32_update form them.
+//
+// Bound by the latency of a step's dependent phases.  Steps of a long run,
+// four kernels -> here: 203 points 10.3 -> 2.3 us, 1280 10.7 -> 2.5, 4112 11.4
+// -> 3.9, 16384 13.1 -> 9.0.
+// ------------------------------------------------------------------------
+struct Loop1dSmem32 {
+  ulonglong2 sums[kLoop1dGroups];        // B: misfit sum (bits) and flags of every group
+  ulonglong2 max[kLoop1dBlocks * (kLoop1dThreads / 32)];   // A: max |dX/dt| (bits), flags
+  ulonglong2 halo[4][2];                 // B: positions -2, -1, m, m + 1: hi; misfit
+  double own[kLoop1dGroups];             // this block's groups, before they are sent
+  unsigned own_flags[kLoop1dGroups];
+  double mean, pad;
+  unsigned long long bar_a, bar_b;
+  int bins[256];                         // of the cell sort
+};
+// then hi [chunk + 4], lo [chunk], per position mu (table), -kappa lap, M_1..4
+// and (M_Fe, X_Fe) [chunk + 2], faces [chunk + 1], dX/dt [chunk], the misfit
+// [chunk + 2], order [chunk + 2] (16 bit)
+inline size_t loop1d_smem32(int chunk) {
+  return sizeof(Loop1dSmem32) + sizeof(float4) * (size_t)(3 * chunk + 4 + 3 * (chunk + 2) + chunk + 1) +
+         sizeof(float2) * (chunk + 2) + sizeof(float) * (chunk + 2) +
+         sizeof(unsigned short) * (chunk + 2);
+}
+constexpr int kLoop1dResort32 = 128;
+
+template <int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    k32_loop1d(Rate32 P, Update32 U, double bn, double b0, int chunk, int nsteps) {
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  extern __shared__ __align__(16) unsigned char lraw[];
+  Loop1dSmem32 &sm = *reinterpret_cast<Loop1dSmem32 *>(lraw);
+  const int MX = chunk + 2;
+  float4 *Hs = reinterpret_cast<float4 *>(lraw + sizeof(Loop1dSmem32));
+  float4 *Ls = Hs + chunk + 4, *Vs = Ls + chunk, *Ks = Vs + MX, *Ms = Ks + MX, *Fs = Ms + MX,
+         *Ds = Fs + chunk + 1;
+  float2 *Es = reinterpret_cast<float2 *>(Ds + chunk);
+  float *Qs = reinterpret_cast<float *>(Es + MX);
+  unsigned short *order = reinterpret_cast<unsigned short *>(Qs + MX);
+  StepState32 *st = P.st;
+  if (st->halt) return;
+  const int n = P.nx, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nw = (int)blockDim.x >> 5, nt = (int)blockDim.x - 32;   // the last warp sums
+  const bool worker = t < nt;
+  const int rank = (int)cluster.block_rank(), nb = (int)cluster.num_blocks();
+  const int i0 = rank * chunk, m = max(0, min(chunk, n - i0));
+  const int ng = (n + 31) / 32;
+  const unsigned bar_a = shared_addr(&sm.bar_a), bar_b = shared_addr(&sm.bar_b);
+  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + (m > 0 ? sizeof(sm.halo) : 0u);
+  double dt = st->dt, time = st->time, xdotmax = st->xdotmax;
+  long long step = st->step;
+  int to_check = U.oob_interval > 0 ? U.oob_interval - (int)(step % U.oob_interval) : -1;
+  unsigned flags = 0;
+  bool halt = false, stalled = false, checked = false;
+
+  auto misfit = [&](const float4 &h, const float4 &l) {
+    float acc = fmaf(h.x + l.x, U.lvec[0], 0.f);
+    acc = fmaf(h.y + l.y, U.lvec[1], acc);
+    acc = fmaf(h.z + l.z, U.lvec[2], acc);
+    return fmaf(h.w + l.w, U.lvec[3], acc);
+  };
+  // The halo entry this thread keeps current: entry h of block b holds the
+  // point at Hs index hsrc of this block (none: hsrc < 0).  4 * nb <= threads.
+  int hsrc = -1;
+  unsigned hdst = 0, hbar = 0;
+  {
+    const int b = t >> 2, h = t & 3;
+    const int bm = b < nb ? max(0, min(chunk, n - b * chunk)) : 0;
+    if (bm > 0 && m > 0) {
+      const int src = wrap_any(b * chunk + (h < 2 ? h - 2 : bm + h - 2), n) - i0;
+      if (src >= 0 && src < m) {
+        hsrc = src + 2;
+        hdst = rank_addr(shared_addr(sm.halo[h]), b);
+        hbar = rank_addr(bar_b, b);
+      }
+    }
+  }
+  auto send_b = [&]() {
+    for (int g = warp; 32 * g < m; g += nw)
+      if (lane < nb)
+        send2(rank_addr(shared_addr(&sm.sums[i0 / 32 + g]), lane), rank_addr(bar_b, lane),
+              (unsigned long long)__double_as_longlong(sm.own[g]), sm.own_flags[g]);
+    if (hsrc >= 0) {
+      const ulonglong2 h = *reinterpret_cast<const ulonglong2 *>(Hs + hsrc);
+      send2(hdst, hbar, h.x, h.y);
+      send2(hdst + 16, hbar, __float_as_uint(Qs[hsrc - 1]), 0);
+    }
+  };
+  // 32 points from p0 (s: this lane's misfit): their sum and flags
+  auto keep_group = [&](float s, int p0, unsigned f) {
+    const double v = P.sp ? group_sum(p0 + lane < m ? (double)s : 0.0) : 0.0;
+    const unsigned any = __reduce_or_sync(0xffffffffu, f);
+    if (lane == 0) {
+      sm.own[p0 >> 5] = v;
+      sm.own_flags[p0 >> 5] = any;
+    }
+  };
+  // positions in the order of their cells (a counting sort over cell_hash_u)
+  auto sort_cells = [&]() {
+    for (int b = t; b < 256; b += (int)blockDim.x) sm.bins[b] = 0;
+    __syncthreads();
+    auto key = [&](int pos) {
+      const float4 h = Hs[pos + 1];
+      const float d[S] = {h.x, h.y, h.z, h.w};
+      float u[S];
+#pragma unroll
+      for (int c = 0; c < S; ++c) u[c] = fmaf(d[c], P.T.inv_step_f, P.T.fb[c]) + (float)P.T.ib[c];
+      return cell_hash_u(u);
+    };
+    for (int pos = t; pos < m + 2; pos += (int)blockDim.x) atomicAdd(&sm.bins[key(pos)], 1);
+    __syncthreads();
+    if (warp == 0) scan_bins256(sm.bins, lane);
+    __syncthreads();
+    for (int pos = t; pos < m + 2; pos += (int)blockDim.x)
+      order[atomicAdd(&sm.bins[key(pos)], 1)] = (unsigned short)pos;
+    __syncthreads();
+  };
+
+  if (t == 0) {
+    mbar_init(bar_a);
+    mbar_init(bar_b);
+  }
+  for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+    const int p = p0 + lane;
+    float s = 0.f;
+    if (p < m) {
+      const float4 h = U.hi[i0 + p], l = U.lo[i0 + p];
+      Hs[p + 2] = h;
+      Ls[p] = l;
+      s = misfit(h, l);
+      Qs[p + 1] = s;
+    }
+    keep_group(s, p0, 0);
+  }
+  __syncthreads();
+  cluster.sync();                        // every block has started and set up its barriers
+  if (t == 0) mbar_expect(bar_b, bytes_b);
+  send_b();
+
+  for (int k = 0; k <= nsteps; ++k) {
+    // B of the step before (k = 0: the state at the launch)
+    stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
+    if (t < 4 && m > 0) {                // halo entries into the chunk's rows
+      const int p = t < 2 ? t : m + t;
+      *reinterpret_cast<ulonglong2 *>(Hs + p) = sm.halo[t][0];
+      if (t == 1 || t == 2) Qs[p - 1] = __uint_as_float((unsigned)sm.halo[t][1].x);
+    }
+    if (checked) {
+      unsigned f = 0;
+      for (int g = lane; g < ng; g += 32) f |= (unsigned)sm.sums[g].y;
+      f = __reduce_or_sync(0xffffffffu, f);
+      flags |= f;
+      if (f & (PF5D_FLAG_NONFINITE | PF5D_FLAG_OOB_HARD)) halt = true;
+    }
+    if (__syncthreads_or(stalled)) stalled = true;
+    if (halt || stalled || k == nsteps) break;
+    if (m > 0 && k % kLoop1dResort32 == 0) sort_cells();
+    unsigned nn = 0;
+    if (worker) {
+      if (m > 0)
+        for (int w = t; w < m + 2; w += nt) {
+          const int pos = order[w];
+          const float4 h = Hs[pos + 1], hp = Hs[pos + 2], hm = Hs[pos];
+          const float d[S] = {h.x, h.y, h.z, h.w};
+          const double sd = dsum32(d);
+          float v[NP];
+          interp32(P, d, sd, nullptr, nullptr, v, &nn);
+          const float np[S] = {hp.x, hp.y, hp.z, hp.w}, nm[S] = {hm.x, hm.y, hm.z, hm.w};
+          float lk[S];
+#pragma unroll
+          for (int c = 0; c < S; ++c) {
+            const float nb2[2] = {np[c], nm[c]};
+            lk[c] = -lap32<2>(nb2, d[c], P.inv_dx2) * P.kappa[c];
+          }
+          Vs[pos] = make_float4(v[0], v[1], v[2], v[3]);
+          Ks[pos] = make_float4(lk[0], lk[1], lk[2], lk[3]);
+          Ms[pos] = make_float4(v[5], v[6], v[7], v[8]);
+          Es[pos] = make_float2(v[4], (float)(P.c_fe - sd));
+        }
+    } else {
+      if (lane == 0) {
+        mbar_expect(bar_a, bytes_a);
+        mbar_expect(bar_b, bytes_b);
+      }
+      if (P.sp) {
+        double total = 0.0;
+        for (int g = lane; g < ng; g += 32)
+          total = total + __longlong_as_double((long long)sm.sums[g].x);
+        total = group_sum(total);
+        if (lane == 0) sm.mean = total / (double)n;
+      }
+    }
+    __syncthreads();
+    // face i lies between mu/M positions i and i+1 (hi positions i+1, i+2)
+    if (m > 0) {
+      const double mean = P.sp ? sm.mean : 0.0;
+      auto mu_at = [&](int q) {
+        const float spv = P.sp ? (float)(bn * ((double)Qs[q] - mean) + b0 * mean) : 0.f;
+        const float4 v = Vs[q], k4 = Ks[q];
+        return make_float4(v.x + fmaf(spv, P.lvec[0], k4.x), v.y + fmaf(spv, P.lvec[1], k4.y),
+                           v.z + fmaf(spv, P.lvec[2], k4.z), v.w + fmaf(spv, P.lvec[3], k4.w));
+      };
+      for (int i = t; i < m + 1; i += (int)blockDim.x)
+        Fs[i] = face_flux32(P, Hs[i + 1], mu_at(i), Ms[i], Es[i], Hs[i + 2], mu_at(i + 1), Ms[i + 1],
+                            Es[i + 1]);
+    }
+    __syncthreads();
+    float vmax32 = 0.f;
+    for (int p = t; p < m; p += (int)blockDim.x) {
+      const float4 a = Fs[p + 1], b = Fs[p];
+      const float4 d = make_float4((a.x - b.x) * P.flux_scale, (a.y - b.y) * P.flux_scale,
+                                   (a.z - b.z) * P.flux_scale, (a.w - b.w) * P.flux_scale);
+      Ds[p] = d;
+      vmax32 = fmaxf(vmax32, fabsf(d.x));
+      vmax32 = fmaxf(vmax32, fabsf(d.y));
+      vmax32 = fmaxf(vmax32, fabsf(d.z));
+      vmax32 = fmaxf(vmax32, fabsf(d.w));
+    }
+    // non-negative floats are ordered as their bits
+    vmax32 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(vmax32)));
+    nn = __reduce_or_sync(0xffffffffu, nn);
+    if (lane < nb)
+      send2(rank_addr(shared_addr(&sm.max[rank * nw + warp]), lane), rank_addr(bar_a, lane),
+            __float_as_uint(vmax32), nn);
+    stalled = stalled || !mbar_wait(bar_a, (unsigned)k & 1u);       // A
+    unsigned gbits = 0;
+    nn = 0;
+    for (int i = lane; i < nb * nw; i += 32) {
+      gbits = max(gbits, (unsigned)sm.max[i].x);
+      nn |= (unsigned)sm.max[i].y;
+    }
+    const double gmax = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, gbits));
+    nn = __reduce_or_sync(0xffffffffu, nn);
+    flags |= nn;
+    if (nn & kNNErrorFlags) {            // the same in every block: stop before the update
+      halt = true;
+      break;
+    }
+    if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
+    time = time + dt;
+    xdotmax = gmax;
+    step = step + 1;
+    checked = --to_check == 0;
+    if (checked) to_check = U.oob_interval;
+    const float dtf = (float)dt;
+    for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+      const int p = p0 + lane;
+      unsigned fo = 0;
+      float s = 0.f;
+      if (p < m) {
+        const float4 H = Hs[p + 2], L = Ls[p], R = Ds[p];
+        float h[S] = {H.x, H.y, H.z, H.w}, l[S] = {L.x, L.y, L.z, L.w};
+        const float r[S] = {R.x, R.y, R.z, R.w};
+        double dd[S];
+        update_point32(U, dtf, r, h, l, dd);
+        const float4 hn = make_float4(h[0], h[1], h[2], h[3]), ln = make_float4(l[0], l[1], l[2], l[3]);
+        Hs[p + 2] = hn;
+        Ls[p] = ln;
+        s = misfit(hn, ln);
+        Qs[p + 1] = s;
+        if (checked) {
+          double x[S];
+#pragma unroll
+          for (int c = 0; c < S; ++c) x[c] = U.x0[c] + dd[c];
+          fo = oob_flags_x(x);
+        }
+      }
+      keep_group(s, p0, fo);
+    }
+    __syncthreads();
+    send_b();
+  }
+
+  if (!stalled)
+    for (int p = t; p < m; p += (int)blockDim.x) {
+      U.hi[i0 + p] = Hs[p + 2];
+      U.lo[i0 + p] = Ls[p];
+      P.dX[i0 + p] = Ds[p];
+      if (U.s) U.s[i0 + p] = Qs[p + 1];
+    }
+  if (stalled && t == 0) {
+    atomicOr(&st->flags, PF5D_FLAG_STALLED);
+    atomicExch(&st->halt, 1u);
+  } else if (rank == 0 && t == 0) {
+    st->dt = dt;
+    st->time = time;
+    st->xdotmax = xdotmax;
+    st->step = step;
+    if (flags) atomicOr(&st->flags, flags);
+    if (halt) atomicExch(&st->halt, 1u);
+  }
+  cluster.sync();                        // no block leaves while another may still send to it
 }
 
 __global__ void k32_bmul(cufftComplex *__restrict__ k, const float *__restrict__ bk, int64_t nk,
@@ -882,6 +1188,8 @@ struct Stepper32 {
   ColPass2D colp;                // 2D elastic term: row transforms + one column kernel
   bool use_colpass = false;
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
+  bool use_loop1d = false;       // 1D steps by k32_loop1d
+  Loop1dShape loop;
   int64_t shape[3] = {1, 1, 1};
   int64_t npts = 0, nk = 0;
   float4 *hi = nullptr, *lo = nullptr, *dX = nullptr;
@@ -1034,6 +1342,13 @@ static pf5d_status graph32(Stepper32 *h, int64_t n, cudaGraphExec_t *out) {
   return PF5D_OK;
 }
 
+// The step loop of a 1D solve (255 registers a thread in small blocks).
+using Loop1dKernel32 = void (*)(Rate32, Update32, double, double, int, int);
+static Loop1dKernel32 loop1d_kernel32(const Stepper32 *h) {
+  return h->loop.threads <= kLoop1dThreads / 2 ? k32_loop1d<kLoop1dThreads / 2>
+                                               : k32_loop1d<kLoop1dThreads>;
+}
+
 static void drop_graphs(Stepper32 *h) {
   for (auto &kv : h->graphs) cudaGraphExecDestroy(kv.second);
   h->graphs.clear();
@@ -1176,6 +1491,11 @@ pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void
   U.oob_interval = desc->oob_interval;
   pf5d_status st = configure32(h, 0);
   if (st != PF5D_OK) return fail(st);
+  if (desc->dim == 1 && npts <= kLoop1dMax && (!desc->elastic || h->closed1d))
+    for (int blocks = kLoop1dBlocks; blocks >= 8 && !h->use_loop1d; blocks /= 2) {
+      h->loop = loop1d_shape(npts, blocks);
+      h->use_loop1d = cluster_fits(loop1d_kernel32(h), h->loop, loop1d_smem32(h->loop.chunk));
+    }
   if ((st = s32_reset(h, X_init, desc->dt0, 0.0, stream)) != PF5D_OK) return fail(st);
   *out = h;
   return PF5D_OK;
@@ -1197,6 +1517,15 @@ pf5d_status s32_reset(Stepper32 *h, const double *X, double dt, double time, voi
 
 pf5d_status s32_advance(Stepper32 *h, int64_t nsteps, void *stream) {
   cudaStream_t s = as_stream(stream);
+  if (h->use_loop1d) {
+    const size_t sm = loop1d_smem32(h->loop.chunk);
+    for (; nsteps > 0; nsteps -= kLoop1dSteps) {
+      const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);
+      PF5D_CUDA(launch_cluster(loop1d_kernel32(h), h->loop, sm, s, h->rp, h->up, h->bn, h->b0,
+                               h->loop.chunk, n));
+    }
+    return PF5D_OK;
+  }
   while (nsteps > 0) {
     const int64_t n = nsteps < kGraphSteps32 ? nsteps : kGraphSteps32;
     cudaGraphExec_t g = nullptr;
@@ -1307,6 +1636,7 @@ const char *s32_rate_kernels(Stepper32 *h) {
 }
 
 int32_t s32_launches_per_step(const Stepper32 *h) {
+  if (h->use_loop1d) return 1;
   const bool split = h->d.dim >= 2 && variants32()[h->variant].split;
   return (split ? 4 : 3) + (h->d.elastic ? 1 : 0);   // rate (+chem), dt, update (+ B(k))
 }

@@ -1427,22 +1427,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     };
     for (int pos = t; pos < m + 2; pos += (int)blockDim.x) atomicAdd(&sm.bins[key(pos)], 1);
     __syncthreads();
-    if (warp == 0) {
-      int v[8], sum = 0;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        v[j] = sum;
-        sum += sm.bins[8 * lane + j];
-      }
-      int before = sum;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int u = __shfl_up_sync(0xffffffffu, before, o);
-        if (lane >= o) before += u;
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) sm.bins[8 * lane + j] = before - sum + v[j];
-    }
+    if (warp == 0) scan_bins256(sm.bins, lane);
     __syncthreads();
     for (int pos = t; pos < m + 2; pos += (int)blockDim.x)
       order[atomicAdd(&sm.bins[key(pos)], 1)] = (unsigned short)pos;
