@@ -19,6 +19,16 @@ constexpr int S = 4;    // independent components
 constexpr int NM = 5;   // mobilities (Fe first)
 constexpr int NP = 9;   // table props: mu1..mu4, M_Fe, M1..M4
 
+// Row r of point g in a buffer of NP values per point (mu_1..4, M_Fe, M_1..4):
+// rows 0..7 as four arrays of pairs, row 8 alone, so that a point's values move
+// as four 16-byte accesses and one of 8, each coalesced over neighbours.
+__host__ __device__ __forceinline__ int64_t mm_index(int64_t npts, int r, int64_t g) {
+  return r < 8 ? (int64_t)(r >> 1) * 2 * npts + 2 * g + (r & 1) : 8 * npts + g;
+}
+__device__ __forceinline__ double mm_row(const double *mm, int64_t npts, int r, int64_t g) {
+  return mm[mm_index(npts, r, g)];
+}
+
 // Periodic neighbour indices (phasefield5d/solver/operators.py:45-46 pattern).
 __device__ __forceinline__ int64_t wrap_p(int64_t i, int64_t n) { return i + 1 < n ? i + 1 : 0; }
 __device__ __forceinline__ int64_t wrap_m(int64_t i, int64_t n) { return i - 1 >= 0 ? i - 1 : n - 1; }
@@ -396,6 +406,35 @@ __device__ __forceinline__ void face_flux(const double Xc[S], const double Mc[NM
   }
 }
 
+// Eight times face_flux's J, bit for bit (short of underflow): factors of two
+// commute with rounding, so the means of the two points are taken as their
+// sums, and what has to be added at one scale is brought there inside an fma
+// whose product is exact.  56 operations instead of 68 (FP64 issue is what
+// bounds the flux kernels); a divergence of these is scaled by inv_dx / 8.
+__device__ __forceinline__ void face_flux8(const double Xc[S], const double Mc[NM],
+                                           const double Xn[S], const double Mn[NM],
+                                           const double g[S], double J8[S]) {
+  double x2[S], m2[NM], p4[S];               // 2 xm, 2 mm, 4 xm mm dk
+#pragma unroll
+  for (int a = 0; a < S; ++a) x2[a] = Xc[a] + Xn[a];
+#pragma unroll
+  for (int a = 0; a < NM; ++a) m2[a] = Mc[a] + Mn[a];
+  double sum2 = x2[0], dot2 = x2[0] * g[0], sum_wk4 = 0.0;
+#pragma unroll
+  for (int a = 1; a < S; ++a) {
+    sum2 = sum2 + x2[a];
+    dot2 = dot2 + x2[a] * g[a];
+  }
+  const double w2 = fma(-0.5, sum2, 1.0) * m2[0];
+#pragma unroll
+  for (int k = 0; k < S; ++k) {
+    p4[k] = x2[k] * m2[1 + k] * fma(-0.5, dot2, g[k]);
+    sum_wk4 = k == 0 ? p4[0] : sum_wk4 + p4[k];
+  }
+#pragma unroll
+  for (int a = 0; a < S; ++a) J8[a] = fma(2.0, p4[a], w2 * x2[a] * dot2) - x2[a] * sum_wk4;
+}
+
 // apply_adaptive_time (phasefield5d/solver/system.py:90-112); Python's min()
 // keeps its first argument unless a later one is strictly smaller, and
 // np.clip is minimum(maximum(a, lo), hi).
@@ -516,5 +555,12 @@ __device__ __forceinline__ int block_exclusive_scan(int *bins, int *wsum, int ti
 // kernel was launched with programmatic stream serialization; a no-op
 // otherwise.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// p as known only after pdl_wait, for loads in plain asm: they can then be
+// scheduled freely, but not before the wait.
+__device__ __forceinline__ const double *after_wait(const double *p) {
+  asm volatile("mov.b64 %0, %0;" : "+l"(p)::"memory");
+  return p;
+}
 
 }  // namespace pf5d

@@ -72,7 +72,7 @@ __device__ __forceinline__ void diag_block_row(double v[K], const bool is_max[K]
 // total flux sum over points and axes of (flux_p - flux_m), with
 // flux_p / flux_m the face fluxes of each point towards its +/- neighbour
 // from the forward / backward mu gradients (operators.py:88-123 gradients,
-// fluxes.py:6-125 compute_fluxes).  mm: mu_1..4 then M_Fe, M_1..4, SoA.
+// fluxes.py:6-125 compute_fluxes).  mm: mu_1..4 then M_Fe, M_1..4 (mm_row).
 __global__ void __launch_bounds__(kDiagThreads) k_diag_pre(DiagGeom G, const double *X,
                                                            const double *dX, const double *mm,
                                                            double *partial) {
@@ -92,24 +92,24 @@ __global__ void __launch_bounds__(kDiagThreads) k_diag_pre(DiagGeom G, const dou
     for (int c = 0; c < S; ++c) {
       v[c] = v[c] + d[c];
       v[S + c] = fmax(v[S + c], fabs(d[c]));
-      muc[c] = mm[c * G.npts + g];
+      muc[c] = mm_row(mm, G.npts, c, g);
     }
 #pragma unroll
-    for (int c = 0; c < NM; ++c) mc[c] = mm[(S + c) * G.npts + g];
+    for (int c = 0; c < NM; ++c) mc[c] = mm_row(mm, G.npts, S + c, g);
     for (int a = 0; a < G.dim; ++a) {
       const int64_t gp = diag_neighbour(G, g, a, +1), gm = diag_neighbour(G, g, a, -1);
       double xn[S], mn[NM], grad[S], fp[S], fm[S];
       diag_load4(X, gp, xn);
 #pragma unroll
-      for (int c = 0; c < NM; ++c) mn[c] = mm[(S + c) * G.npts + gp];
+      for (int c = 0; c < NM; ++c) mn[c] = mm_row(mm, G.npts, S + c, gp);
 #pragma unroll
-      for (int c = 0; c < S; ++c) grad[c] = (mm[c * G.npts + gp] - muc[c]) * G.inv_dx;
+      for (int c = 0; c < S; ++c) grad[c] = (mm_row(mm, G.npts, c, gp) - muc[c]) * G.inv_dx;
       face_flux(xc, mc, xn, mn, grad, fp);
       diag_load4(X, gm, xn);
 #pragma unroll
-      for (int c = 0; c < NM; ++c) mn[c] = mm[(S + c) * G.npts + gm];
+      for (int c = 0; c < NM; ++c) mn[c] = mm_row(mm, G.npts, S + c, gm);
 #pragma unroll
-      for (int c = 0; c < S; ++c) grad[c] = (muc[c] - mm[c * G.npts + gm]) * G.inv_dx;
+      for (int c = 0; c < S; ++c) grad[c] = (muc[c] - mm_row(mm, G.npts, c, gm)) * G.inv_dx;
       face_flux(xc, mc, xn, mn, grad, fm);
 #pragma unroll
       for (int c = 0; c < S; ++c) v[2 * S + c] = v[2 * S + c] + (fp[c] - fm[c]);

@@ -219,7 +219,7 @@ __device__ __forceinline__ void gather_rest(G &g, const Table &T, int tid, unsig
 
 // The four components of a point; wide: the field is 32-byte aligned, so they
 // are one 256-bit load (half the L1 wavefronts of two 16-byte ones, whose
-// lanes each touch half of every line).
+// lanes each touch half of every line).  p derives from an after_wait pointer.
 __device__ __forceinline__ void load_comp4(const double *p, bool wide, double v[S]) {
   if (wide) {
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"

@@ -1552,14 +1552,14 @@ pf5d_status s32_state(Stepper32 *h, pf5d_step_state *out, void *stream) {
 }
 
 // FP64 copies for the save-step reductions: dX/dt (4 per point) and mu/M
-// (SoA, 9 rows), from the FP32 buffers.
+// (mm_row), from the FP32 buffers.
 __global__ void k32_widen(const float *__restrict__ src, int64_t n, double *__restrict__ dst) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     dst[i] = (double)src[i];
 }
 
-// FP64 mu/M rows (SoA, 9 rows: mu_1..4, M_Fe, M_1..4) from the split buffers.
+// FP64 mu/M rows (mm_row: mu_1..4, M_Fe, M_1..4) from the split buffers.
 __global__ void k32_widen_mm(Rate32 P, double *__restrict__ dst) {
   const int64_t n = P.npts;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
@@ -1568,7 +1568,7 @@ __global__ void k32_widen_mm(Rate32 P, double *__restrict__ dst) {
     const float2 f = P.mm_f[i];
     const float v[NP] = {mu.x, mu.y, mu.z, mu.w, f.x, m.x, m.y, m.z, m.w};
 #pragma unroll
-    for (int r = 0; r < NP; ++r) dst[r * n + i] = (double)v[r];
+    for (int r = 0; r < NP; ++r) dst[mm_index(n, r, i)] = (double)v[r];
   }
 }
 

@@ -17,9 +17,8 @@
 //        - dX/dt written once; each block stores its max |dX/dt| in its
 //          own slot (plain store).
 //      Variants (autotuned, all computing the same values): tile shapes,
-//      a split form (k_chem writes mu/M once per point, the tile kernel
-//      reads them back), table-cell sort, shared table window, per-point
-//      faces.
+//      a split form (k_chem writes mu/M once per point, k_flux reads them
+//      back), table-cell sort, shared table window, per-point faces.
 //   5. k_dt_finish (one block): max over the slots, the adaptive dt rule,
 //      dt / time / step advanced on the device.
 //   6. k_update_step: X += dX*dt; clamp; s for the next step; every
@@ -33,8 +32,6 @@
 #include <cstring>
 #include <map>
 #include <vector>
-
-#include <cuda_pipeline_primitives.h>
 
 #include "pf5d_cluster.cuh"
 #include "pf5d_device.cuh"
@@ -64,10 +61,11 @@ struct RateParams {
   Table T;
   Vec4 kappa, lvec;
   double inv_dx, inv_dx2;
+  double inv_dx8;              // inv_dx / 8, of a divergence of face_flux8's
   double ctld, t_cfl, lower, upper, factor;
   int adaptive;
   StepState *st;
-  double *mm;                  // split rate: mu_1..4, M_Fe, M_1..4 per point, SoA [NP][npts]
+  double *mm;                  // split rate: mu_1..4, M_Fe, M_1..4 per point (mm_row)
   int64_t npts;
   double *partial;             // per-block max |dX/dt| of the last rate launch
 };
@@ -347,25 +345,8 @@ __device__ __forceinline__ void mu_plane64(const RateParams &P, const double *Xm
   }
 }
 
-// mu/M of one plane (tile + 1-cell halo, or tile only) read from the split
-// buffer P.mm (written by k_chem) into dst, in mu_plane64's layout.
-template <int TX, int TY, int NTH = TX * TY>
-__device__ __forceinline__ void load_mu_plane(const RateParams &P, int64_t zoff, const int *wx,
-                                              const int *wy, bool interior_only, double *dst,
-                                              int tid) {
-  using G = PlaneGeom<TX, TY, NTH>;
-  for (int pos = tid; pos < G::PM; pos += G::NT) {
-    const int my = pos / G::MX, mx = pos - my * G::MX;
-    const bool ex = (mx == 0 || mx == G::MX - 1), ey = (my == 0 || my == G::MY - 1);
-    if (interior_only ? (ex || ey) : (ex && ey)) continue;
-    const double *src = P.mm + zoff + (int64_t)wy[my + 1] * P.nx + wx[mx + 1];
-#pragma unroll
-    for (int c = 0; c < NP; ++c) dst[c * G::PM + pos] = __ldg(src + c * P.npts);
-  }
-}
-
 // Split rate evaluation, first kernel: chemical potential and mobility at
-// every point of a field into P.mm (SoA rows), each point once.  The table
+// every point of a field into P.mm, each point once.  The table
 // values come first (pf5d_gather.cuh), then each thread takes its own points
 // in order: Laplacian (operators.py:49-76: +axis0, -axis0, +axis1, ...), then
 // mu = v - lap*kappa (+ s' * l).  A block's points are 512 in a row (1D), 32
@@ -398,6 +379,7 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
   __shared__ ChemSmem g;
   pdl_wait();
   if (P.st->halt) return;
+  const double *X = after_wait(P.X);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int bx = blockIdx.x * G::BX, by = blockIdx.y * G::BY, bz = blockIdx.z * G::BZ;
   const int64_t plane = (int64_t)P.ny * P.nx;
@@ -414,7 +396,7 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
     const int x = px(j, lane, w), y = py(j, w), z = pz(j);
     const bool valid = x < P.nx && y < P.ny && z < P.nz;
     double xc[S] = {0.0, 0.0, 0.0, 0.0};
-    if (valid) load_comp4(P.X + 4 * (z * plane + (int64_t)y * P.nx + x), wide, xc);
+    if (valid) load_comp4(X + 4 * (z * plane + (int64_t)y * P.nx + x), wide, xc);
     kr[j] = gather_add(g, P.T, valid, xc, j * NT + tid);
   }
   const int nitems = gather_sort(g, kr, tid);
@@ -422,13 +404,13 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
   unsigned flags = 0;
   gather_rest<VEC>(g, P.T, tid, &flags, [&](int q, double x[S]) {
     const int j = q / NT, v = (q / 32) % (NT / 32);
-    load_comp4(P.X + 4 * (pz(j) * plane + (int64_t)py(j, v) * P.nx + px(j, q & 31, v)), wide, x);
+    load_comp4(X + 4 * (pz(j) * plane + (int64_t)py(j, v) * P.nx + px(j, q & 31, v)), wide, x);
   });
   raise_rate_flags(P.st, flags);
   if (kr[0] == kNoKey) return;                  // none of this thread's points is in the field
   double below[S], xc[S], above[S];             // along the marching axis (y in 2D, z in 3D)
   const int x0 = px(0, lane, w), y0 = py(0, w), z0 = pz(0);
-  auto at = [&](int z, int y, int x) { return P.X + 4 * (z * plane + (int64_t)y * P.nx + x); };
+  auto at = [&](int z, int y, int x) { return X + 4 * (z * plane + (int64_t)y * P.nx + x); };
   if (DIM == 2) load_comp4(at(0, y0 == 0 ? P.ny - 1 : y0 - 1, x0), wide, below);
   if (DIM == 3) load_comp4(at(z0 == 0 ? P.nz - 1 : z0 - 1, y0, x0), wide, below);
   load_comp4(at(z0, y0, x0), wide, xc);
@@ -464,10 +446,12 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
       const double lk = lap[c] * P.kappa.v[c];
       double m = v[c] - lk;
       if (P.sp) m = m + spv * P.lvec.v[c];
-      P.mm[c * P.npts + gi] = m;
+      v[c] = m;
     }
+    double2 *o = reinterpret_cast<double2 *>(P.mm) + gi;
 #pragma unroll
-    for (int c = 0; c < NM; ++c) P.mm[(S + c) * P.npts + gi] = v[S + c];
+    for (int r = 0; r < 4; ++r) o[r * P.npts] = make_double2(v[2 * r], v[2 * r + 1]);
+    P.mm[8 * P.npts + gi] = v[8];
     if (DIM != 1) {
 #pragma unroll
       for (int c = 0; c < S; ++c) {
@@ -539,7 +523,7 @@ __device__ __forceinline__ void face_between(const double *XL, const double *ML,
     Mc[c] = ML[(S + c) * PM + ql];
     Mn[c] = MH[(S + c) * PM + qh];
   }
-  face_flux(Xc, Mc, Xn, Mn, g, J);
+  face_flux8(Xc, Mc, Xn, Mn, g, J);
 }
 
 // All x- and y-faces of one plane tile into Fx / Fy (flat loop: every
@@ -594,8 +578,8 @@ __device__ __forceinline__ void load_plane(const double *__restrict__ X, int64_t
 // A block is NTH threads in one dimension (at least one per tile point; with
 // NTH >= the mu/M position count every position takes one pass).  SORT:
 // mu/M positions evaluated in table-cell order.
-template <int TX, int TY, int MINB, bool VEC, bool WIN, bool SPLIT = false, int NTH = TX * TY,
-          int SORT = 0, bool PERPOINT = false>
+template <int TX, int TY, int MINB, bool VEC, bool WIN, int NTH = TX * TY, int SORT = 0,
+          bool PERPOINT = false>
 __global__ void __launch_bounds__(NTH, MINB) k_rate_tile2d(RateParams P) {
   using G = PlaneGeom<TX, TY, NTH>;
   static_assert(NTH >= TX * TY && NTH % 32 == 0, "one thread per tile point at least");
@@ -630,12 +614,9 @@ __global__ void __launch_bounds__(NTH, MINB) k_rate_tile2d(RateParams P) {
   __syncthreads();
   load_plane<TX, TY, NTH>(P.X, 0, wx, wy, P.nx, Xs, tid);
   __syncthreads();
-  if constexpr (SPLIT)
-    load_mu_plane<TX, TY, NTH>(P, 0, wx, wy, false, Ms, tid);
-  else
-    mu_plane64<TX, TY, 2, VEC, WIN, NTH, SORT>(P, nullptr, Xs, nullptr, Ms, 0, wx, wy, false,
-                                               reinterpret_cast<double2 *>(Fx), win_lo, &flags,
-                                               tid, ss);
+  mu_plane64<TX, TY, 2, VEC, WIN, NTH, SORT>(P, nullptr, Xs, nullptr, Ms, 0, wx, wy, false,
+                                             reinterpret_cast<double2 *>(Fx), win_lo, &flags, tid,
+                                             ss);
   __syncthreads();
   double jyp[S], jym[S], jxp[S], jxm[S];
   const bool mine = tid < TX * TY && x0 + tx < P.nx && y0 + ty < P.ny;
@@ -670,7 +651,7 @@ __global__ void __launch_bounds__(NTH, MINB) k_rate_tile2d(RateParams P) {
       double a = jyp[c] - jym[c];
       a = a + jxp[c];
       a = a - jxm[c];
-      out[c] = a * P.inv_dx;
+      out[c] = a * P.inv_dx8;
       const double v = fabs(out[c]);
       if (v > vmax) vmax = v;
     }
@@ -829,7 +810,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
           v = v - jym[c];
           v = v + jxp[c];
           v = v - jxm[c];
-          out[c] = v * P.inv_dx;
+          out[c] = v * P.inv_dx8;
           const double m = fabs(out[c]);
           if (m > vmax) vmax = m;
         }
@@ -856,7 +837,7 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
       for (int c = 0; c < S; ++c) {
         double v = a[c] + F[c * G::NFX + ty * (TX + 1) + tx + 1];
         v = v - F[c * G::NFX + ty * (TX + 1) + tx];
-        out[c] = v * P.inv_dx;
+        out[c] = v * P.inv_dx8;
         const double m = fabs(out[c]);
         if (m > vmax) vmax = m;
       }
@@ -871,191 +852,168 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
 }
 
 // ------------------------------------------------------------------------
-// Split rate evaluation, second kernel in 3D: faces and divergence of a
-// TY x TX plane tile marching along axis 0, from X and the mu/M rows that
-// k_chem wrote.  The X and mu/M of each plane (tile + 1-cell halo) go
-// through a three-plane ring in shared memory that cp.async fills two
-// planes ahead, so the loads of plane z+2 run under the faces of plane z.
-// Faces and the divergence sum in k_rate_march3d's order (fluxes.py:352-395:
-// axis 0, then 1, then 2), so the same bits.
+// Split rate evaluation, second kernel: faces and divergence from X and the
+// mu/M that k_chem wrote, without shared memory or barriers.  A warp takes 32
+// neighbouring columns and marches along axis 0 (2D: rows, 3D: planes); a
+// thread keeps its point's X, mu and M in registers, so
+//   * the face along the march is evaluated once and carried to the next row,
+//   * the face to the next column takes that column's values from the next
+//     lane, and its flux goes on to that lane: the outer lanes only serve
+//     their neighbours, and a warp finishes 30 columns,
+//   * in 3D the two faces along axis 1 read the rows above and below, which
+//     the block's other warps load too (4 warps, 4 rows).
+// The next row's loads are issued before the faces that do not need them.
+// Divergence in the reference's order: axis 0, then 1, then 2
+// (fluxes.py:349-395).
+//
+// Three-dimensional fields: bound by FP64 issue (52% of the pipe) and by the
+// latency of the loads that 12 warps per SM leave (DRAM 45%); the next plane
+// but one is prefetched into L2.  256^3: 0.76 ms as a 32x4 tile with a shared
+// cp.async ring and five faces per point, 0.63 here.  R = 2 rows per thread
+// take 3.5 faces per point instead of 4 but 204 registers (8 warps): 0.67.
+// Two-dimensional: 512^2 rate stage 39.1 us as one fused tile kernel (31%
+// halo recomputation, four faces per point), 29.8 split; 4 rows per warp keep
+// 16 warps per SM there, 2 rows are better below about 400^2, where they are
+// what fills the chip.
 // ------------------------------------------------------------------------
-template <int TX, int TY>
-struct Flux3Geom64 {
-  static constexpr int MX = TX + 2, MY = TY + 2, PM = MX * MY, NT = TX * TY;
-  static constexpr int NFX = TY * (TX + 1), NFY = (TY + 1) * TX;
-  static constexpr size_t slot = (size_t)(S + NP) * PM;          // doubles: X rows, then mu/M rows
-  static constexpr size_t smem(bool perpoint) {
-    return (3 * slot + (perpoint ? 0 : (size_t)S * (NFX + NFY)) + NT / 32) * sizeof(double) +
-           (MX + MY) * sizeof(int);
-  }
-};
+constexpr int kFluxThreads = 128, kFluxCols = 30;
 
-// X, mu and M of one position read out of a plane's rows (stride PM), and
-// the face flux between two such positions, lower -> upper: the operands
-// and operation order of face_between, so the same bits.
+// X, mu and M of one point
 struct Pt64 {
   double x[S], mu[S], m[NM];
 };
 
-template <int PM>
-__device__ __forceinline__ void load_pt64(const double *X, const double *M, int p, Pt64 &q) {
-#pragma unroll
-  for (int c = 0; c < S; ++c) {
-    q.x[c] = X[c * PM + p];
-    q.mu[c] = M[c * PM + p];
-  }
-#pragma unroll
-  for (int c = 0; c < NM; ++c) q.m[c] = M[(S + c) * PM + p];
+__device__ __forceinline__ void load_pt64(const RateParams &P, const double *X, int64_t g, bool wide,
+                                          Pt64 &q) {
+  load_comp4(X + 4 * g, wide, q.x);
+  const double2 *mm = reinterpret_cast<const double2 *>(P.mm) + g;
+  const double2 a = __ldg(mm), b = __ldg(mm + P.npts), c = __ldg(mm + 2 * P.npts),
+                d = __ldg(mm + 3 * P.npts);
+  q.mu[0] = a.x;
+  q.mu[1] = a.y;
+  q.mu[2] = b.x;
+  q.mu[3] = b.y;
+  q.m[0] = c.x;
+  q.m[1] = c.y;
+  q.m[2] = d.x;
+  q.m[3] = d.y;
+  q.m[4] = __ldg(P.mm + 8 * P.npts + g);
 }
 
+// The point's lines into L2.
+__device__ __forceinline__ void prefetch_pt64(const RateParams &P, const double *X, int64_t g) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(X + 4 * g));
+#pragma unroll
+  for (int r = 0; r < 4; ++r)
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(P.mm + 2 * (r * P.npts + g)));
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(P.mm + 8 * P.npts + g));
+}
+
+// Eight times the flux from point lo to its neighbour hi along an axis.
 __device__ __forceinline__ void face_pts64(const Pt64 &lo, const Pt64 &hi, double inv_dx,
-                                           double J[S]) {
+                                           double J8[S]) {
   double g[S];
 #pragma unroll
   for (int c = 0; c < S; ++c) g[c] = (hi.mu[c] - lo.mu[c]) * inv_dx;
-  face_flux(lo.x, lo.m, hi.x, hi.m, g, J);
+  face_flux8(lo.x, lo.m, hi.x, hi.m, g, J8);
 }
 
-template <int TX, int TY, int MINB, bool PERPOINT>
-__global__ void __launch_bounds__(TX * TY, MINB) k_flux3_64(RateParams P, int zc) {
-  using G = Flux3Geom64<TX, TY>;
+template <int DIM, int R, int MINB>
+__global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int rows) {
+  static_assert(DIM == 3 || R == 1, "rows per thread are of axis 1");
+  __shared__ double red[kFluxThreads / 32];
   pdl_wait();
   if (P.st->halt) return;
-  extern __shared__ double sm[];
-  double *ring = sm;                                         // [3][S + NP][PM]
-  double *Fx = ring + 3 * G::slot;                           // [S][NFX] (flat faces)
-  double *Fy = Fx + (PERPOINT ? 0 : S * G::NFX);             // [S][NFY]
-  double *red = Fy + (PERPOINT ? 0 : S * G::NFY);            // [NT/32]
-  int *wx = reinterpret_cast<int *>(red + G::NT / 32);
-  int *wy = wx + G::MX;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-  const int zb = blockIdx.z * zc;
-  const int ze = min(zb + zc, P.nz);
-  const int64_t plane = (int64_t)P.ny * P.nx;
-  for (int i = tid; i < G::MX + G::MY; i += G::NT) {
-    if (i < G::MX) wx[i] = wrap_any(x0 + i - 1, P.nx);
-    else wy[i - G::MX] = wrap_any(y0 + (i - G::MX) - 1, P.ny);
-  }
-  __syncthreads();
-  auto sX = [&](int z) { return ring + ((z - zb + 3) % 3) * G::slot; };
-  auto sM = [&](int z) { return sX(z) + S * G::PM; };
-  auto issue = [&](int z, bool interior_only) {
-    const int64_t zoff = (int64_t)wrap_any(z, P.nz) * plane;
-    double *x = sX(z), *m = sM(z);
-    for (int pos = tid; pos < G::PM; pos += G::NT) {
-      const int my = pos / G::MX, mx = pos - my * G::MX;
-      const bool ex = (mx == 0 || mx == G::MX - 1), ey = (my == 0 || my == G::MY - 1);
-      if (interior_only ? (ex || ey) : (ex && ey)) continue;
-      const int64_t g = zoff + (int64_t)wy[my] * P.nx + wx[mx];
-#pragma unroll
-      for (int c = 0; c < S; ++c) __pipeline_memcpy_async(x + c * G::PM + pos, P.X + 4 * g + c, 8);
-#pragma unroll
-      for (int r = 0; r < NP; ++r)
-        __pipeline_memcpy_async(m + r * G::PM + pos, P.mm + r * P.npts + g, 8);
-    }
-    __pipeline_commit();
-  };
-  auto face = [&](int zl, int pl, int zh, int ph, double J[S]) {
-    face_between<G::PM, G::PM>(sX(zl), sM(zl), pl, pl, sX(zh), sM(zh), ph, ph, P.inv_dx, J);
-  };
-  const int p = (ty + 1) * G::MX + (tx + 1);
-  const bool in_tile = (x0 + tx < P.nx) && (y0 + ty < P.ny);
-  issue(zb - 1, true);
-  issue(zb, false);
-  issue(zb + 1, false);
-  __pipeline_wait_prior(1);
-  __syncthreads();
-  // PERPOINT: this point's X/mu/M at plane z stay in registers (cur) and
-  // become the lower side of the next plane's axis-0 face.
-  Pt64 cur;
-  double Jm[S];
-  if constexpr (PERPOINT) {
-    Pt64 below;
-    load_pt64<G::PM>(sX(zb - 1), sM(zb - 1), p, below);
-    load_pt64<G::PM>(sX(zb), sM(zb), p, cur);
-    face_pts64(below, cur, P.inv_dx, Jm);
-  } else {
-    face(zb - 1, p, zb, p, Jm);
-  }
+  const double *X = after_wait(P.X);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int col = blockIdx.x * kFluxCols + lane - 1, x = wrap_any(col, P.nx);
+  // axis 0: the march, over [first, last); 3D: axis 1 is this warp's R rows
+  const int n0 = DIM == 3 ? P.nz : P.ny;
+  const int y = (blockIdx.y * 4 + w) * R;              // 3D
+  const int first = (DIM == 3 ? blockIdx.z : y) * rows, last = min(first + rows, n0);
+  const bool out_lane = lane > 0 && lane <= kFluxCols && col < P.nx;
+  const bool wide = ((uintptr_t)P.X & 31) == 0;
   double vmax = 0.0;
-  for (int z = zb; z < ze; ++z) {
-    __pipeline_wait_prior(0);          // plane z+1 copied (this thread's part)
-    __syncthreads();                   // ... and every thread's; the slot of z-1 is free
-    if (z + 2 <= ze) issue(z + 2, false);
-    double a[S];
-    double jyp[S], jym[S], jxp[S], jxm[S];
-    if constexpr (PERPOINT) {
-      // each point evaluates its four in-plane faces (each face by both of
-      // its cells, identical operands and order)
-      Pt64 up, nb;
-      load_pt64<G::PM>(sX(z + 1), sM(z + 1), p, up);
-      face_pts64(cur, up, P.inv_dx, a);
-      const double *Xz = sX(z), *Mz = sM(z);
-      load_pt64<G::PM>(Xz, Mz, p + G::MX, nb);
-      face_pts64(cur, nb, P.inv_dx, jyp);
-      load_pt64<G::PM>(Xz, Mz, p - G::MX, nb);
-      face_pts64(nb, cur, P.inv_dx, jym);
-      load_pt64<G::PM>(Xz, Mz, p + 1, nb);
-      face_pts64(cur, nb, P.inv_dx, jxp);
-      load_pt64<G::PM>(Xz, Mz, p - 1, nb);
-      face_pts64(nb, cur, P.inv_dx, jxm);
-      cur = up;
-    } else {
-      face(z, p, z + 1, p, a);
+  if (first < n0 && (DIM == 2 || y < P.ny)) {          // whole warps
+    auto at = [&](int i, int yy) {
+      return DIM == 3 ? ((int64_t)i * P.ny + yy) * P.nx + x : (int64_t)i * P.nx + x;
+    };
+    // a thread's rows past the field's last one repeat it and write nothing
+    auto row = [&](int r) { return DIM == 3 ? min(y + r, P.ny - 1) : 0; };
+    const int ym = y == 0 ? P.ny - 1 : y - 1, yp = y + R >= P.ny ? 0 : y + R;
+    Pt64 cur[R];
+    double Jm[R][S];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      Pt64 below;
+      load_pt64(P, X, at(first == 0 ? n0 - 1 : first - 1, row(r)), wide, below);
+      load_pt64(P, X, at(first, row(r)), wide, cur[r]);
+      face_pts64(below, cur[r], P.inv_dx, Jm[r]);
     }
+    for (int i = first; i < last; ++i) {
+      const int ip = i + 1 == n0 ? 0 : i + 1;
+      if (DIM == 3 && i + 2 < n0) {
 #pragma unroll
-    for (int c = 0; c < S; ++c) {
-      const double jz = a[c];
-      a[c] = jz - Jm[c];
-      Jm[c] = jz;
-    }
-    if constexpr (!PERPOINT) {
-      for (int f = tid; f < G::NFX + G::NFY; f += G::NT) {
-        double J[S];
-        if (f < G::NFX) {
-          const int fy = f / (TX + 1), fx = f - fy * (TX + 1);
-          const int pl = (fy + 1) * G::MX + fx;
-          face(z, pl, z, pl + 1, J);
+        for (int r = 0; r < R; ++r) prefetch_pt64(P, X, at(i + 2, row(r)));
+      }
+      double jym[S];
+      if (DIM == 3) {
+        Pt64 nb;
+        load_pt64(P, X, at(i, ym), wide, nb);
+        face_pts64(nb, cur[0], P.inv_dx, jym);
+      }
 #pragma unroll
-          for (int c = 0; c < S; ++c) Fx[c * G::NFX + f] = J[c];
-        } else {
-          const int f2 = f - G::NFX;
-          const int fy = f2 / TX, fx = f2 - fy * TX;
-          const int pl = fy * G::MX + (fx + 1);
-          face(z, pl, z, pl + G::MX, J);
+      for (int r = 0; r < R; ++r) {
+        Pt64 up, nb;
+        load_pt64(P, X, at(ip, row(r)), wide, up);
+        double jx[S], jl[S], jyp[S], jz[S], out[S];
 #pragma unroll
-          for (int c = 0; c < S; ++c) Fy[c * G::NFY + f2] = J[c];
+        for (int c = 0; c < S; ++c) {
+          nb.x[c] = __shfl_down_sync(0xffffffffu, cur[r].x[c], 1);
+          nb.mu[c] = __shfl_down_sync(0xffffffffu, cur[r].mu[c], 1);
         }
-      }
-      __syncthreads();
 #pragma unroll
-      for (int c = 0; c < S; ++c) {
-        jyp[c] = Fy[c * G::NFY + (ty + 1) * TX + tx];
-        jym[c] = Fy[c * G::NFY + ty * TX + tx];
-        jxp[c] = Fx[c * G::NFX + ty * (TX + 1) + tx + 1];
-        jxm[c] = Fx[c * G::NFX + ty * (TX + 1) + tx];
-      }
-    }
-    if (in_tile) {
-      double out[S];
+        for (int c = 0; c < NM; ++c) nb.m[c] = __shfl_down_sync(0xffffffffu, cur[r].m[c], 1);
+        face_pts64(cur[r], nb, P.inv_dx, jx);
 #pragma unroll
-      for (int c = 0; c < S; ++c) {
-        double v = a[c] + jyp[c];
-        v = v - jym[c];
-        v = v + jxp[c];
-        v = v - jxm[c];
-        out[c] = v * P.inv_dx;
-        const double m = fabs(out[c]);
-        if (m > vmax) vmax = m;
+        for (int c = 0; c < S; ++c) jl[c] = __shfl_up_sync(0xffffffffu, jx[c], 1);
+        if (DIM == 3) {
+          // the last row's upper neighbour (for a row that repeats: unused)
+          if (r == R - 1 || y + r + 1 >= P.ny) {
+            load_pt64(P, X, at(i, yp), wide, nb);
+            face_pts64(cur[r], nb, P.inv_dx, jyp);
+          } else {
+            face_pts64(cur[r], cur[r + 1 < R ? r + 1 : r], P.inv_dx, jyp);
+          }
+        }
+        face_pts64(cur[r], up, P.inv_dx, jz);
+#pragma unroll
+        for (int c = 0; c < S; ++c) {
+          double v = jz[c] - Jm[r][c];
+          if (DIM == 3) {
+            v = v + jyp[c];
+            v = v - jym[c];
+            jym[c] = jyp[c];
+          }
+          v = v + jx[c];
+          v = v - jl[c];
+          out[c] = v * P.inv_dx8;
+          Jm[r][c] = jz[c];
+        }
+        if (out_lane && (DIM == 2 || y + r < P.ny)) {
+#pragma unroll
+          for (int c = 0; c < S; ++c) {
+            const double m = fabs(out[c]);
+            if (m > vmax) vmax = m;
+          }
+          asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(P.dX + 4 * at(i, row(r))),
+                       "d"(out[0]), "d"(out[1]), "d"(out[2]), "d"(out[3])
+                       : "memory");
+        }
+        cur[r] = up;
       }
-      const int64_t g = (int64_t)z * plane + (int64_t)(y0 + ty) * P.nx + (x0 + tx);
-      double2 *o = reinterpret_cast<double2 *>(P.dX + 4 * g);
-      o[0] = make_double2(out[0], out[1]);
-      o[1] = make_double2(out[2], out[3]);
     }
   }
-  __pipeline_wait_prior(0);
   finish_rate(P, vmax, red);
 }
 
@@ -1125,7 +1083,7 @@ __global__ void __launch_bounds__(TX) k_rate_1d(RateParams P) {
       Mc[c] = Ms[S + c][f];
       Mn[c] = Ms[S + c][f + 1];
     }
-    face_flux(Xc, Mc, Xn, Mn, g, J);
+    face_flux8(Xc, Mc, Xn, Mn, g, J);
 #pragma unroll
     for (int c = 0; c < S; ++c) Fx[c][f] = J[c];
   }
@@ -1135,7 +1093,7 @@ __global__ void __launch_bounds__(TX) k_rate_1d(RateParams P) {
     double out[S];
 #pragma unroll
     for (int c = 0; c < S; ++c) {
-      out[c] = (Fx[c][tx + 1] - Fx[c][tx]) * P.inv_dx;
+      out[c] = (Fx[c][tx + 1] - Fx[c][tx]) * P.inv_dx8;
       const double v = fabs(out[c]);
       if (v > vmax) vmax = v;
     }
@@ -1533,7 +1491,7 @@ __global__ void __launch_bounds__(MAXT, 1)
           Mc[c] = Ms[(S + c) * MX + i];
           Mn[c] = Ms[(S + c) * MX + i + 1];
         }
-        face_flux(Xc, Mc, Xn, Mn, g, J);
+        face_flux8(Xc, Mc, Xn, Mn, g, J);
 #pragma unroll
         for (int c = 0; c < S; ++c) Fs[c * FX + i] = J[c];
       }
@@ -1543,7 +1501,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     for (int p = t; p < m; p += (int)blockDim.x)
 #pragma unroll
       for (int c = 0; c < S; ++c) {
-        const double d = (Fs[c * FX + p + 1] - Fs[c * FX + p]) * P.inv_dx;
+        const double d = (Fs[c * FX + p + 1] - Fs[c * FX + p]) * P.inv_dx8;
         Ds[c * chunk + p] = d;
         const double v = fabs(d);
         if (v > vmax) vmax = v;
@@ -1677,6 +1635,7 @@ constexpr int kGraphSteps = 50;      // steps per captured graph
 // read mu/M back).  All variants compute every value the same way.
 struct RateVariant {
   int tx, ty, minb;
+  int ty2 = 0;      // rows of a 2D tile, where not ty
   int nth;          // threads of a 2D block (1D block; >= tx * ty)
   bool win;
   bool split;
@@ -1706,16 +1665,16 @@ RateVariant make_variant() {
     const int s2 = (int)tile2d_smem<TX, TY, NTH, SORT>(), s3 = (int)march3d_smem<TX, TY, SORT>();
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
     if (vec) {
-      cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, true, WIN, false, NTH, SORT, PP>, a, s2);
+      cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, true, WIN, NTH, SORT, PP>, a, s2);
       cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, true, WIN, SORT, PP>, a, s3);
     } else {
-      cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, false, WIN, false, NTH, SORT, PP>, a, s2);
+      cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, false, WIN, NTH, SORT, PP>, a, s2);
       cudaFuncSetAttribute(k_rate_march3d<TX, TY, MINB, false, WIN, SORT, PP>, a, s3);
     }
   };
   v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
-    if (vec) launch_pdl(k_rate_tile2d<TX, TY, MINB, true, WIN, false, NTH, SORT, PP>, g, b, sm, s, P);
-    else launch_pdl(k_rate_tile2d<TX, TY, MINB, false, WIN, false, NTH, SORT, PP>, g, b, sm, s, P);
+    if (vec) launch_pdl(k_rate_tile2d<TX, TY, MINB, true, WIN, NTH, SORT, PP>, g, b, sm, s, P);
+    else launch_pdl(k_rate_tile2d<TX, TY, MINB, false, WIN, NTH, SORT, PP>, g, b, sm, s, P);
   };
   v.launch3d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P,
                   int zc) {
@@ -1723,7 +1682,7 @@ RateVariant make_variant() {
     else launch_pdl(k_rate_march3d<TX, TY, MINB, false, WIN, SORT, PP>, g, b, sm, s, P, zc);
   };
   v.kernels = [](bool vec, int dim) {
-    if (dim == 2) return kname("k_rate_tile2d", {TX, TY, MINB, vec, WIN, 0, NTH, SORT, PP});
+    if (dim == 2) return kname("k_rate_tile2d", {TX, TY, MINB, vec, WIN, NTH, SORT, PP});
     return kname("k_rate_march3d", {TX, TY, MINB, vec, WIN, SORT, PP});
   };
   return v;
@@ -1739,38 +1698,30 @@ void launch_chem(bool vec, cudaStream_t s, const RateParams &P) {
   else launch_pdl(k_chem<DIM, false>, g, dim3(kChemNT), 0, s, P);
 }
 
-// Split variant: k_chem, then faces and divergence by the tile kernel in 2D
-// and by the cp.async marching kernel (PP: per-point faces) in 3D.
-template <int TX, int TY, int MINB, bool PP>
+// Split variant: k_chem, then k_flux; in 2D a warp marches over ROWS rows (in
+// 3D rate_grid_of sets the planes of a chunk).
+template <int ROWS, int R, int MINB>
 RateVariant make_split_variant() {
   RateVariant v;
-  v.tx = TX;
-  v.ty = TY;
+  v.tx = kFluxCols;
+  v.ty = 4 * R;
+  v.ty2 = 4 * ROWS;
   v.minb = MINB;
-  v.nth = TX * TY;
+  v.nth = kFluxThreads;
   v.win = false;
   v.split = true;
-  v.smem2d = tile2d_smem<TX, TY>();
-  v.smem3d = Flux3Geom64<TX, TY>::smem(PP);
-  v.set_attrs = [](bool) {
-    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k_rate_tile2d<TX, TY, MINB, true, false, true>, a,
-                         (int)tile2d_smem<TX, TY>());
-    cudaFuncSetAttribute(k_flux3_64<TX, TY, MINB, PP>, a, (int)Flux3Geom64<TX, TY>::smem(PP));
-  };
-  v.launch2d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P) {
+  v.smem2d = v.smem3d = 0;
+  v.set_attrs = [](bool) {};
+  v.launch2d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P) {
     launch_chem<2>(vec, s, P);
-    launch_pdl(k_rate_tile2d<TX, TY, MINB, true, false, true>, g, b, sm, s, P);
+    launch_pdl(k_flux<2, 1, MINB>, g, dim3(kFluxThreads), 0, s, P, ROWS);
   };
-  v.launch3d = [](bool vec, dim3 g, dim3 b, size_t sm, cudaStream_t s, const RateParams &P,
-                  int zc) {
+  v.launch3d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P, int zc) {
     launch_chem<3>(vec, s, P);
-    launch_pdl(k_flux3_64<TX, TY, MINB, PP>, g, b, sm, s, P, zc);
+    launch_pdl(k_flux<3, R, MINB>, g, dim3(kFluxThreads), 0, s, P, zc);
   };
   v.kernels = [](bool vec, int dim) {
-    const std::string chem = kname("k_chem", {dim, vec}) + " + ";
-    if (dim == 2) return chem + kname("k_rate_tile2d", {TX, TY, MINB, 1, 0, 1, TX * TY, 0, 0});
-    return chem + kname("k_flux3_64", {TX, TY, MINB, PP});
+    return kname("k_chem", {dim, vec}) + " + " + kname("k_flux", {dim, dim == 2 ? 1 : R, MINB});
   };
   return v;
 }
@@ -1787,10 +1738,7 @@ const std::vector<RateVariant> &rate_variants() {
       make_variant<32, 8, 2, false, 256, 2, true>(), make_variant<32, 8, 2, false, 256, 2, false>(),
       make_variant<32, 4, 4, false, 128, 2, true>(),
       make_variant<32, 8, 3, false, 256, false, true>(), make_variant<64, 4, 2, true, 256, false, true>(),
-      make_split_variant<32, 4, 3, true>(), make_split_variant<32, 4, 3, false>(),
-      make_split_variant<32, 8, 2, true>(), make_split_variant<32, 8, 2, false>(),
-      make_split_variant<64, 4, 1, true>(), make_split_variant<32, 4, 2, true>(),
-      make_split_variant<32, 8, 3, true>()};
+      make_split_variant<4, 1, 3>(), make_split_variant<2, 1, 3>(), make_split_variant<8, 2, 2>()};
   return v;
 }
 
@@ -1801,7 +1749,8 @@ dim3 rate_grid_of(const pf5d_stepper *h, int variant, int *zc_out) {
   *zc_out = 1;
   if (h->d.dim == 1) return dim3((unsigned)((P.nx + kTX1 - 1) / kTX1));
   const RateVariant &v = rate_variants()[variant];
-  const unsigned gx = (unsigned)((P.nx + v.tx - 1) / v.tx), gy = (unsigned)((P.ny + v.ty - 1) / v.ty);
+  const int ty = h->d.dim == 2 && v.ty2 ? v.ty2 : v.ty;
+  const unsigned gx = (unsigned)((P.nx + v.tx - 1) / v.tx), gy = (unsigned)((P.ny + ty - 1) / ty);
   if (h->d.dim == 2) return dim3(gx, gy, 1);
   // Chunk of axis-0 planes per block: ~8 resident-block waves, >= 4 planes.
   const int64_t tiles = (int64_t)gx * gy;
@@ -2136,6 +2085,7 @@ pf5d_status pf5d_stepper_create(const pf5d_stepper_desc *desc, double *X, void *
     P.lvec.v[c] = desc->lvec[c];
   }
   P.inv_dx = 1.0 / desc->dx;
+  P.inv_dx8 = 0.125 * P.inv_dx;
   P.inv_dx2 = 1.0 / (desc->dx * desc->dx);
   P.ctld = desc->ctld;
   P.t_cfl = desc->t_cfl;
