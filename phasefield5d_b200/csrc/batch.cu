@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     unsigned flags = 0;
     float vmax;
     if (B.dim == 2)
-      vmax = tile2d32_body<TX, TY, WIN, SORT, false, PP>(P, local % B.ntx, local / B.ntx, work,
+      vmax = tile2d32_body<TX, TY, WIN, SORT, PP>(P, local % B.ntx, local / B.ntx, work,
                                                           &flags, tid);
     else
       vmax = tile1d32_body<NT>(B, P, local, reinterpret_cast<float *>(work), &flags, tid);

@@ -572,25 +572,6 @@ __device__ __forceinline__ void mu_plane32(const Rate32 &P, const float *Xm, con
   }
 }
 
-// mu/M of one plane (tile + 1-cell halo, or the tile only) read from the
-// split buffers (written by k32_chem) into dst, in mu_plane32's layout.
-template <int TX, int TY>
-__device__ __forceinline__ void load_mu_plane32(const Rate32 &P, int64_t zoff, const int *wx,
-                                                const int *wy, bool interior_only, float *dst,
-                                                int tid) {
-  using G = PlaneGeom<TX, TY>;
-  for (int pos = tid; pos < G::PM; pos += G::NT) {
-    const int my = pos / G::MX, mx = pos - my * G::MX;
-    if (skip_pos<G::MX, G::MY>(mx, my, interior_only)) continue;
-    const int64_t g = zoff + (int64_t)wy[my + 1] * P.nx + wx[mx + 1];
-    const float4 mu = __ldg(P.mm_mu + g), m = __ldg(P.mm_m + g);
-    const float2 f = __ldg(P.mm_f + g);
-    const float v[NPM] = {mu.x, mu.y, mu.z, mu.w, f.x, m.x, m.y, m.z, m.w, f.y};
-#pragma unroll
-    for (int r = 0; r < NPM; ++r) dst[r * G::PM + pos] = v[r];
-  }
-}
-
 // Shared memory common to the plane kernels, after the kernel-specific
 // arrays: block-max scratch (double), the table window (float4), window
 // reduction scratch and origin (int), halo index tables (int).
@@ -656,7 +637,7 @@ struct Tile2dSmem32 {
 
 // Evaluates tile (bx, by) of solve P and writes its dX/dt; returns this
 // thread's max |dX/dt|.  Ends with all threads past a barrier.
-template <int TX, int TY, bool WIN, int SORT = 0, bool SPLIT = false, bool PERPOINT = false>
+template <int TX, int TY, bool WIN, int SORT = 0, bool PERPOINT = false>
 __device__ __forceinline__ float tile2d32_body(const Rate32 &P, int bx, int by, float4 *sm4,
                                                unsigned *flags, int tid) {
   using G = PlaneGeom<TX, TY>;
@@ -682,11 +663,8 @@ __device__ __forceinline__ float tile2d32_body(const Rate32 &P, int bx, int by, 
   __syncthreads();
   load_plane32<TX, TY>(P.D, 0, wx, wy, P.nx, Xs, tid);
   __syncthreads();
-  if constexpr (SPLIT)
-    load_mu_plane32<TX, TY>(P, 0, wx, wy, false, Ms, tid);
-  else
-    mu_plane32<TX, TY, 2, WIN, SORT>(P, nullptr, Xs, nullptr, Ms, 0, wx, wy, false, win, wred,
-                                     win_lo, flags, tid, ss);
+  mu_plane32<TX, TY, 2, WIN, SORT>(P, nullptr, Xs, nullptr, Ms, 0, wx, wy, false, win, wred, win_lo,
+                                   flags, tid, ss);
   __syncthreads();
   float vmax = 0.f;
   if constexpr (PERPOINT) {

@@ -1,6 +1,7 @@
 // pf5d_gather.cuh -- table values (mu, M) of a block of points with the
-// gathers of one table cell shared, for the FP64 kernels that evaluate every
-// point once (the split rate stage and the drop-in interpolation).
+// gathers of one table cell shared, for the kernels that evaluate every point
+// once (the split rate stages): the ordering of a block's points by cell, used
+// by both forms, and the FP64 values.
 //
 // What bounds a one-point-per-thread evaluation is not DRAM (the nodes a
 // block touches stay in L1) but the path from L1 into the registers: 16 nodes
@@ -13,8 +14,8 @@
 // A block of NT threads takes NT * PER points:
 //   1. gather_add: each point's cell and fractions (interpolation.py:110-121)
 //      into shared memory, and its rank among the points of its bin (a hash of
-//      the cell; bin 255: outside the linear region).  Lanes of a warp with
-//      the same bin take one atomic together, and keep their order;
+//      the cell; bin 255: outside the linear region; gather_rank).  Lanes of a
+//      warp with the same bin take one atomic together, and keep their order;
 //   2. gather_sort: prefix sum over the bins, the points in bin order, and
 //      each bin's run cut into work items of up to K points;
 //   3. gather_values: a thread evaluates an item.  Every point has its own
@@ -35,18 +36,25 @@ constexpr int kGatherBins = 256;
 constexpr int kNoKey = -1;                                      // no point (past the field's edge)
 
 template <int NT_, int PER_, int K_>
-struct GatherSmem {
-  static constexpr int NT = NT_, PER = PER_, K = K_, kGatherPoints = NT * PER;
-  double2 v[4][kGatherPoints];      // t0 t1 | t2 t3, then mu1 mu2 | mu3 mu4 | M_Fe M1 | M2 M3
-  double v8[kGatherPoints];         // M4
-  int cell[kGatherPoints];
+struct GatherOrder {
+  static constexpr int NT = NT_, PER = PER_, K = K_, N = NT * PER;
+  int cell[N];                      // -1: outside the linear region
   int base[kGatherBins + 1];        // points (low half) and items (high half) before each bin
   int wsum[NT / 32 + 1];
   int nleft;
-  unsigned items[kGatherPoints / K + kGatherBins];
-  unsigned short order[kGatherPoints];
-  unsigned short left[kGatherPoints];
+  unsigned items[N / K + kGatherBins];
+  unsigned short order[N];
+  unsigned short left[N];
 };
+
+// FP64: fractions, then values
+template <int N>
+struct GatherValues {
+  double2 v[4][N];                  // t0 t1 | t2 t3, then mu1 mu2 | mu3 mu4 | M_Fe M1 | M2 M3
+  double v8[N];                     // M4
+};
+template <int NT, int PER, int K>
+struct GatherSmem : GatherValues<NT * PER>, GatherOrder<NT, PER, K> {};
 
 // Table cell of x exactly as the reference computes it (interpolation.py:103-121).
 __device__ __forceinline__ bool cell64(const Table &T, const double x[S], int ii[S], double tt[S]) {
@@ -63,29 +71,39 @@ __device__ __forceinline__ void gather_begin(G &g, int tid) {
   if (tid == 0) g.nleft = 0;
 }
 
-// Point x in slot q (valid lanes only hold one); returns its bin and rank,
-// key | rank << 16, or kNoKey.  Called by whole warps.
+// Rank of the point in slot q in the bin of its cell (ii, where it lies in the
+// linear region); returns bin and rank, key | rank << 16.  Called by the lanes
+// `active` of a warp.
 template <typename G>
-__device__ __forceinline__ int gather_add(G &g, const Table &T, bool valid,
-                                          const double x[S], int q) {
-  const unsigned active = __ballot_sync(0xffffffffu, valid);
-  if (!valid) return kNoKey;
-  int ii[S];
-  double tt[S];
-  int cell = -1, key = kGatherBins - 1;
-  if (cell64(T, x, ii, tt)) {
-    cell = ((ii[0] * T.n + ii[1]) * T.n + ii[2]) * T.n + ii[3];
-    key = (int)((unsigned)(41 * ii[0] + 13 * ii[1] + 5 * ii[2] + ii[3]) % (kGatherBins - 1u));
-    g.v[0][q] = make_double2(tt[0], tt[1]);
-    g.v[1][q] = make_double2(tt[2], tt[3]);
-  }
-  g.cell[q] = cell;
+__device__ __forceinline__ int gather_rank(G &g, unsigned active, bool linear, const int ii[S], int n,
+                                           int q) {
+  const int key = linear ? (int)((unsigned)(41 * ii[0] + 13 * ii[1] + 5 * ii[2] + ii[3]) %
+                                 (kGatherBins - 1u))
+                         : kGatherBins - 1;
+  g.cell[q] = linear ? ((ii[0] * n + ii[1]) * n + ii[2]) * n + ii[3] : -1;
   const unsigned same = __match_any_sync(active, key);
   const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;
   int before = 0;
   if (lane == lead) before = atomicAdd(&g.base[key], __popc(same));
   before = __shfl_sync(active, before, lead);
   return key | ((before + __popc(same & ((1u << lane) - 1u))) << 16);
+}
+
+// Point x in slot q (valid lanes only hold one); returns gather_rank's answer
+// or kNoKey.  Called by whole warps.
+template <typename G>
+__device__ __forceinline__ int gather_add(G &g, const Table &T, bool valid, const double x[S],
+                                          int q) {
+  const unsigned active = __ballot_sync(0xffffffffu, valid);
+  if (!valid) return kNoKey;
+  int ii[S] = {0, 0, 0, 0};
+  double tt[S];
+  const bool linear = cell64(T, x, ii, tt);
+  if (linear) {
+    g.v[0][q] = make_double2(tt[0], tt[1]);
+    g.v[1][q] = make_double2(tt[2], tt[3]);
+  }
+  return gather_rank(g, active, linear, ii, T.n, q);
 }
 
 // Points in bin order and the work items; kr: gather_add's answers for this
@@ -135,7 +153,18 @@ __device__ __forceinline__ void gather_get(const G &g, int q, double v[NP]) {
   v[8] = g.v8[q];
 }
 
-// The work items (barrier before and after by the caller of gather_rest).
+// The points that no item evaluated, one per thread: rest(q).  Barriers before
+// and after.
+template <typename G, typename Rest>
+__device__ __forceinline__ void gather_others(G &g, int tid, Rest rest) {
+  __syncthreads();
+  const int far0 = g.base[kGatherBins - 1] & 0xffff;
+  const int nfar = (g.base[kGatherBins] & 0xffff) - far0, n = nfar + g.nleft;
+  for (int l = tid; l < n; l += G::NT) rest(l < nfar ? (int)g.order[far0 + l] : (int)g.left[l - nfar]);
+  __syncthreads();
+}
+
+// The work items (gather_rest follows).
 template <bool VEC, typename G>
 __device__ __forceinline__ void gather_values(G &g, const Table &T, int nitems, int tid) {
   constexpr int K = G::K;
@@ -204,17 +233,12 @@ __device__ __forceinline__ void gather_values(G &g, const Table &T, int nitems, 
 template <bool VEC, typename G, typename Point>
 __device__ __forceinline__ void gather_rest(G &g, const Table &T, int tid, unsigned *flags,
                                             Point point) {
-  __syncthreads();
-  const int far0 = g.base[kGatherBins - 1] & 0xffff;
-  const int nfar = (g.base[kGatherBins] & 0xffff) - far0, n = nfar + g.nleft;
-  for (int l = tid; l < n; l += G::NT) {
-    const int q = l < nfar ? (int)g.order[far0 + l] : (int)g.left[l - nfar];
+  gather_others(g, tid, [&](int q) {
     double x[S], v[NP];
     point(q, x);
     interp_point<VEC>(T, x, v, flags);
     gather_put(g, q, v);
-  }
-  __syncthreads();
+  });
 }
 
 // The four components of a point; wide: the field is 32-byte aligned, so they

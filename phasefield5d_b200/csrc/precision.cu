@@ -25,7 +25,6 @@
 #include <map>
 #include <vector>
 
-#include <cuda_pipeline_primitives.h>
 #include <cufft.h>
 
 #include "pf5d_cluster.cuh"
@@ -33,6 +32,7 @@
 #include "pf5d_fft.h"
 #include "pf5d_fp32c.h"
 #include "pf5d_fp32c.cuh"
+#include "pf5d_gather.cuh"
 #include "pf5d_host.h"
 #include "pf5d_tiles.cuh"
 #include "pf5d_window.cuh"
@@ -43,16 +43,15 @@ namespace pf5d {
 // Rate kernels (same tiling as the FP64 kernels)
 // ------------------------------------------------------------------------
 
-template <int TX, int TY, int MINB, bool WIN, int SORT = 0, bool SPLIT = false,
-          bool PERPOINT = false>
+template <int TX, int TY, int MINB, bool WIN, int SORT = 0, bool PERPOINT = false>
 __global__ void __launch_bounds__(TX * TY, MINB) k32_rate_tile2d(Rate32 P) {
   pdl_wait();
   if (P.st->halt) return;
   extern __shared__ float4 sm4[];
   const int tid = threadIdx.y * TX + threadIdx.x;
   unsigned flags = 0;
-  const float vmax = tile2d32_body<TX, TY, WIN, SORT, SPLIT, PERPOINT>(P, blockIdx.x, blockIdx.y,
-                                                                      sm4, &flags, tid);
+  const float vmax = tile2d32_body<TX, TY, WIN, SORT, PERPOINT>(P, blockIdx.x, blockIdx.y, sm4,
+                                                               &flags, tid);
   raise_rate_flags(P.st, flags);
   finish_rate32(P, vmax, Tile2dSmem32<TX, TY, SORT>::red(sm4));
 }
@@ -361,170 +360,92 @@ __global__ void k32_mass_final(const double *partial, int nparts, double *out) {
 // ------------------------------------------------------------------------
 // Split rate evaluation, first kernel: mu/M and the closure X_Fe at every
 // point of a 1D/2D/3D field into the split buffers (mm_mu, mm_m, mm_f).
-//
-// A block of 256 threads takes a brick of 256 K points (32 x 8 x K in 3D,
-// 32 x 8K in 2D, 256K in 1D) in six phases:
-//   1. per point: Laplacian (neighbour order +axis0, -axis0, ...), the mu
-//      offset s' l - kappa lap, the FP64 closure, the table cell and its
-//      fractions (the deviation itself for points outside the linear region);
-//   2. counting sort of the points by a hash of their exact cell (bin 255
-//      holds the points outside the linear region);
-//   3. each linear bin's run is cut into work items of up to K consecutive
-//      points;
-//   4. a thread evaluates a work item: the 16 corner nodes of the item's
-//      cell are loaded once and accumulated into every point of the item
-//      with the point's own weights, so the table traffic per point drops
-//      K-fold (the lanes of a warp hold neighbouring items, mostly of the
-//      same cell, so the loads are broadcasts).  A point whose exact cell
-//      differs from the item's first (a hash collision) is set aside;
-//   5. the points set aside and those outside the linear region (nearest
-//      table row), one per thread;
-//   6. the block's outputs are stored coalesced.
-// Per point the block keeps three float4 in shared memory (point-major, so a
-// thread reads or writes a point's values with vector loads): the cell
-// fractions (or the deviation d outside the linear region), the mu offset,
-// and (cell, X_Fe); the outputs overwrite them as (mu), (M_Fe, M_1..3),
-// (M_4, X_Fe).  Every value is formed by the same routines, in the same
-// order, as in the fused kernels (weights32 / corner_acc32, mu_offset32,
+// The table values come first, up to K points of a cell per node load
+// (pf5d_gather.cuh); then each thread takes its own points in order:
+// Laplacian (neighbour order +axis0, -axis0, ...), mu offset, closure.  A
+// thread's points are consecutive along y (2D) or z (3D), so it loads each
+// point of that axis once.  Every value is formed by the same routines, in the
+// same order, as in the fused kernels (weights32 / corner_acc32, mu_offset32,
 // dsum32).
+//
+// Bound by the L1 data path, like the FP64 form's k_chem.  Rate stage (both
+// kernels, ms), earlier kernels -> here: 256^3 0.927 -> 0.830, with two phases
+// 1.21 -> 0.99; 512^2 0.0318 (fused) -> 0.0187.  512 points per block (PER = 4)
+// keep a cell's run longer than K; below about 400^2 they leave SMs idle, and
+// PER = 1 or 2 takes 0.0131 instead of 0.0161 at 389x250.  In 3D K = 2 with 24
+// warps per SM beats K = 4 with 16 (0.95); in 2D, where few blocks run at a
+// time anyway, K = 4 wins by a little.
 // ------------------------------------------------------------------------
-constexpr int kChemThreads = 256;
-
-template <int DIM, int K>
-struct ChemGeom {
-  static constexpr int NPB = kChemThreads * K;                     // points per block
-  static constexpr int BX = DIM == 1 ? NPB : 32;
-  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? 8 * K : 8);
-  static constexpr int BZ = DIM == 3 ? K : 1;
-  static constexpr int NITEMS = NPB / K + 256;                      // upper bound on items
-  // pio[3][NPB] float4 (point-major); items[NITEMS] u32; order, prank, left
-  // [NPB] u16; skey, pkey [NPB] u8; hist / cnt / ibase [256] int; wsum, nleft
-  static constexpr size_t smem = (size_t)3 * 16 * NPB + NITEMS * 4 + 3 * NPB * 2 + 2 * NPB +
-                                 3 * 256 * 4 + 16 * 4;
+template <int NT, int PER, int K>
+struct GatherSmem32 : GatherOrder<NT, PER, K> {
+  float4 v[2][NT * PER];            // fractions, then mu 1..4 | M_Fe, M_1..3
+  float v8[NT * PER];               // M_4
 };
 
-__device__ __forceinline__ int cell_key32(const int ii[S]) {
-  return (int)((unsigned)(41 * ii[0] + 13 * ii[1] + 5 * ii[2] + ii[3]) % 255u);
-}
+constexpr int kChemNT32 = 128;
 
-template <int DIM, int K, int MINB>
-__global__ void __launch_bounds__(kChemThreads, MINB) k32_chem(Rate32 P) {
-  using G = ChemGeom<DIM, K>;
-  constexpr int NT = kChemThreads, NPB = G::NPB;
-  extern __shared__ float4 sm4[];
-  float4 *pio = sm4;                                                   // 3 per point
-  unsigned *items = reinterpret_cast<unsigned *>(pio + 3 * NPB);
-  unsigned short *order = reinterpret_cast<unsigned short *>(items + G::NITEMS);
-  unsigned short *prank = order + NPB;
-  unsigned short *left = prank + NPB;
-  unsigned char *skey = reinterpret_cast<unsigned char *>(left + NPB);
-  unsigned char *pkey = skey + NPB;
-  int *hist = reinterpret_cast<int *>(pkey + NPB);                     // NPB % 4 == 0
-  int *cnt = hist + 256;
-  int *ibase = cnt + 256;
-  int *wsum = ibase + 256;
-  int *nleft = wsum + 12;
+template <int DIM, int PER>
+struct ChemTile32 {
+  static constexpr int NT = kChemNT32;
+  static constexpr int BX = DIM == 1 ? NT * PER : 32;
+  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? NT / 32 * PER : NT / 32);
+  static constexpr int BZ = DIM == 3 ? PER : 1;
+};
+
+template <int DIM, int PER, int K, int MINB>
+__global__ void __launch_bounds__(kChemNT32, MINB) k32_chem(Rate32 P) {
+  using G = ChemTile32<DIM, PER>;
+  constexpr int NT = kChemNT32;
+  __shared__ GatherSmem32<NT, PER, K> g;
   pdl_wait();
   if (P.st->halt) return;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  const int bx = blockIdx.x * G::BX, by = blockIdx.y * G::BY, bz = blockIdx.z * G::BZ;
   const Table32 &T = P.T;
   const int64_t plane = (int64_t)P.ny * P.nx;
-  hist[tid] = 0;
-  if (tid == 0) *nleft = 0;
+  // the point in slot q = j * NT + w * 32 + lane
+  auto px = [&](int j, int l, int v) { return DIM == 1 ? bx + j * NT + v * 32 + l : bx + l; };
+  auto py = [&](int j, int v) { return DIM == 1 ? 0 : (DIM == 2 ? by + PER * v + j : by + v); };
+  auto pz = [&](int j) { return DIM == 3 ? bz + j : 0; };
+  auto at = [&](int z, int y, int x) { return z * plane + (int64_t)y * P.nx + x; };
+  gather_begin(g, tid);
   __syncthreads();
-  // 1. per-point inputs
-#pragma unroll 1
-  for (int j = 0; j < K; ++j) {
-    const int q = tid + j * NT;
-    const int qx = q % G::BX, qy = (q / G::BX) % G::BY, qz = q / (G::BX * G::BY);
-    const int x = blockIdx.x * G::BX + qx, y = blockIdx.y * G::BY + qy, z = blockIdx.z * G::BZ + qz;
-    prank[q] = 0xFFFFu;
-    if (x >= P.nx || y >= P.ny || z >= P.nz) continue;
-    const int64_t zo = (int64_t)z * plane, g = zo + (int64_t)y * P.nx + x;
-    auto ld = [&](int64_t gi, float v[S]) {
-      const float4 a = __ldg(P.D + gi);
-      v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
-    };
-    constexpr int NB = 2 * DIM;
-    float d[S], nb[NB][S];
-    ld(g, d);
-    int k = 0;
-    if (DIM == 3) {
-      const int zp = z + 1 == P.nz ? 0 : z + 1, zm = z == 0 ? P.nz - 1 : z - 1;
-      ld((int64_t)zp * plane + (int64_t)y * P.nx + x, nb[k++]);
-      ld((int64_t)zm * plane + (int64_t)y * P.nx + x, nb[k++]);
-    }
-    if (DIM >= 2) {
-      const int yp = y + 1 == P.ny ? 0 : y + 1, ym = y == 0 ? P.ny - 1 : y - 1;
-      ld(zo + (int64_t)yp * P.nx + x, nb[k++]);
-      ld(zo + (int64_t)ym * P.nx + x, nb[k++]);
-    }
-    const int xp = x + 1 == P.nx ? 0 : x + 1, xm = x == 0 ? P.nx - 1 : x - 1;
-    ld(zo + (int64_t)y * P.nx + xp, nb[k++]);
-    ld(zo + (int64_t)y * P.nx + xm, nb[k]);
-    float lap[S], off[S];
+  int kr[PER];
 #pragma unroll
-    for (int c = 0; c < S; ++c) {
-      float n[NB];
-#pragma unroll
-      for (int i = 0; i < NB; ++i) n[i] = nb[i][c];
-      lap[c] = lap32<NB>(n, d[c], P.inv_dx2);
+  for (int j = 0; j < PER; ++j) {
+    const int x = px(j, lane, w), y = py(j, w), z = pz(j);
+    const bool valid = x < P.nx && y < P.ny && z < P.nz;
+    const unsigned active = __ballot_sync(0xffffffffu, valid);
+    kr[j] = kNoKey;
+    if (valid) {
+      const float4 d4 = __ldg(P.D + at(z, y, x));
+      const float d[S] = {d4.x, d4.y, d4.z, d4.w};
+      int ii[S] = {0, 0, 0, 0};
+      float tt[S];
+      const bool linear = cell32(T, d, dsum32(d), ii, tt);
+      const int q = j * NT + tid;
+      if (linear) g.v[0][q] = make_float4(tt[0], tt[1], tt[2], tt[3]);
+      kr[j] = gather_rank(g, active, linear, ii, T.n, q);
     }
-    mu_offset32(P, lap, P.sp ? __ldg(P.sp + g) : 0.f, off);
-    const double sd = dsum32(d);
-    int ii[S];
-    float tt[S];
-    int cell = -1, key = 255;
-    if (cell32(T, d, sd, ii, tt)) {
-      cell = ((ii[0] * T.n + ii[1]) * T.n + ii[2]) * T.n + ii[3];
-      key = cell_key32(ii);
-    } else {
-#pragma unroll
-      for (int c = 0; c < S; ++c) tt[c] = d[c];
-    }
-    pio[3 * q] = make_float4(tt[0], tt[1], tt[2], tt[3]);
-    pio[3 * q + 1] = make_float4(off[0], off[1], off[2], off[3]);
-    pio[3 * q + 2] = make_float4(__int_as_float(cell), (float)(P.c_fe - sd), 0.f, 0.f);
-    pkey[q] = (unsigned char)key;
-    prank[q] = (unsigned short)atomicAdd(&hist[key], 1);
   }
-  __syncthreads();
-  // 2. counting sort by cell key
-  cnt[tid] = hist[tid];
-  const int nvalid = block_exclusive_scan<256, NT>(hist, wsum, tid);
-  for (int q = tid; q < NPB; q += NT) {
-    if (prank[q] == 0xFFFFu) continue;
-    const int b = pkey[q], s = hist[b] + prank[q];
-    order[s] = (unsigned short)q;
-    skey[s] = (unsigned char)b;
-  }
-  // 3. work items: runs of up to K points of one linear bin
-  ibase[tid] = tid == 255 ? 0 : (cnt[tid] + K - 1) / K;
-  const int nitems = block_exclusive_scan<256, NT>(ibase, wsum, tid);
-  const int lin_end = nvalid - cnt[255];            // bin 255 (nearest row) sorts last
-  for (int s = tid; s < lin_end; s += NT) {
-    const int b = skey[s], r = s - hist[b];
-    if (r % K == 0) items[ibase[b] + r / K] = (unsigned)s | ((unsigned)min(K, cnt[b] - r) << 16);
-  }
-  __syncthreads();
-  // 4. the work items
+  const int nitems = gather_sort(g, kr, tid);
   const float4 *g4 = reinterpret_cast<const float4 *>(T.grid);
   const int64_t s3 = 3, s2 = 3 * (int64_t)T.n, s1 = s2 * T.n, s0 = s1 * T.n;
   for (int it = tid; it < nitems; it += NT) {
-    const unsigned e = items[it];
-    const int s = (int)(e & 0xFFFFu), m = (int)(e >> 16);
+    const unsigned e = g.items[it];
+    const int s = (int)(e & 0xffffu), m = (int)(e >> 16);
     int q[K];
-    bool use[K];
     Weights32 W[K];
-    int cell0 = 0;
+    const int cell0 = g.cell[g.order[s]];
+    unsigned mine = 0;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      q[j] = j < m ? (int)order[s + j] : 0;
-      const int cj = __float_as_int(pio[3 * q[j] + 2].x);
-      if (j == 0) cell0 = cj;
-      use[j] = j < m && cj == cell0;
-      if (j < m && !use[j]) left[atomicAdd(nleft, 1)] = (unsigned short)q[j];
-      const float4 t4 = pio[3 * q[j]];
+      q[j] = g.order[s + (j < m ? j : 0)];
+      if (j < m) {
+        if (g.cell[q[j]] == cell0) mine |= 1u << j;
+        else g.left[atomicAdd(&g.nleft, 1)] = (unsigned short)q[j];
+      }
+      const float4 t4 = g.v[0][q[j]];
       const float tt[S] = {t4.x, t4.y, t4.z, t4.w};
       W[j] = weights32(tt);
     }
@@ -538,188 +459,185 @@ __global__ void __launch_bounds__(kChemThreads, MINB) k32_chem(Rate32 P) {
 #pragma unroll
       for (int j = 0; j < K; ++j) corner_acc32(c, W[j].wa[c >> 2] * W[j].wb[c & 3], a, b, f, acc[j]);
     }
-    // mu = table value + offset; rows in chem32's order (X_Fe stays in row 9)
 #pragma unroll
-    for (int j = 0; j < K; ++j) {
-      if (!use[j]) continue;
-      float4 *o = pio + 3 * q[j];
-      const float4 off = o[1];
-      o[0] = make_float4(acc[j][0] + off.x, acc[j][1] + off.y, acc[j][2] + off.z, acc[j][3] + off.w);
-      o[1] = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
-      o[2].x = acc[j][8];
+    for (int j = 0; j < K; ++j)
+      if (mine & (1u << j)) {
+        g.v[0][q[j]] = make_float4(acc[j][0], acc[j][1], acc[j][2], acc[j][3]);
+        g.v[1][q[j]] = make_float4(acc[j][4], acc[j][5], acc[j][6], acc[j][7]);
+        g.v8[q[j]] = acc[j][8];
+      }
+  }
+  unsigned flags = 0;
+  gather_others(g, tid, [&](int q) {
+    const int j = q / NT, v = (q / 32) % (NT / 32);
+    const float4 d4 = __ldg(P.D + at(pz(j), py(j, v), px(j, q & 31, v)));
+    const float d[S] = {d4.x, d4.y, d4.z, d4.w};
+    float o[NP];
+    interp32(P, d, dsum32(d), nullptr, nullptr, o, &flags);
+    g.v[0][q] = make_float4(o[0], o[1], o[2], o[3]);
+    g.v[1][q] = make_float4(o[4], o[5], o[6], o[7]);
+    g.v8[q] = o[8];
+  });
+  raise_rate_flags(P.st, flags);
+  if (kr[0] == kNoKey) return;                  // none of this thread's points is in the field
+  const int x0 = px(0, lane, w), y0 = py(0, w), z0 = pz(0);
+  float4 below, dc = __ldg(P.D + at(z0, y0, x0)), above;   // along the marching axis
+  if (DIM == 2) below = __ldg(P.D + at(0, y0 == 0 ? P.ny - 1 : y0 - 1, x0));
+  if (DIM == 3) below = __ldg(P.D + at(z0 == 0 ? P.nz - 1 : z0 - 1, y0, x0));
+#pragma unroll
+  for (int j = 0; j < PER; ++j) {
+    if (kr[j] == kNoKey) break;
+    const int x = px(j, lane, w), y = py(j, w), z = pz(j), q = j * NT + tid;
+    constexpr int NB = 2 * DIM;
+    float4 n4[NB];
+    int k = 0;
+    if (DIM == 1) {
+      if (j > 0) dc = __ldg(P.D + at(0, 0, x));
+    } else {
+      above = __ldg(P.D + (DIM == 2 ? at(0, y + 1 == P.ny ? 0 : y + 1, x)
+                                    : at(z + 1 == P.nz ? 0 : z + 1, y, x)));
+      n4[k++] = above;
+      n4[k++] = below;
+    }
+    if (DIM == 3) {
+      n4[k++] = __ldg(P.D + at(z, y + 1 == P.ny ? 0 : y + 1, x));
+      n4[k++] = __ldg(P.D + at(z, y == 0 ? P.ny - 1 : y - 1, x));
+    }
+    n4[k++] = __ldg(P.D + at(z, y, x + 1 == P.nx ? 0 : x + 1));
+    n4[k] = __ldg(P.D + at(z, y, x == 0 ? P.nx - 1 : x - 1));
+    const int64_t gi = at(z, y, x);
+    const float d[S] = {dc.x, dc.y, dc.z, dc.w};
+    float lap[S], off[S];
+    {
+      float n[S][NB];
+#pragma unroll
+      for (int i = 0; i < NB; ++i) {
+        n[0][i] = n4[i].x;
+        n[1][i] = n4[i].y;
+        n[2][i] = n4[i].z;
+        n[3][i] = n4[i].w;
+      }
+#pragma unroll
+      for (int c = 0; c < S; ++c) lap[c] = lap32<NB>(n[c], d[c], P.inv_dx2);
+    }
+    mu_offset32(P, lap, P.sp ? __ldg(P.sp + gi) : 0.f, off);
+    const float4 a = g.v[0][q], b = g.v[1][q];
+    P.mm_mu[gi] = make_float4(a.x + off[0], a.y + off[1], a.z + off[2], a.w + off[3]);
+    P.mm_m[gi] = make_float4(b.y, b.z, b.w, g.v8[q]);
+    P.mm_f[gi] = make_float2(b.x, (float)(P.c_fe - dsum32(d)));
+    if (DIM != 1) {
+      below = dc;
+      dc = above;
     }
   }
-  __syncthreads();
-  // 5. points set aside and points outside the linear region, one per thread
-  unsigned flags = 0;
-  const int nnn = cnt[255], nl = nnn + *nleft;
-  for (int l = tid; l < nl; l += NT) {
-    const int q = l < nnn ? (int)order[lin_end + l] : (int)left[l - nnn];
-    float4 *o = pio + 3 * q;
-    const int cell = __float_as_int(o[2].x);
-    const float4 a4 = o[0];
-    const float a[S] = {a4.x, a4.y, a4.z, a4.w};
-    float v[NP];
-    if (cell < 0) nearest_row32(T, a, v, &flags);
-    else interp_nodes32(g4 + (int64_t)cell * 3, (int)s0, (int)s1, (int)s2, (int)s3, a, v);
-    const float4 off = o[1];
-    o[0] = make_float4(v[0] + off.x, v[1] + off.y, v[2] + off.z, v[3] + off.w);
-    o[1] = make_float4(v[4], v[5], v[6], v[7]);
-    o[2].x = v[8];
-  }
-  raise_rate_flags(P.st, flags);
-  __syncthreads();
-  // 6. coalesced stores
-#pragma unroll 1
-  for (int j = 0; j < K; ++j) {
-    const int q = tid + j * NT;
-    const int qx = q % G::BX, qy = (q / G::BX) % G::BY, qz = q / (G::BX * G::BY);
-    const int x = blockIdx.x * G::BX + qx, y = blockIdx.y * G::BY + qy, z = blockIdx.z * G::BZ + qz;
-    if (x >= P.nx || y >= P.ny || z >= P.nz) continue;
-    const int64_t g = (int64_t)z * plane + (int64_t)y * P.nx + x;
-    const float4 a = pio[3 * q], b = pio[3 * q + 1], c = pio[3 * q + 2];
-    P.mm_mu[g] = a;
-    P.mm_m[g] = make_float4(b.y, b.z, b.w, c.x);
-    P.mm_f[g] = make_float2(b.x, c.y);
-  }
 }
 
-template <int DIM, int K, int MINB>
-void chem32_attrs() {
-  cudaFuncSetAttribute(k32_chem<DIM, K, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)ChemGeom<DIM, K>::smem);
-}
-
-template <int DIM, int K, int MINB>
+template <int DIM, int PER, int K, int MINB>
 void launch_chem32(cudaStream_t s, const Rate32 &P) {
-  using G = ChemGeom<DIM, K>;
+  using G = ChemTile32<DIM, PER>;
   const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
                (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-  launch_pdl(k32_chem<DIM, K, MINB>, g, dim3(kChemThreads), G::smem, s, P);
+  launch_pdl(k32_chem<DIM, PER, K, MINB>, g, dim3(kChemNT32), 0, s, P);
 }
 
 // ------------------------------------------------------------------------
-// Split rate evaluation, second kernel in 3D: face fluxes and divergence of
-// a TX x TY plane tile marching along axis 0, from the split buffers.  Each
-// plane position of the tile and its 1-cell halo (corners skipped) is
-// staged as it is stored -- float4 D, float4 mu, float4 M, float2 (M_Fe,
-// X_Fe) -- by cp.async into a three-slot ring, so plane z+2 is in flight
-// while plane z is evaluated.  PERPOINT: each point evaluates its four
-// in-plane faces (a face by both of its cells, with the same operands and
-// operation order); otherwise each in-plane face is evaluated once into
-// shared buffers.  Same face routine and divergence order as the fused
-// marching kernel.
+// Split rate evaluation, second kernel: faces and divergence from D and the
+// split buffers, without shared memory or barriers, as the FP64 form's k_flux:
+// a warp of 32 columns (30 of them finished) marches along axis 0, carries the
+// face along the march, and hands on the face between columns by shuffles.
+// Same face routine and divergence order as the fused kernels.
+//
+// Bound by the latency of its loads and by issue.  256^3: 0.337 ms as a 32x8
+// tile with a shared cp.async ring and five faces per point.
 // ------------------------------------------------------------------------
-template <int TX, int TY>
-struct Flux3Geom {
-  static constexpr int MX = TX + 2, MY = TY + 2, PM = MX * MY, NT = TX * TY;
-  static constexpr int NFX = TY * (TX + 1), NFY = (TY + 1) * TX;
-  static constexpr size_t slot = (size_t)PM * (3 * 16 + 8);       // bytes per ring slot
-  static constexpr size_t smem(bool perpoint) {
-    return 3 * slot + (perpoint ? 0 : (size_t)(NFX + NFY) * 16) + (NT / 32) * 8 +
-           (MX + MY) * 4;
-  }
+constexpr int kFluxThreads32 = 128, kFluxCols32 = 30;
+
+struct Pt32 {
+  float4 d, mu, m;
+  float2 f;
 };
 
-template <int TX, int TY, int MINB, bool PERPOINT>
-__global__ void __launch_bounds__(TX * TY, MINB) k32_flux3(Rate32 P, int zc) {
-  using G = Flux3Geom<TX, TY>;
-  static_assert(G::slot % 16 == 0, "ring slots must stay 16-byte aligned");
+__device__ __forceinline__ Pt32 load_pt32(const Rate32 &P, int64_t g) {
+  return Pt32{__ldg(P.D + g), __ldg(P.mm_mu + g), __ldg(P.mm_m + g), __ldg(P.mm_f + g)};
+}
+
+__device__ __forceinline__ float4 face_pts32(const Rate32 &P, const Pt32 &lo, const Pt32 &hi) {
+  return face_flux32(P, lo.d, lo.mu, lo.m, lo.f, hi.d, hi.mu, hi.m, hi.f);
+}
+
+__device__ __forceinline__ float4 shfl_down4(const float4 &v) {
+  return make_float4(__shfl_down_sync(0xffffffffu, v.x, 1), __shfl_down_sync(0xffffffffu, v.y, 1),
+                     __shfl_down_sync(0xffffffffu, v.z, 1), __shfl_down_sync(0xffffffffu, v.w, 1));
+}
+
+template <int DIM, int R, int MINB>
+__global__ void __launch_bounds__(kFluxThreads32, MINB) k32_flux(Rate32 P, int rows) {
+  static_assert(DIM == 3 || R == 1, "rows per thread are of axis 1");
+  __shared__ double red[kFluxThreads32 / 32];
   pdl_wait();
   if (P.st->halt) return;
-  extern __shared__ float4 sm4[];
-  // ring slot r: D[PM], mu[PM], M[PM] (float4) then F[PM] (float2)
-  float4 *ring = sm4;
-  float4 *Fx = reinterpret_cast<float4 *>(reinterpret_cast<char *>(sm4) + 3 * G::slot);
-  float4 *Fy = Fx + (PERPOINT ? 0 : G::NFX);
-  double *red = reinterpret_cast<double *>(Fy + (PERPOINT ? 0 : G::NFY));
-  int *wx = reinterpret_cast<int *>(red + G::NT / 32);
-  int *wy = wx + G::MX;
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * TX + tx;
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY;
-  const int zb = blockIdx.z * zc;
-  const int ze = min(zb + zc, P.nz);
-  const int64_t plane = (int64_t)P.ny * P.nx;
-  for (int i = tid; i < G::MX + G::MY; i += G::NT) {
-    if (i < G::MX) wx[i] = wrap_any(x0 + i - 1, P.nx);
-    else wy[i - G::MX] = wrap_any(y0 + (i - G::MX) - 1, P.ny);
-  }
-  __syncthreads();
-  auto sD = [&](int z) { return ring + ((z - zb + 3) % 3) * (G::slot / 16); };
-  auto sMu = [&](int z) { return sD(z) + G::PM; };
-  auto sM = [&](int z) { return sD(z) + 2 * G::PM; };
-  auto sF = [&](int z) { return reinterpret_cast<float2 *>(sD(z) + 3 * G::PM); };
-  auto issue = [&](int z, bool interior_only) {
-    const int64_t zoff = (int64_t)wrap_any(z, P.nz) * plane;
-    float4 *d = sD(z), *mu = sMu(z), *m = sM(z);
-    float2 *f = sF(z);
-    for (int pos = tid; pos < G::PM; pos += G::NT) {
-      const int my = pos / G::MX, mx = pos - my * G::MX;
-      const bool ex = (mx == 0 || mx == G::MX - 1), ey = (my == 0 || my == G::MY - 1);
-      if (interior_only ? (ex || ey) : (ex && ey)) continue;
-      const int64_t g = zoff + (int64_t)wy[my] * P.nx + wx[mx];
-      __pipeline_memcpy_async(d + pos, P.D + g, 16);
-      __pipeline_memcpy_async(mu + pos, P.mm_mu + g, 16);
-      __pipeline_memcpy_async(m + pos, P.mm_m + g, 16);
-      __pipeline_memcpy_async(f + pos, P.mm_f + g, 8);
-    }
-    __pipeline_commit();
-  };
-  auto face = [&](int zl, int pl, int zh, int ph) {
-    return face_flux32(P, sD(zl)[pl], sMu(zl)[pl], sM(zl)[pl], sF(zl)[pl], sD(zh)[ph],
-                       sMu(zh)[ph], sM(zh)[ph], sF(zh)[ph]);
-  };
-  const int p = (ty + 1) * G::MX + (tx + 1);
-  const bool in_tile = (x0 + tx < P.nx) && (y0 + ty < P.ny);
-  issue(zb - 1, true);
-  issue(zb, false);
-  issue(zb + 1, false);
-  __pipeline_wait_prior(1);
-  __syncthreads();
-  float4 Jm = face(zb - 1, p, zb, p);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int col = blockIdx.x * kFluxCols32 + lane - 1, x = wrap_any(col, P.nx);
+  // axis 0: the march, over [first, last); 3D: axis 1 is this warp's R rows
+  const int n0 = DIM == 3 ? P.nz : P.ny;
+  const int y = (blockIdx.y * 4 + w) * R;              // 3D
+  const int first = (DIM == 3 ? blockIdx.z : blockIdx.y * 4 + w) * rows;
+  const int last = min(first + rows, n0);
+  const bool out_lane = lane > 0 && lane <= kFluxCols32 && col < P.nx;
   float vmax = 0.f;
-  for (int z = zb; z < ze; ++z) {
-    __pipeline_wait_prior(0);          // plane z+1 copied (this thread's part)
-    __syncthreads();                   // ... and every thread's; slot of z-1 free
-    if (z + 2 <= ze) issue(z + 2, false);
-    const float4 Jz = face(z, p, z + 1, p);
-    float4 jyp, jym, jxp, jxm;
-    if constexpr (PERPOINT) {
-      jyp = face(z, p, z, p + G::MX);
-      jym = face(z, p - G::MX, z, p);
-      jxp = face(z, p, z, p + 1);
-      jxm = face(z, p - 1, z, p);
-    } else {
-      for (int f = tid; f < G::NFX + G::NFY; f += G::NT) {
-        if (f < G::NFX) {
-          const int fy = f / (TX + 1), fx = f - fy * (TX + 1);
-          const int pl = (fy + 1) * G::MX + fx;
-          Fx[f] = face(z, pl, z, pl + 1);
-        } else {
-          const int f2 = f - G::NFX;
-          const int fy = f2 / TX, fx = f2 - fy * TX;
-          const int pl = fy * G::MX + (fx + 1);
-          Fy[f2] = face(z, pl, z, pl + G::MX);
-        }
-      }
-      __syncthreads();
-      jyp = Fy[(ty + 1) * TX + tx];
-      jym = Fy[ty * TX + tx];
-      jxp = Fx[ty * (TX + 1) + tx + 1];
-      jxm = Fx[ty * (TX + 1) + tx];
-    }
-    if (in_tile) {
-      const float a[S] = {Jz.x - Jm.x, Jz.y - Jm.y, Jz.z - Jm.z, Jz.w - Jm.w};
-      const float ay[S] = {jyp.x - jym.x, jyp.y - jym.y, jyp.z - jym.z, jyp.w - jym.w};
-      const float ax[S] = {jxp.x - jxm.x, jxp.y - jxm.y, jxp.z - jxm.z, jxp.w - jxm.w};
-      float out[S];
+  if (first < n0 && (DIM == 2 || y < P.ny)) {          // whole warps
+    auto at = [&](int i, int yy) {
+      return DIM == 3 ? ((int64_t)i * P.ny + yy) * P.nx + x : (int64_t)i * P.nx + x;
+    };
+    // a thread's rows past the field's last one repeat it and write nothing
+    auto row = [&](int r) { return DIM == 3 ? min(y + r, P.ny - 1) : 0; };
+    const int ym = y == 0 ? P.ny - 1 : y - 1, yp = y + R >= P.ny ? 0 : y + R;
+    Pt32 cur[R];
+    float4 jm[R];
 #pragma unroll
-      for (int c = 0; c < S; ++c) out[c] = ((a[c] + ay[c]) + ax[c]) * P.flux_scale;
-      store_rate(P.dX, (int64_t)z * plane + (int64_t)(y0 + ty) * P.nx + (x0 + tx), out, vmax);
+    for (int r = 0; r < R; ++r) {
+      const Pt32 below = load_pt32(P, at(first == 0 ? n0 - 1 : first - 1, row(r)));
+      cur[r] = load_pt32(P, at(first, row(r)));
+      jm[r] = face_pts32(P, below, cur[r]);
     }
-    Jm = Jz;
+    for (int i = first; i < last; ++i) {
+      const int ip = i + 1 == n0 ? 0 : i + 1;
+      Pt32 up[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) up[r] = load_pt32(P, at(ip, row(r)));
+      float4 jym = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (DIM == 3) jym = face_pts32(P, load_pt32(P, at(i, ym)), cur[0]);
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        Pt32 nb{shfl_down4(cur[r].d), shfl_down4(cur[r].mu), shfl_down4(cur[r].m),
+                make_float2(__shfl_down_sync(0xffffffffu, cur[r].f.x, 1),
+                            __shfl_down_sync(0xffffffffu, cur[r].f.y, 1))};
+        const float4 jx = face_pts32(P, cur[r], nb);
+        const float4 jl = make_float4(
+            __shfl_up_sync(0xffffffffu, jx.x, 1), __shfl_up_sync(0xffffffffu, jx.y, 1),
+            __shfl_up_sync(0xffffffffu, jx.z, 1), __shfl_up_sync(0xffffffffu, jx.w, 1));
+        float4 jyp = jym;
+        if (DIM == 3) {
+          // the last row's upper neighbour (for a row that repeats: unused)
+          if (r == R - 1 || y + r + 1 >= P.ny) nb = load_pt32(P, at(i, yp));
+          else nb = cur[r + 1 < R ? r + 1 : r];
+          jyp = face_pts32(P, cur[r], nb);
+        }
+        const float4 jz = face_pts32(P, cur[r], up[r]);
+        float out[S];
+        const float az[S] = {jz.x - jm[r].x, jz.y - jm[r].y, jz.z - jm[r].z, jz.w - jm[r].w};
+        const float ay[S] = {jyp.x - jym.x, jyp.y - jym.y, jyp.z - jym.z, jyp.w - jym.w};
+        const float ax[S] = {jx.x - jl.x, jx.y - jl.y, jx.z - jl.z, jx.w - jl.w};
+#pragma unroll
+        for (int c = 0; c < S; ++c)
+          out[c] = (DIM == 3 ? (az[c] + ay[c]) + ax[c] : az[c] + ax[c]) * P.flux_scale;
+        if (out_lane && (DIM == 2 || y + r < P.ny)) store_rate(P.dX, at(i, row(r)), out, vmax);
+        jm[r] = jz;
+        jym = jyp;
+        cur[r] = up[r];
+      }
+    }
   }
-  __pipeline_wait_prior(0);
   finish_rate32(P, vmax, red);
 }
 
@@ -1091,6 +1009,7 @@ constexpr int kGraphSteps32 = 50;
 
 struct Variant32 {
   int tx, ty, minb;
+  int ty2 = 0;                  // rows of a 2D tile, where not ty
   bool split;
   size_t smem2d, smem3d;
   void (*set_attrs)();
@@ -1110,56 +1029,47 @@ Variant32 make_variant32() {
   v.smem3d = march3d32_smem<TX, TY, SORT>();
   v.set_attrs = []() {
     const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k32_rate_tile2d<TX, TY, MINB, WIN, SORT, false, PP>, a,
+    cudaFuncSetAttribute(k32_rate_tile2d<TX, TY, MINB, WIN, SORT, PP>, a,
                          (int)tile2d32_smem<TX, TY, SORT>());
     cudaFuncSetAttribute(k32_rate_march3d<TX, TY, MINB, WIN, SORT>, a,
                          (int)march3d32_smem<TX, TY, SORT>());
   };
   v.launch2d = [](dim3 g, dim3 b, size_t sm, cudaStream_t s, const Rate32 &P) {
-    launch_pdl(k32_rate_tile2d<TX, TY, MINB, WIN, SORT, false, PP>, g, b, sm, s, P);
+    launch_pdl(k32_rate_tile2d<TX, TY, MINB, WIN, SORT, PP>, g, b, sm, s, P);
   };
   v.launch3d = [](dim3 g, dim3 b, size_t sm, cudaStream_t s, const Rate32 &P, int zc) {
     launch_pdl(k32_rate_march3d<TX, TY, MINB, WIN, SORT>, g, b, sm, s, P, zc);
   };
   v.kernels = [](int dim) {
-    if (dim == 2) return kname("k32_rate_tile2d", {TX, TY, MINB, WIN, SORT, 0, PP});
+    if (dim == 2) return kname("k32_rate_tile2d", {TX, TY, MINB, WIN, SORT, PP});
     return kname("k32_rate_march3d", {TX, TY, MINB, WIN, SORT});
   };
   return v;
 }
 
-// Split variant: k32_chem (K points per work item, KMINB resident blocks)
-// over all points, then the tile kernel (2D) or the marching flux kernel
-// (3D, PP: per-point faces) reading mu/M back.
-template <int TX, int TY, int MINB, int K, int KMINB, bool PP = false>
+// Split variant: k32_chem, then k32_flux; in 2D a warp marches over ROWS rows
+// (in 3D grid32_of sets the planes of a chunk).
+template <int ROWS, int R, int MINB, int PER, int K, int KMINB>
 Variant32 make_split_variant32() {
   Variant32 v;
-  v.tx = TX;
-  v.ty = TY;
+  v.tx = kFluxCols32;
+  v.ty = 4 * R;
+  v.ty2 = 4 * ROWS;
   v.minb = MINB;
   v.split = true;
-  v.smem2d = tile2d32_smem<TX, TY>();
-  v.smem3d = Flux3Geom<TX, TY>::smem(PP);
-  v.set_attrs = []() {
-    const auto a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-    cudaFuncSetAttribute(k32_rate_tile2d<TX, TY, MINB, false, false, true>, a,
-                         (int)tile2d32_smem<TX, TY>());
-    cudaFuncSetAttribute(k32_flux3<TX, TY, MINB, PP>, a, (int)Flux3Geom<TX, TY>::smem(PP));
-    chem32_attrs<2, K, KMINB>();
-    chem32_attrs<3, K, KMINB>();
+  v.smem2d = v.smem3d = 0;
+  v.set_attrs = []() {};
+  v.launch2d = [](dim3 g, dim3, size_t, cudaStream_t s, const Rate32 &P) {
+    launch_chem32<2, PER, K, KMINB>(s, P);
+    launch_pdl(k32_flux<2, 1, MINB>, g, dim3(kFluxThreads32), 0, s, P, ROWS);
   };
-  v.launch2d = [](dim3 g, dim3 b, size_t sm, cudaStream_t s, const Rate32 &P) {
-    launch_chem32<2, K, KMINB>(s, P);
-    launch_pdl(k32_rate_tile2d<TX, TY, MINB, false, false, true>, g, b, sm, s, P);
-  };
-  v.launch3d = [](dim3 g, dim3 b, size_t sm, cudaStream_t s, const Rate32 &P, int zc) {
-    launch_chem32<3, K, KMINB>(s, P);
-    launch_pdl(k32_flux3<TX, TY, MINB, PP>, g, b, sm, s, P, zc);
+  v.launch3d = [](dim3 g, dim3, size_t, cudaStream_t s, const Rate32 &P, int zc) {
+    launch_chem32<3, PER, K, KMINB>(s, P);
+    launch_pdl(k32_flux<3, R, MINB>, g, dim3(kFluxThreads32), 0, s, P, zc);
   };
   v.kernels = [](int dim) {
-    const std::string chem = kname("k32_chem", {dim, K, KMINB}) + " + ";
-    if (dim == 2) return chem + kname("k32_rate_tile2d", {TX, TY, MINB, 0, 0, 1, 0});
-    return chem + kname("k32_flux3", {TX, TY, MINB, PP});
+    return kname("k32_chem", {dim, PER, K, KMINB}) + " + " +
+           kname("k32_flux", {dim, dim == 2 ? 1 : R, MINB});
   };
   return v;
 }
@@ -1175,10 +1085,9 @@ const std::vector<Variant32> &variants32() {
       make_variant32<32, 8, 3, false, 2, true>(), make_variant32<32, 16, 2, false, 2, true>(),
       make_variant32<32, 16, 2, false, 2, false>(),
       make_variant32<32, 8, 3, false, false, true>(), make_variant32<32, 16, 2, false, false, true>(),
-      make_split_variant32<32, 8, 3, 2, 4, true>(), make_split_variant32<32, 8, 3, 4, 2, true>(),
-      make_split_variant32<32, 8, 3, 2, 4, false>(), make_split_variant32<32, 8, 3, 4, 2, false>(),
-      make_split_variant32<32, 16, 1, 4, 2, true>(), make_split_variant32<32, 4, 6, 4, 2, true>(),
-      make_split_variant32<64, 4, 3, 4, 2, true>(), make_split_variant32<32, 8, 3, 2, 3, true>()};
+      make_split_variant32<4, 1, 4, 4, 4, 4>(), make_split_variant32<4, 1, 5, 4, 3, 5>(),
+      make_split_variant32<4, 1, 6, 4, 2, 6>(), make_split_variant32<2, 1, 4, 2, 3, 5>(),
+      make_split_variant32<2, 1, 4, 1, 2, 6>()};
   return v;
 }
 
@@ -1227,7 +1136,8 @@ static dim3 grid32_of(const Stepper32 *h, int variant, int *zc_out) {
   *zc_out = 1;
   if (h->d.dim == 1) return dim3((unsigned)((P.nx + kTX1_32 - 1) / kTX1_32));
   const Variant32 &v = variants32()[variant];
-  const unsigned gx = (unsigned)((P.nx + v.tx - 1) / v.tx), gy = (unsigned)((P.ny + v.ty - 1) / v.ty);
+  const int ty = h->d.dim == 2 && v.ty2 ? v.ty2 : v.ty;
+  const unsigned gx = (unsigned)((P.nx + v.tx - 1) / v.tx), gy = (unsigned)((P.ny + ty - 1) / ty);
   if (h->d.dim == 2) return dim3(gx, gy, 1);
   const int64_t tiles = (int64_t)gx * gy;
   const int64_t target = (int64_t)sm_count() * v.minb * 4;
@@ -1582,9 +1492,9 @@ pf5d_status s32_step_save_inputs(Stepper32 *h, double *X_out, double *dX_out, do
   pf5d_status st = launch_rate32(h, s);
   if (st != PF5D_OK) return st;
   switch (h->d.dim) {
-    case 1: chem32_attrs<1, 2, 3>(); launch_chem32<1, 2, 3>(s, h->rp); break;
-    case 2: chem32_attrs<2, 2, 3>(); launch_chem32<2, 2, 3>(s, h->rp); break;
-    default: chem32_attrs<3, 2, 3>(); launch_chem32<3, 2, 3>(s, h->rp);
+    case 1: launch_chem32<1, 4, 4, 4>(s, h->rp); break;
+    case 2: launch_chem32<2, 4, 4, 4>(s, h->rp); break;
+    default: launch_chem32<3, 4, 4, 4>(s, h->rp);
   }
   PF5D_LAUNCHED();
   k32_join<<<grid_for(h->npts, 256, 4), 256, 0, s>>>(h->hi, h->lo, h->npts, h->up, X_out);

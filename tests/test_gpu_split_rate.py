@@ -27,27 +27,32 @@ def _field(kind, shape, rng):
     return rng.dirichlet(np.full(5, 3.0), size=shape)[..., 1:]      # all over, some far
 
 
-def _run(prob, X, variant, table):
+def _run(prob, X, variant, table, precision="fp64"):
+    """Field and dX/dt after two steps (the precision form's dX/dt is float32
+    and not compared)."""
     from phasefield5d_b200.stepper import Stepper
     st = Stepper(grid=prob.grid, resolution=prob.cfg.resolution, node_coord=prob.node_coord, X=X,
                  X0=prob.X0, kappa=prob.kappa, dx=prob.dx, lvec=prob.lvec, bk=prob.bk,
-                 ctld=prob.ctld, t_cfl=prob.t_cfl, dt=1e-3 * prob.t_cfl, autotune=False, table=table)
+                 ctld=prob.ctld, t_cfl=prob.t_cfl, dt=1e-3 * prob.t_cfl, autotune=False, table=table,
+                 precision=precision)
     st.set_variant(variant)
     st.run(2)
-    out = st.X.cpu().numpy(), st.rate().cpu().numpy()
+    state = st.state()
+    out = (st.field().cpu().numpy(),
+           st.rate().cpu().numpy() if precision == "fp64" else np.array([state["xdotmax"]]))
     st.close()
     return out
 
 
-def _split_variants(prob):
+def _split_variants(prob, precision="fp64"):
     from phasefield5d_b200.stepper import Stepper
-    st = Stepper.from_problem(prob, autotune=False)
+    st = Stepper.from_problem(prob, autotune=False, precision=precision)
     names = []
     for v in range(st.n_variants):
         st.set_variant(v)
         names.append(st.rate_kernels)
     st.close()
-    return [v for v, n in enumerate(names) if n.startswith("k_chem")]
+    return [v for v, n in enumerate(names) if n.startswith(("k_chem", "k32_chem"))]
 
 
 @pytest.mark.parametrize("kind", ["cell", "node", "spread"])
@@ -66,3 +71,19 @@ def test_split_rate_bitwise_equals_fused(torch_cuda, shape, kind):
         for table in (None, table9):
             got = _run(prob, X, v, table)
             assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1]), (v, table is None)
+
+
+@pytest.mark.parametrize("kind", ["cell", "node", "spread"])
+@pytest.mark.parametrize("shape", [(3, 5), (16, 32), (17, 33), (50, 130), (4, 4, 32), (3, 5, 33),
+                                   (5, 9, 65), (9, 17, 31), (2, 3, 4)])
+def test_split_rate_fp32c_bitwise_equals_fused(torch_cuda, shape, kind):
+    from phasefield5d_b200 import workload as W
+    cfg = W.SolveConfig(system_dim=len(shape), initial_composition=(0.1, 0.2, 0.2, 0.25),
+                        resolution=0.05, kappa_value=5e-16, mw=4, ppw=16, shape=shape, n_k=500)
+    prob = W.build_problem(cfg)
+    X = _field(kind, shape, np.random.default_rng(3))
+    ref = _run(prob, X, 0, None, "fp32c")
+    assert np.isfinite(ref[0]).all() and ref[1].max() > 0
+    for v in _split_variants(prob, "fp32c"):
+        got = _run(prob, X, v, None, "fp32c")
+        assert np.array_equal(got[0], ref[0]) and np.array_equal(got[1], ref[1]), v
