@@ -349,34 +349,34 @@ __device__ __forceinline__ void mu_plane64(const RateParams &P, const double *Xm
 // every point of a field into P.mm, each point once.  The table
 // values come first (pf5d_gather.cuh), then each thread takes its own points
 // in order: Laplacian (operators.py:49-76: +axis0, -axis0, +axis1, ...), then
-// mu = v - lap*kappa (+ s' * l).  A block's points are 512 in a row (1D), 32
-// columns by 16 rows (2D), or 32 columns by 4 rows by 4 planes (3D), and a
-// thread's four are consecutive along y (2D) or z (3D), so it loads each point
-// of that axis once.
+// mu = v - lap*kappa (+ s' * l).  A block's points are 128 PER in a row (1D),
+// 32 columns by 4 PER rows (2D), or 32 columns by 4 rows by PER planes (3D),
+// and a thread's PER are consecutive along y (2D) or z (3D), so it loads each
+// point of that axis once.
 //
 // Bound by the L1 data path (67% of its wavefronts' rate at 128x256x256, FP64
 // pipe 38%).  One point per thread (1.21 ms at 256^3, on-node composition)
 // moved every node into registers once per point; with K = 3 points of a cell
 // per load it is 0.99 ms.  K = 4 needs 168 registers, and the 12 warps per SM
 // that leaves lose more (1.18) than the fewer loads give; K = 2 with the same
-// 16 warps is 1.01.  512 points per block keep a cell's run longer than K in
-// fields that spread over many cells: with 256 points 1.05, 1.24 against 1.05
-// ms in a field of two phases.
-constexpr int kChemNT = 128, kChemPer = 4, kChemK = 3, kChemMinB = 4;
-using ChemSmem = GatherSmem<kChemNT, kChemPer, kChemK>;
+// 16 warps is 1.01.  PER = 4 keeps a cell's run longer than K in fields that
+// spread over many cells (rate stage with two phases: 1.97 ms, PER = 2 2.11);
+// below about 400^2 points its blocks leave SMs idle, and PER = 2 takes over:
+// 389x250 rate stage 22.0 -> 17.6 us (27.4 -> 22.1 with two phases).
+constexpr int kChemNT = 128, kChemMinB = 4;
 
-template <int DIM>
+template <int DIM, int PER>
 struct ChemTile {
-  static constexpr int BX = DIM == 1 ? kChemNT * kChemPer : 32;
-  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? kChemNT / 32 * kChemPer : kChemNT / 32);
-  static constexpr int BZ = DIM == 3 ? kChemPer : 1;
+  static constexpr int BX = DIM == 1 ? kChemNT * PER : 32;
+  static constexpr int BY = DIM == 1 ? 1 : (DIM == 2 ? kChemNT / 32 * PER : kChemNT / 32);
+  static constexpr int BZ = DIM == 3 ? PER : 1;
 };
 
-template <int DIM, bool VEC>
+template <int DIM, bool VEC, int PER, int K>
 __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
-  using G = ChemTile<DIM>;
-  constexpr int NT = kChemNT, PER = kChemPer;
-  __shared__ ChemSmem g;
+  using G = ChemTile<DIM, PER>;
+  constexpr int NT = kChemNT;
+  __shared__ GatherSmem<NT, PER, K> g;
   pdl_wait();
   if (P.st->halt) return;
   const double *X = after_wait(P.X);
@@ -1689,18 +1689,18 @@ RateVariant make_variant() {
 }
 
 // The split form's mu/M kernel.
-template <int DIM>
+template <int DIM, int PER, int K>
 void launch_chem(bool vec, cudaStream_t s, const RateParams &P) {
-  using G = ChemTile<DIM>;
+  using G = ChemTile<DIM, PER>;
   const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
                (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-  if (vec) launch_pdl(k_chem<DIM, true>, g, dim3(kChemNT), 0, s, P);
-  else launch_pdl(k_chem<DIM, false>, g, dim3(kChemNT), 0, s, P);
+  if (vec) launch_pdl(k_chem<DIM, true, PER, K>, g, dim3(kChemNT), 0, s, P);
+  else launch_pdl(k_chem<DIM, false, PER, K>, g, dim3(kChemNT), 0, s, P);
 }
 
 // Split variant: k_chem, then k_flux; in 2D a warp marches over ROWS rows (in
 // 3D rate_grid_of sets the planes of a chunk).
-template <int ROWS, int R, int MINB>
+template <int ROWS, int R, int MINB, int PER, int K>
 RateVariant make_split_variant() {
   RateVariant v;
   v.tx = kFluxCols;
@@ -1713,15 +1713,15 @@ RateVariant make_split_variant() {
   v.smem2d = v.smem3d = 0;
   v.set_attrs = [](bool) {};
   v.launch2d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P) {
-    launch_chem<2>(vec, s, P);
+    launch_chem<2, PER, K>(vec, s, P);
     launch_pdl(k_flux<2, 1, MINB>, g, dim3(kFluxThreads), 0, s, P, ROWS);
   };
   v.launch3d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P, int zc) {
-    launch_chem<3>(vec, s, P);
+    launch_chem<3, PER, K>(vec, s, P);
     launch_pdl(k_flux<3, R, MINB>, g, dim3(kFluxThreads), 0, s, P, zc);
   };
   v.kernels = [](bool vec, int dim) {
-    return kname("k_chem", {dim, vec}) + " + " + kname("k_flux", {dim, dim == 2 ? 1 : R, MINB});
+    return kname("k_chem", {dim, vec, PER, K}) + " + " + kname("k_flux", {dim, dim == 2 ? 1 : R, MINB});
   };
   return v;
 }
@@ -1738,7 +1738,8 @@ const std::vector<RateVariant> &rate_variants() {
       make_variant<32, 8, 2, false, 256, 2, true>(), make_variant<32, 8, 2, false, 256, 2, false>(),
       make_variant<32, 4, 4, false, 128, 2, true>(),
       make_variant<32, 8, 3, false, 256, false, true>(), make_variant<64, 4, 2, true, 256, false, true>(),
-      make_split_variant<4, 1, 3>(), make_split_variant<2, 1, 3>(), make_split_variant<8, 2, 2>()};
+      make_split_variant<4, 1, 3, 4, 3>(), make_split_variant<2, 1, 3, 2, 2>(),
+      make_split_variant<2, 1, 3, 2, 3>(), make_split_variant<4, 2, 2, 4, 2>()};
   return v;
 }
 
@@ -2292,9 +2293,9 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
     if ((st = launch_rate(h, s)) != PF5D_OK) return st;
     // mu and M of this step at every point, then the "before" reductions
     switch (dim) {
-      case 1: launch_chem<1>(h->vec, s, h->rp); break;
-      case 2: launch_chem<2>(h->vec, s, h->rp); break;
-      default: launch_chem<3>(h->vec, s, h->rp);
+      case 1: launch_chem<1, 4, 3>(h->vec, s, h->rp); break;
+      case 2: launch_chem<2, 4, 3>(h->vec, s, h->rp); break;
+      default: launch_chem<3, 4, 3>(h->vec, s, h->rp);
     }
     PF5D_LAUNCHED();
     Xpre = h->X;
