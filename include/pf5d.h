@@ -227,12 +227,13 @@ pf5d_status pf5d_stepper_mass(pf5d_stepper *h, double *mean_out, void *stream);
  * stepper's state exactly as that stage does inside a step. */
 #define PF5D_STAGE_RATE 0        /* rate kernel(s) (mu/M + flux divergence) and the dt controller */
 #define PF5D_STAGE_UPDATE 1      /* update, clamp, next misfit, OOB test       */
-#define PF5D_STAGE_FFT_FWD 2     /* cuFFT D2Z of the misfit (2D with a power-of-two
-                                    axis 0 up to 1024: the row D2Z); 1D solves up to
+#define PF5D_STAGE_FFT_FWD 2     /* cuFFT D2Z of the misfit (2D, and FP64 3D, with a
+                                    power-of-two axis 0 from 8 to 1024: over the
+                                    other axes only); 1D solves up to
                                     16384 points: the whole elastic term in closed form */
-#define PF5D_STAGE_BMUL 3        /* B(k) multiply (2D column pass: axis-0 transform,
+#define PF5D_STAGE_BMUL 3        /* B(k) multiply (column pass: axis-0 transform,
                                     multiply, inverse; nothing in the 1D closed form) */
-#define PF5D_STAGE_FFT_INV 4     /* cuFFT Z2D (2D column pass: the row Z2D; nothing in
+#define PF5D_STAGE_FFT_INV 4     /* cuFFT Z2D (column pass: over the other axes; nothing in
                                     the 1D closed form)                          */
 pf5d_status pf5d_stepper_launch_stage(pf5d_stepper *h, int32_t stage, void *stream);
 /* Autotuner: time every rate-kernel variant (plane tile shape x resident
@@ -278,8 +279,7 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
 int32_t pf5d_stepper_variant_count(const pf5d_stepper *h);
 /* Kernels of this library that one step launches with the current variant
  * (rate kernel(s), dt controller, update, and when elasticity is on the B(k)
- * multiply or, in 2D with a power-of-two axis 0, the column kernel; cuFFT's
- * own kernels not counted); 1 for a 1D solve that the step loop advances (one
+ * multiply or the column kernel in its place; cuFFT's own kernels not counted); 1 for a 1D solve that the step loop advances (one
  * launch for up to 2000 steps); 0 for a null stepper. */
 int32_t pf5d_stepper_launches_per_step(const pf5d_stepper *h);
 /* The kernel instances one rate stage of the current variant launches, as

@@ -10,7 +10,7 @@
 
 #include "pf5d_device.cuh"
 #include "pf5d_fft.h"
-#include "pf5d_stockham.cuh"
+#include "pf5d_colfft.cuh"
 
 namespace pf5d {
 
@@ -66,67 +66,67 @@ pf5d_status fft_inverse(FFTPair *p, cufftDoubleComplex *k, double *s, cudaStream
 }
 
 // ------------------------------------------------------------------------
-// 2D column pass: for a group of kColGroup spectrum columns (axis-1 indices
-// of the row transforms' output), the length-N0 transform along axis 0, the
-// B(k)/N multiply and the inverse transform, in shared memory.  Transforms:
-// mixed-radix Stockham autosort (radix-8 stages, then one radix-4 or radix-2
-// stage; natural order after every stage), forward exp(-2 pi i jk/N0),
-// inverse exp(+2 pi i jk/N0), both unnormalised like cuFFT's (the 1/N is
-// in B).
+// Column pass: along axis 0 of the spectrum, the length-N transform, the
+// B(k)/N multiply and the inverse transform, COLS neighbouring columns per
+// block (N / 8 threads each, pf5d_colfft.cuh); the spectrum is read and written
+// once.  The twiddles and B(k) do not depend on the kernel before, so they are
+// loaded ahead of the wait for it.
+//
+// Bound by latency in 2D (one round of blocks): 512^2 8.4 us as one 256-thread
+// block per column with every stage in shared memory, 4.4 here, the whole term
+// 14.5 -> 10.0 (FP32c 12.5 -> 8.1), with the same bits.  By HBM in 3D: 256^3
+// 84 us for 0.68 GB (8.1 TB/s of which L2 serves a part), the whole term
+// 364 us with cuFFT's 3D plans and a separate multiply -> 312; 64x100x90
+// 26 -> 19.5.  The precision form keeps the 3D plans: its elastic term is FP32,
+// and another order of roundings there shows in late fields (4e-10 of X).
 // ------------------------------------------------------------------------
-constexpr int kColGroup = 1;
-
-template <typename C, int N0>
-__global__ void __launch_bounds__(kColThreads)
-    k_colpass(C *__restrict__ k, const typename CT<C>::R *__restrict__ bk, int nk1,
-              const C *__restrict__ tw, const unsigned *halt) {
+template <typename C, int N, int COLS>
+__global__ void __launch_bounds__(N / 8 * COLS)
+    k_colpass(C *__restrict__ k, const typename CT<C>::R *__restrict__ bk, int64_t ncol,
+              const C *__restrict__ table, const unsigned *halt) {
+  using F = ColFFT<C, N, COLS>;
   extern __shared__ __align__(16) unsigned char craw[];
-  C *cbuf = reinterpret_cast<C *>(craw);             // [2][kColGroup][N0]
+  C *buf = reinterpret_cast<C *>(craw);
+  const int cc = threadIdx.x % COLS, t = threadIdx.x / COLS;
+  const int64_t c = (int64_t)blockIdx.x * COLS + cc;
+  const bool valid = c < ncol;
+  F fft;
+  fft.load_twiddles(table, t);
+  typename CT<C>::R m[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) m[r] = valid ? __ldg(bk + (int64_t)(t + F::T * r) * ncol + c) : 0;
+  pdl_wait();
   if (halt && *halt) return;
-  const int tid = threadIdx.x, c0 = blockIdx.x * kColGroup;
-  C *a = cbuf, *b = cbuf + kColGroup * N0;
-  C *kk = k;
-  for (int e = tid; e < kColGroup * N0; e += kColThreads) {
-    const int r = e / kColGroup, cc = e - r * kColGroup, c = c0 + cc;
-    a[cc * N0 + r] = c < nk1 ? kk[(int64_t)r * nk1 + c] : cmk<C>(0, 0);
-  }
-  __syncthreads();
-  C *f = stockham<C, N0, false>(a, b, tw, tid);
-  C *g = f == a ? b : a;
-  for (int e = tid; e < kColGroup * N0; e += kColThreads) {
-    const int cc = e / N0, r = e - cc * N0, c = c0 + cc;
-    const typename CT<C>::R m = c < nk1 ? bk[(int64_t)r * nk1 + c] : 0;
-    C v = f[e];
-    v.x = v.x * m;
-    v.y = v.y * m;
-    f[e] = v;
-  }
-  __syncthreads();
-  f = stockham<C, N0, true>(f, g, tw, tid);
-  for (int e = tid; e < kColGroup * N0; e += kColThreads) {
-    const int r = e / kColGroup, cc = e - r * kColGroup, c = c0 + cc;
-    if (c < nk1) kk[(int64_t)r * nk1 + c] = f[cc * N0 + r];
-  }
+  C v[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) v[r] = valid ? k[(int64_t)(t + F::T * r) * ncol + c] : cmk<C>(0, 0);
+  fft.template run<false>(v, buf, t, cc);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) v[r] = cmk<C>(v[r].x * m[r], v[r].y * m[r]);
+  fft.template run<true>(v, buf, t, cc);
+  if (!valid) return;
+#pragma unroll
+  for (int r = 0; r < 8; ++r) k[(int64_t)(t + F::T * r) * ncol + c] = v[r];
 }
 
 template <typename C>
-static pf5d_status colpass_dispatch(const ColPass2D *c, C *k, const typename CT<C>::R *bk,
+static pf5d_status colpass_dispatch(const ColPass *c, C *k, const typename CT<C>::R *bk,
                                     const C *tw, const unsigned *halt, cudaStream_t stream);
 
-pf5d_status colpass_create(const int64_t *shape, ColPass2D *c, bool fp32) {
-  const int64_t n0 = shape[0], n1 = shape[1];
-  PF5D_REQUIRE(n0 >= 8 && n0 <= 1024 && (n0 & (n0 - 1)) == 0 && n1 >= 2, PF5D_ERR_ARG,
+pf5d_status colpass_create(int dim, const int64_t *shape, ColPass *c, bool fp32) {
+  const int64_t n0 = shape[0], last = shape[dim - 1];
+  PF5D_REQUIRE((dim == 2 || dim == 3) && colpass_fits(n0) && last >= 2, PF5D_ERR_ARG,
                "column pass needs a power-of-two axis 0 in [8, 1024]");
   c->n0 = (int)n0;
-  c->nk1 = (int)(n1 / 2 + 1);
+  c->ncol = (dim == 3 ? shape[1] : 1) * (last / 2 + 1);
   c->fp32 = fp32;
-  long long n[1] = {(long long)n1};
+  long long n[2] = {(long long)shape[1], (long long)last};
   size_t ws = 0;
   PF5D_CUFFT(cufftCreate(&c->rfwd));
-  PF5D_CUFFT(cufftMakePlanMany64(c->rfwd, 1, n, nullptr, 1, 0, nullptr, 1, 0,
+  PF5D_CUFFT(cufftMakePlanMany64(c->rfwd, dim - 1, n, nullptr, 1, 0, nullptr, 1, 0,
                                  fp32 ? CUFFT_R2C : CUFFT_D2Z, n0, &ws));
   PF5D_CUFFT(cufftCreate(&c->rinv));
-  PF5D_CUFFT(cufftMakePlanMany64(c->rinv, 1, n, nullptr, 1, 0, nullptr, 1, 0,
+  PF5D_CUFFT(cufftMakePlanMany64(c->rinv, dim - 1, n, nullptr, 1, 0, nullptr, 1, 0,
                                  fp32 ? CUFFT_C2R : CUFFT_Z2D, n0, &ws));
   c->ready = true;
   // exp(-2 pi i m / n0) in FP64, rounded once for the FP32 form
@@ -148,7 +148,7 @@ pf5d_status colpass_create(const int64_t *shape, ColPass2D *c, bool fp32) {
   return colpass_dispatch<double2>(c, nullptr, nullptr, nullptr, nullptr, nullptr);
 }
 
-void colpass_destroy(ColPass2D *c) {
+void colpass_destroy(ColPass *c) {
   if (c->ready) {
     cufftDestroy(c->rfwd);
     cufftDestroy(c->rinv);
@@ -160,67 +160,78 @@ void colpass_destroy(ColPass2D *c) {
   c->ready = false;
 }
 
-pf5d_status colpass_rows_forward(ColPass2D *c, double *s, cufftDoubleComplex *k,
+pf5d_status colpass_rows_forward(ColPass *c, double *s, cufftDoubleComplex *k,
                                  cudaStream_t stream) {
   PF5D_CUFFT(cufftSetStream(c->rfwd, stream));
   PF5D_CUFFT(cufftExecD2Z(c->rfwd, s, k));
   return PF5D_OK;
 }
 
-pf5d_status colpass_rows_inverse(ColPass2D *c, cufftDoubleComplex *k, double *s,
+pf5d_status colpass_rows_inverse(ColPass *c, cufftDoubleComplex *k, double *s,
                                  cudaStream_t stream) {
   PF5D_CUFFT(cufftSetStream(c->rinv, stream));
   PF5D_CUFFT(cufftExecZ2D(c->rinv, k, s));
   return PF5D_OK;
 }
 
-template <typename C, int N0>
-static pf5d_status launch_colpass(const ColPass2D *c, C *k, const typename CT<C>::R *bk,
+template <typename C, int N, int COLS>
+static pf5d_status launch_colpass(const ColPass *c, C *k, const typename CT<C>::R *bk,
                                   const C *tw, const unsigned *halt, cudaStream_t stream) {
-  const int smem = 2 * N0 * (int)sizeof(C);
+  const int smem = N * COLS * (int)sizeof(C);
   if (!k) {                          // set-up call from colpass_create
-    PF5D_CUDA(cudaFuncSetAttribute(k_colpass<C, N0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   smem));
+    PF5D_CUDA(cudaFuncSetAttribute(k_colpass<C, N, COLS>,
+                                   cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     return PF5D_OK;
   }
-  k_colpass<C, N0><<<(unsigned)c->nk1, kColThreads, smem, stream>>>(k, bk, c->nk1, tw, halt);
-  PF5D_LAUNCHED();
+  PF5D_CUDA(launch_pdl(k_colpass<C, N, COLS>, dim3((unsigned)((c->ncol + COLS - 1) / COLS)),
+                       dim3(N / 8 * COLS), smem, stream, k, bk, c->ncol, tw, halt));
   return PF5D_OK;
 }
 
+// Columns per block: 8 fill whole lines, but a 2D spectrum has too few columns
+// for that many per SM; 2 there.
+template <typename C, int N>
+static pf5d_status launch_columns(const ColPass *c, C *k, const typename CT<C>::R *bk,
+                                  const C *tw, const unsigned *halt, cudaStream_t stream) {
+  constexpr int MANY = N <= 512 ? 8 : 4;
+  if (c->ncol >= (int64_t)sm_count() * 2 * MANY)
+    return launch_colpass<C, N, MANY>(c, k, bk, tw, halt, stream);
+  return launch_colpass<C, N, 2>(c, k, bk, tw, halt, stream);
+}
+
 template <typename C>
-static pf5d_status colpass_dispatch(const ColPass2D *c, C *k, const typename CT<C>::R *bk,
+static pf5d_status colpass_dispatch(const ColPass *c, C *k, const typename CT<C>::R *bk,
                                     const C *tw, const unsigned *halt, cudaStream_t stream) {
   switch (c->n0) {
-    case 8: return launch_colpass<C, 8>(c, k, bk, tw, halt, stream);
-    case 16: return launch_colpass<C, 16>(c, k, bk, tw, halt, stream);
-    case 32: return launch_colpass<C, 32>(c, k, bk, tw, halt, stream);
-    case 64: return launch_colpass<C, 64>(c, k, bk, tw, halt, stream);
-    case 128: return launch_colpass<C, 128>(c, k, bk, tw, halt, stream);
-    case 256: return launch_colpass<C, 256>(c, k, bk, tw, halt, stream);
-    case 512: return launch_colpass<C, 512>(c, k, bk, tw, halt, stream);
-    case 1024: return launch_colpass<C, 1024>(c, k, bk, tw, halt, stream);
+    case 8: return launch_columns<C, 8>(c, k, bk, tw, halt, stream);
+    case 16: return launch_columns<C, 16>(c, k, bk, tw, halt, stream);
+    case 32: return launch_columns<C, 32>(c, k, bk, tw, halt, stream);
+    case 64: return launch_columns<C, 64>(c, k, bk, tw, halt, stream);
+    case 128: return launch_columns<C, 128>(c, k, bk, tw, halt, stream);
+    case 256: return launch_columns<C, 256>(c, k, bk, tw, halt, stream);
+    case 512: return launch_columns<C, 512>(c, k, bk, tw, halt, stream);
+    case 1024: return launch_columns<C, 1024>(c, k, bk, tw, halt, stream);
     default: set_error("column pass: unsupported n0 %d", c->n0); return PF5D_ERR_ARG;
   }
 }
 
-pf5d_status colpass_columns(ColPass2D *c, cufftDoubleComplex *k, const double *bk,
+pf5d_status colpass_columns(ColPass *c, cufftDoubleComplex *k, const double *bk,
                             const unsigned *halt, cudaStream_t stream) {
   return colpass_dispatch<double2>(c, reinterpret_cast<double2 *>(k), bk, c->tw, halt, stream);
 }
 
-pf5d_status colpass_columns32(ColPass2D *c, cufftComplex *k, const float *bk,
+pf5d_status colpass_columns32(ColPass *c, cufftComplex *k, const float *bk,
                               const unsigned *halt, cudaStream_t stream) {
   return colpass_dispatch<float2>(c, reinterpret_cast<float2 *>(k), bk, c->tw32, halt, stream);
 }
 
-pf5d_status colpass_rows_forward32(ColPass2D *c, float *s, cufftComplex *k, cudaStream_t stream) {
+pf5d_status colpass_rows_forward32(ColPass *c, float *s, cufftComplex *k, cudaStream_t stream) {
   PF5D_CUFFT(cufftSetStream(c->rfwd, stream));
   PF5D_CUFFT(cufftExecR2C(c->rfwd, s, k));
   return PF5D_OK;
 }
 
-pf5d_status colpass_rows_inverse32(ColPass2D *c, cufftComplex *k, float *s, cudaStream_t stream) {
+pf5d_status colpass_rows_inverse32(ColPass *c, cufftComplex *k, float *s, cudaStream_t stream) {
   PF5D_CUFFT(cufftSetStream(c->rinv, stream));
   PF5D_CUFFT(cufftExecC2R(c->rinv, k, s));
   return PF5D_OK;

@@ -25,34 +25,36 @@ void fft_destroy(FFTPair *p);
 pf5d_status fft_forward(FFTPair *p, double *s, cufftDoubleComplex *k, cudaStream_t stream);
 pf5d_status fft_inverse(FFTPair *p, cufftDoubleComplex *k, double *s, cudaStream_t stream);
 
-// 2D elastic term in three passes instead of cuFFT's four plus the multiply:
-// row D2Z over axis 1 (cuFFT, batched over the n0 rows), then ONE kernel per
-// group of spectrum columns that runs the length-n0 transform along axis 0,
-// multiplies by B(k)/N and runs the inverse transform back (k_colpass), then
-// row Z2D.  Used when n0 is a power of two in [8, 1024].
-struct ColPass2D {
-  cufftHandle rfwd = 0, rinv = 0;     // batched row transforms
-  int n0 = 0, nk1 = 0;                // rows, spectrum columns (n1/2 + 1)
+// 2D and 3D elastic term in three passes: batched transforms over the other
+// axes (cuFFT; rows in 2D, planes in 3D), then ONE kernel that runs the
+// transform along axis 0, multiplies by B(k)/N and runs the inverse transform
+// back (k_colpass), then the inverse batched transforms.  Used when axis 0 is a
+// power of two in [8, 1024].
+struct ColPass {
+  cufftHandle rfwd = 0, rinv = 0;     // batched row (2D) / plane (3D) transforms
+  int n0 = 0;
+  int64_t ncol = 0;                   // spectrum columns along axis 0
   double2 *tw = nullptr;              // exp(-2 pi i m / n0), m < n0 (FP64 form)
   float2 *tw32 = nullptr;             // the same rounded to FP32 (FP32c form)
-  bool fp32 = false;                  // FP32c: R2C / C2R rows, float2 spectrum
+  bool fp32 = false;                  // FP32c: R2C / C2R, float2 spectrum
   bool ready = false;
 };
 
-pf5d_status colpass_create(const int64_t *shape, ColPass2D *c, bool fp32);
-void colpass_destroy(ColPass2D *c);
+inline bool colpass_fits(int64_t n0) { return n0 >= 8 && n0 <= 1024 && (n0 & (n0 - 1)) == 0; }
+pf5d_status colpass_create(int dim, const int64_t *shape, ColPass *c, bool fp32);
+void colpass_destroy(ColPass *c);
 // s -> s' in place through k (scratch spectrum), bk = B(k)/N on the half grid.
-pf5d_status colpass_rows_forward(ColPass2D *c, double *s, cufftDoubleComplex *k,
+pf5d_status colpass_rows_forward(ColPass *c, double *s, cufftDoubleComplex *k,
                                  cudaStream_t stream);
-pf5d_status colpass_columns(ColPass2D *c, cufftDoubleComplex *k, const double *bk,
+pf5d_status colpass_columns(ColPass *c, cufftDoubleComplex *k, const double *bk,
                             const unsigned *halt, cudaStream_t stream);
-pf5d_status colpass_rows_inverse(ColPass2D *c, cufftDoubleComplex *k, double *s,
+pf5d_status colpass_rows_inverse(ColPass *c, cufftDoubleComplex *k, double *s,
                                  cudaStream_t stream);
 // The FP32c form's passes (float field, cufftComplex spectrum, B(k)/N in FP32).
-pf5d_status colpass_rows_forward32(ColPass2D *c, float *s, cufftComplex *k, cudaStream_t stream);
-pf5d_status colpass_columns32(ColPass2D *c, cufftComplex *k, const float *bk,
+pf5d_status colpass_rows_forward32(ColPass *c, float *s, cufftComplex *k, cudaStream_t stream);
+pf5d_status colpass_columns32(ColPass *c, cufftComplex *k, const float *bk,
                               const unsigned *halt, cudaStream_t stream);
-pf5d_status colpass_rows_inverse32(ColPass2D *c, cufftComplex *k, float *s, cudaStream_t stream);
+pf5d_status colpass_rows_inverse32(ColPass *c, cufftComplex *k, float *s, cudaStream_t stream);
 
 struct Vec4 {
   double v[4];

@@ -1094,7 +1094,7 @@ const std::vector<Variant32> &variants32() {
 struct Stepper32 {
   pf5d_stepper_desc d{};
   bool closed1d = false;         // 1D elastic term in closed form (k32_elastic1d)
-  ColPass2D colp;                // 2D elastic term: row transforms + one column kernel
+  ColPass colp;                // elastic term: batched transforms + one column kernel
   bool use_colpass = false;
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
   bool use_loop1d = false;       // 1D steps by k32_loop1d
@@ -1323,9 +1323,8 @@ pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void
       set_error("device allocation failed");
       return fail(PF5D_ERR_CUDA);
     }
-    const int64_t n0 = h->shape[0];
-    if (desc->dim == 2 && n0 >= 8 && n0 <= 1024 && (n0 & (n0 - 1)) == 0) {
-      h->use_colpass = colpass_create(h->shape, &h->colp, true) == PF5D_OK;
+    if (desc->dim == 2 && colpass_fits(h->shape[0])) {
+      h->use_colpass = colpass_create(desc->dim, h->shape, &h->colp, true) == PF5D_OK;
       if (!h->use_colpass) colpass_destroy(&h->colp);
     }
   }

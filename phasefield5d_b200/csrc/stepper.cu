@@ -6,6 +6,8 @@
 //      previous step, or by k_misfit at start)
 //   2. k_bmul: S(k) *= B(k)/N
 //   3. cuFFT Z2D -> s'(x)
+//      (2D and 3D with a power-of-two axis 0: 1 and 3 over the other axes,
+//      and k_colpass for axis 0 and the multiply)
 //   4. k_rate_*: fused chemical potential + flux divergence.  Per tile of a
 //      plane (x fastest), marching plane by plane along axis 0:
 //        - X planes with a 2-cell halo staged in shared memory (ring of 3),
@@ -1615,7 +1617,7 @@ struct pf5d_stepper {
   double *diag_ws = nullptr;     // save-step partial rows + mean
   double *partial = nullptr;     // rate kernel block maxima
   bool closed1d = false;         // 1D elastic term in closed form (k_elastic1d)
-  ColPass2D colp;                // 2D elastic term: row transforms + one column kernel
+  ColPass colp;                // elastic term: batched transforms + one column kernel
   bool use_colpass = false;
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
   bool use_loop1d = false;       // 1D steps by k_loop1d
@@ -2052,9 +2054,8 @@ pf5d_status pf5d_stepper_create(const pf5d_stepper_desc *desc, double *X, void *
   if (desc->elastic) {
     if ((st = fft_create(desc->dim, h->shape, &h->fft)) != PF5D_OK) return fail(st);
     if ((st = upload_bk_scaled(desc->bk, h->fft.nk, npts, &h->bk)) != PF5D_OK) return fail(st);
-    const int64_t n0 = h->shape[0];
-    if (desc->dim == 2 && n0 >= 8 && n0 <= 1024 && (n0 & (n0 - 1)) == 0) {
-      h->use_colpass = colpass_create(h->shape, &h->colp, false) == PF5D_OK;
+    if (desc->dim >= 2 && colpass_fits(h->shape[0])) {
+      h->use_colpass = colpass_create(desc->dim, h->shape, &h->colp, false) == PF5D_OK;
       if (!h->use_colpass) colpass_destroy(&h->colp);
     }
     if (cudaMalloc(&h->s, npts * sizeof(double)) != cudaSuccess ||
