@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "pf5d_device.cuh"
+#include "pf5d_gather.cuh"
 #include "pf5d_host.h"
 
 namespace pf5d {
@@ -91,6 +92,46 @@ __global__ void k_laplacian(int dim, int64_t n0, int64_t n1, int64_t n2, int nc,
   }
 }
 
+// Four components in 16-byte aligned rows, one point per thread: a block is 32
+// columns by 8 rows of a plane, so a point's in-plane neighbours are its own
+// lines.  Bound by the reads: 128^3 72 us with 64-bit index arithmetic and scalar
+// loads -> 35.
+template <int DIM, int W>
+__global__ void __launch_bounds__(256) k_laplacian4(int n0, int n1, int n2,
+                                                    const double *__restrict__ c, double inv_dx2,
+                                                    double *__restrict__ out) {
+  // (z, y, x) of the point: axes from the back, the missing ones of length 1
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z;
+  const int nx = DIM == 1 ? n0 : (DIM == 2 ? n1 : n2), ny = DIM == 1 ? 1 : (DIM == 2 ? n0 : n1);
+  const int nz = DIM == 3 ? n0 : 1;
+  if (x >= nx || y >= ny) return;
+  auto at = [&](int zz, int yy, int xx) { return 4 * (((int64_t)zz * ny + yy) * nx + xx); };
+  double v[S], lap[S], a[S], b[S];
+  load_comp4<W>(c + at(z, y, x), v);
+  if (DIM == 3) {
+    load_comp4<W>(c + at(z + 1 == nz ? 0 : z + 1, y, x), a);
+    load_comp4<W>(c + at(z == 0 ? nz - 1 : z - 1, y, x), b);
+#pragma unroll
+    for (int s = 0; s < S; ++s) lap[s] = a[s] + b[s];
+  }
+  if (DIM >= 2) {
+    load_comp4<W>(c + at(z, y + 1 == ny ? 0 : y + 1, x), a);
+    load_comp4<W>(c + at(z, y == 0 ? ny - 1 : y - 1, x), b);
+#pragma unroll
+    for (int s = 0; s < S; ++s) lap[s] = DIM == 3 ? (lap[s] + a[s]) + b[s] : a[s] + b[s];
+  }
+  load_comp4<W>(c + at(z, y, x + 1 == nx ? 0 : x + 1), a);
+  load_comp4<W>(c + at(z, y, x == 0 ? nx - 1 : x - 1), b);
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const double sum = DIM == 1 ? a[s] + b[s] : (lap[s] + a[s]) + b[s];
+    lap[s] = (sum - 2.0 * DIM * v[s]) * inv_dx2;
+  }
+  double2 *o = reinterpret_cast<double2 *>(out + at(z, y, x));
+  o[0] = make_double2(lap[0], lap[1]);
+  o[1] = make_double2(lap[2], lap[3]);
+}
+
 struct Kappa {
   double k[8];
 };
@@ -118,45 +159,165 @@ __device__ __forceinline__ void load5(const double *p, double v[NM]) {
   for (int s = 0; s < NM; ++s) v[s] = p[s];
 }
 
-__global__ void k_divergence(int dim, int64_t n0, int64_t n1, int64_t n2,
-                             const double *__restrict__ X, const double *__restrict__ M,
-                             int64_t ms, const double *__restrict__ mu, int64_t mus,
-                             double inv_dx, double *__restrict__ out) {
-  const int64_t npts = n0 * n1 * n2;
-  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npts;
-       p += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k = p % n2, j = (p / n2) % n1, i = p / (n2 * n1);
-    int64_t nb[6];
-    nb[0] = (wrap_p(i, n0) * n1 + j) * n2 + k;
-    nb[1] = (wrap_m(i, n0) * n1 + j) * n2 + k;
-    nb[2] = (i * n1 + wrap_p(j, n1)) * n2 + k;
-    nb[3] = (i * n1 + wrap_m(j, n1)) * n2 + k;
-    nb[4] = (i * n1 + j) * n2 + wrap_p(k, n2);
-    nb[5] = (i * n1 + j) * n2 + wrap_m(k, n2);
-    double Xc[S], Mc[NM], muc[S];
-    load4(X + p * S, Xc);
-    load5(M + p * ms, Mc);
-    load4(mu + p * mus, muc);
-    double acc[S];
-    for (int f = 0; f < 2 * dim; ++f) {
-      const int64_t q = nb[f];
-      double Xn[S], Mn[NM], mun[S], g[S], J[S];
-      load4(X + q * S, Xn);
-      load5(M + q * ms, Mn);
-      load4(mu + q * mus, mun);
+// A warp takes 32 neighbouring columns of the last axis and marches along the
+// first, as the split rate stage's k_flux: the face along the march is carried,
+// the face between columns handed on by shuffles (30 columns are finished), and
+// in 3D the rows above and below are read where the block's other warps read
+// them.  1D: no march; the faces between columns are all there is.
+// ROWS9: mu and M are the two parts of rows of nine values (interp[..., :4] and
+// interp[..., 4:]); a warp then reads its 32 rows, one run of 2304 bytes, in
+// memory order and turns them in shared memory, where loads of a column of the
+// rows would touch 18 lines each.
+// Bound by the latency of the loads.  128^3, rows of nine: 212 us with a
+// point and its six neighbours per thread -> 162.
+constexpr int kDivThreads = 128, kDivCols = 30;
+
+struct DivView {
+  const double *X, *mu, *M;
+  int64_t mus, ms;
+};
+
+struct DivPoint {
+  double x[S], mu[S], m[NM];
+};
+
+template <int DIM, bool ROWS9, int W>
+__global__ void __launch_bounds__(kDivThreads, 4)
+    k_divergence(int n0, int n1, int n2, DivView V, double inv_dx, double *__restrict__ out, int rows) {
+  __shared__ double turn[kDivThreads / 32][ROWS9 ? 32 * NP : 1];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int nx = DIM == 1 ? n0 : (DIM == 2 ? n1 : n2), ny = DIM == 3 ? n1 : 1;
+  const int nm = DIM == 1 ? 1 : n0;                    // length of the march
+  // block: column tile, then (2D) four chunks of the march or (3D) four rows,
+  // then (3D) a chunk
+  const int tiles = (nx + kDivCols - 1) / kDivCols, ny4 = (ny + 3) / 4;
+  const int rest = blockIdx.x / tiles;
+  const int tile = DIM == 1 ? blockIdx.x * 4 + w : blockIdx.x % tiles;
+  const int y = DIM == 3 ? rest % ny4 * 4 + w : 0;
+  const int64_t first64 = DIM == 1 ? 0 : (int64_t)(DIM == 3 ? rest / ny4 : rest * 4 + w) * rows;
+  if (first64 >= nm || y >= ny || tile >= tiles) return;       // whole warps
+  const int first = (int)first64, last = min(first + rows, nm);
+  const int col0 = tile * kDivCols - 1, col = col0 + lane, x = wrap_any(col, nx);
+  int off[NP];                                         // this lane's elements of a row of rows
+  if (ROWS9) {
 #pragma unroll
-      for (int s = 0; s < S; ++s) g[s] = (f & 1) ? (muc[s] - mun[s]) * inv_dx : (mun[s] - muc[s]) * inv_dx;
-      face_flux(Xc, Mc, Xn, Mn, g, J);
+    for (int k = 0; k < NP; ++k) {
+      const int e = lane + 32 * k;
+      off[k] = wrap_any(col0 + e / NP, nx) * NP + e % NP;
+    }
+  }
+  auto load = [&](int i, int yy, DivPoint &q) {
+    const int64_t line = ((int64_t)i * ny + yy) * nx, p = line + x;
+    load_comp4<W>(V.X + 4 * p, q.x);
+    if (ROWS9) {
+      double *buf = turn[w];
+      double v[NP];
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-        if (f == 0) acc[s] = J[s];
-        else if (f & 1) acc[s] = acc[s] - J[s];
-        else acc[s] = acc[s] + J[s];
-      }
+      for (int k = 0; k < NP; ++k) v[k] = __ldg(V.mu + line * NP + off[k]);
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < NP; ++k) buf[lane + 32 * k] = v[k];
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < S; ++s) q.mu[s] = buf[lane * NP + s];
+#pragma unroll
+      for (int s = 0; s < NM; ++s) q.m[s] = buf[lane * NP + S + s];
+    } else {
+#pragma unroll
+      for (int s = 0; s < S; ++s) q.mu[s] = __ldg(V.mu + p * V.mus + s);
+#pragma unroll
+      for (int s = 0; s < NM; ++s) q.m[s] = __ldg(V.M + p * V.ms + s);
+    }
+  };
+  auto face = [&](const DivPoint &lo, const DivPoint &hi, double J8[S]) {
+    double g[S];
+#pragma unroll
+    for (int s = 0; s < S; ++s) g[s] = (hi.mu[s] - lo.mu[s]) * inv_dx;
+    face_flux8(lo.x, lo.m, hi.x, hi.m, g, J8);
+  };
+  const double inv_dx8 = 0.125 * inv_dx;
+  const bool out2 = ((uintptr_t)out & 15) == 0;
+  const int yp = y + 1 == ny ? 0 : y + 1, ym = y == 0 ? ny - 1 : y - 1;
+  DivPoint cur;
+  double Jm[S];
+  load(first, y, cur);
+  if (DIM > 1) {
+    DivPoint below;
+    load(first == 0 ? nm - 1 : first - 1, y, below);
+    face(below, cur, Jm);
+  }
+  for (int i = first; i < last; ++i) {
+    DivPoint up, nb;
+    double jx[S], jl[S], jyp[S], jym[S], jz[S];
+    if (DIM > 1) load(i + 1 == nm ? 0 : i + 1, y, up);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      nb.x[s] = __shfl_down_sync(0xffffffffu, cur.x[s], 1);
+      nb.mu[s] = __shfl_down_sync(0xffffffffu, cur.mu[s], 1);
     }
 #pragma unroll
-    for (int s = 0; s < S; ++s) out[p * S + s] = acc[s] * inv_dx;
+    for (int s = 0; s < NM; ++s) nb.m[s] = __shfl_down_sync(0xffffffffu, cur.m[s], 1);
+    face(cur, nb, jx);
+#pragma unroll
+    for (int s = 0; s < S; ++s) jl[s] = __shfl_up_sync(0xffffffffu, jx[s], 1);
+    if (DIM == 3) {
+      load(i, yp, nb);
+      face(cur, nb, jyp);
+      load(i, ym, nb);
+      face(nb, cur, jym);
+    }
+    if (DIM > 1) face(cur, up, jz);
+    if (lane > 0 && lane <= kDivCols && col < nx) {
+      double *o = out + 4 * (((int64_t)i * ny + y) * nx + x);
+      double v[S];
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        if (DIM == 1) {
+          v[s] = jx[s] - jl[s];
+        } else {
+          v[s] = jz[s] - Jm[s];
+          if (DIM == 3) v[s] = (v[s] + jyp[s]) - jym[s];
+          v[s] = (v[s] + jx[s]) - jl[s];
+        }
+        v[s] = v[s] * inv_dx8;
+      }
+      if (out2) {
+        reinterpret_cast<double2 *>(o)[0] = make_double2(v[0], v[1]);
+        reinterpret_cast<double2 *>(o)[1] = make_double2(v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int s = 0; s < S; ++s) o[s] = v[s];
+      }
+    }
+    if (DIM > 1) {
+#pragma unroll
+      for (int s = 0; s < S; ++s) Jm[s] = jz[s];
+      cur = up;
+    }
   }
+}
+
+template <int DIM>
+static void launch_divergence(int n0, int n1, int n2, const DivView &V, double inv_dx, double *out,
+                              cudaStream_t s) {
+  const int nx = DIM == 1 ? n0 : (DIM == 2 ? n1 : n2), nm = DIM == 1 ? 1 : n0;
+  const int tiles = (nx + kDivCols - 1) / kDivCols;
+  // rows of a march: 16 (one face more per 16 rows), fewer where that leaves
+  // less than 12 warps per SM
+  const int64_t lines = (int64_t)tiles * (DIM == 3 ? (n1 + 3) / 4 * 4 : 1) * nm;
+  const int64_t fill = lines / ((int64_t)sm_count() * 12);
+  const int rows = (int)(fill < 2 ? 2 : (fill > 16 ? 16 : fill));
+  const int64_t chunks = (nm + rows - 1) / rows;
+  const int64_t blocks = DIM == 1   ? (tiles + 3) / 4
+                         : DIM == 2 ? tiles * ((chunks + 3) / 4)
+                                    : tiles * chunks * ((n1 + 3) / 4);
+  const dim3 grid((unsigned)blocks);
+  const bool wide = aligned_to(V.X, 32);
+  const bool rows9 = V.M == V.mu + S && V.mus == NP && V.ms == NP &&
+                     nx < (1 << 27);                   // 32-bit offsets in a row of rows
+  auto kernel = rows9 ? (wide ? k_divergence<DIM, true, 4> : k_divergence<DIM, true, 1>)
+                      : (wide ? k_divergence<DIM, false, 4> : k_divergence<DIM, false, 1>);
+  kernel<<<grid, kDivThreads, 0, s>>>(n0, n1, n2, V, inv_dx, out, rows);
 }
 
 // ---------------------------------------------- save-step gradients/fluxes
@@ -415,8 +576,19 @@ pf5d_status pf5d_laplacian(int32_t dim, const int64_t *shape, int32_t ncomp, con
   PF5D_REQUIRE(c && out && ncomp > 0, PF5D_ERR_ARG, "bad arguments");
   const double inv_dx2 = 1.0 / (dx * dx);
   const int64_t npts = n0 * n1 * n2;
-  k_laplacian<<<grid_for(npts, 256), 256, 0, as_stream(stream)>>>(dim, n0, n1, n2, ncomp, c,
-                                                                   inv_dx2, out);
+  const int64_t ny = dim == 1 ? 1 : shape[dim - 2], nx = shape[dim - 1], nz = dim == 3 ? n0 : 1;
+  if (ncomp == S && (((uintptr_t)c | (uintptr_t)out) & 15) == 0 && nx < (1 << 30) &&
+      ny <= 8 * 65535 && nz <= 65535) {
+    const dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz), block(32, 8);
+    const bool wide = aligned_to(c, 32);
+    auto kernel = dim == 1   ? (wide ? k_laplacian4<1, 4> : k_laplacian4<1, 2>)
+                  : dim == 2 ? (wide ? k_laplacian4<2, 4> : k_laplacian4<2, 2>)
+                             : (wide ? k_laplacian4<3, 4> : k_laplacian4<3, 2>);
+    kernel<<<grid, block, 0, as_stream(stream)>>>((int)n0, (int)n1, (int)n2, c, inv_dx2, out);
+  } else {
+    k_laplacian<<<grid_for(npts, 256), 256, 0, as_stream(stream)>>>(dim, n0, n1, n2, ncomp, c,
+                                                                     inv_dx2, out);
+  }
   PF5D_LAUNCHED();
   return PF5D_OK;
 }
@@ -444,10 +616,12 @@ pf5d_status pf5d_divergence_from_mu(int32_t dim, const int64_t *shape, int32_t n
   PF5D_REQUIRE(ncomp == S, PF5D_ERR_ARG, "ncomp must be %d", S);
   PF5D_REQUIRE(X && M && mu && out && m_stride >= NM && mu_stride >= S, PF5D_ERR_ARG,
                "bad arguments");
-  const int64_t npts = n0 * n1 * n2;
-  k_divergence<<<grid_for(npts, 128), 128, 0, as_stream(stream)>>>(dim, n0, n1, n2, X, M,
-                                                                   m_stride, mu, mu_stride,
-                                                                   inv_dx, out);
+  const DivView V{X, mu, M, mu_stride, m_stride};
+  const int a = (int)n0, b = (int)n1, c = (int)n2;
+  cudaStream_t s = as_stream(stream);
+  if (dim == 1) launch_divergence<1>(a, b, c, V, inv_dx, out, s);
+  else if (dim == 2) launch_divergence<2>(a, b, c, V, inv_dx, out, s);
+  else launch_divergence<3>(a, b, c, V, inv_dx, out, s);
   PF5D_LAUNCHED();
   return PF5D_OK;
 }

@@ -19,7 +19,8 @@ struct FFTPair {
   bool ready = false;
 };
 
-pf5d_status fft_create(int dim, const int64_t *shape, FFTPair *p);
+// plans = false: the sizes only (the transforms run another way).
+pf5d_status fft_create(int dim, const int64_t *shape, FFTPair *p, bool plans = true);
 void fft_destroy(FFTPair *p);
 // s (real, npts) -> k (complex, nk); k -> s.  Both on `stream`.
 pf5d_status fft_forward(FFTPair *p, double *s, cufftDoubleComplex *k, cudaStream_t stream);

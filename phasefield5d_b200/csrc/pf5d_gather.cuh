@@ -33,12 +33,13 @@
 namespace pf5d {
 
 constexpr int kGatherBins = 256;
+constexpr unsigned kFarCell = ~0u;                              // n^4 cells, n < 256
 constexpr int kNoKey = -1;                                      // no point (past the field's edge)
 
 template <int NT_, int PER_, int K_>
 struct GatherOrder {
   static constexpr int NT = NT_, PER = PER_, K = K_, N = NT * PER;
-  int cell[N];                      // -1: outside the linear region
+  unsigned cell[N];                 // kFarCell: outside the linear region
   int base[kGatherBins + 1];        // points (low half) and items (high half) before each bin
   int wsum[NT / 32 + 1];
   int nleft;
@@ -80,7 +81,7 @@ __device__ __forceinline__ int gather_rank(G &g, unsigned active, bool linear, c
   const int key = linear ? (int)((unsigned)(41 * ii[0] + 13 * ii[1] + 5 * ii[2] + ii[3]) %
                                  (kGatherBins - 1u))
                          : kGatherBins - 1;
-  g.cell[q] = linear ? ((ii[0] * n + ii[1]) * n + ii[2]) * n + ii[3] : -1;
+  g.cell[q] = linear ? (((unsigned)ii[0] * n + ii[1]) * n + ii[2]) * n + ii[3] : kFarCell;
   const unsigned same = __match_any_sync(active, key);
   const int lane = threadIdx.x & 31, lead = __ffs(same) - 1;
   int before = 0;
@@ -175,7 +176,7 @@ __device__ __forceinline__ void gather_values(G &g, const Table &T, int nitems, 
     const int s = (int)(e & 0xffffu), m = (int)(e >> 16);
     int q[K];
     double t[K][S], u[K][S];
-    const int cell0 = g.cell[g.order[s]];
+    const unsigned cell0 = g.cell[g.order[s]];
     unsigned mine = 0;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -241,22 +242,30 @@ __device__ __forceinline__ void gather_rest(G &g, const Table &T, int tid, unsig
   });
 }
 
-// The four components of a point; wide: the field is 32-byte aligned, so they
-// are one 256-bit load (half the L1 wavefronts of two 16-byte ones, whose
-// lanes each touch half of every line).  p derives from an after_wait pointer.
-__device__ __forceinline__ void load_comp4(const double *p, bool wide, double v[S]) {
-  if (wide) {
+// The four components of a point by loads of W doubles: 4 for a field on a
+// 32-byte boundary (one 256-bit load moves half the L1 wavefronts of two
+// 16-byte ones, whose lanes each touch half of every line), 2 on 16 bytes.  W is
+// known to the kernel: a choice at run time, in the loops, cost the split rate
+// stage 5%.  p derives from an after_wait pointer where the kernel waits for
+// another.
+template <int W>
+__device__ __forceinline__ void load_comp4(const double *p, double v[S]) {
+  if constexpr (W == 4) {
     asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
         : "=d"(v[0]), "=d"(v[1]), "=d"(v[2]), "=d"(v[3])
         : "l"(p));
-  } else {
+  } else if constexpr (W == 2) {
     const double2 a = __ldg(reinterpret_cast<const double2 *>(p));
     const double2 b = __ldg(reinterpret_cast<const double2 *>(p) + 1);
     v[0] = a.x;
     v[1] = a.y;
     v[2] = b.x;
     v[3] = b.y;
+  } else {
+#pragma unroll
+    for (int c = 0; c < S; ++c) v[c] = __ldg(p + c);
   }
 }
+inline bool aligned_to(const void *p, size_t bytes) { return ((uintptr_t)p & (bytes - 1)) == 0; }
 
 }  // namespace pf5d

@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kChemNT32, MINB) k32_chem(Rate32 P) {
     const int s = (int)(e & 0xffffu), m = (int)(e >> 16);
     int q[K];
     Weights32 W[K];
-    const int cell0 = g.cell[g.order[s]];
+    const unsigned cell0 = g.cell[g.order[s]];
     unsigned mine = 0;
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -1292,19 +1292,7 @@ pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void
     return fail(PF5D_ERR_CUDA);
   }
   if (desc->elastic) {
-    long long n[3];
-    for (int d = 0; d < desc->dim; ++d) n[d] = desc->shape[d];
     h->nk = npts / desc->shape[desc->dim - 1] * (desc->shape[desc->dim - 1] / 2 + 1);
-    size_t ws = 0;
-    if (cufftCreate(&h->fwd) != CUFFT_SUCCESS || cufftCreate(&h->inv) != CUFFT_SUCCESS ||
-        cufftMakePlanMany64(h->fwd, desc->dim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, 1,
-                            &ws) != CUFFT_SUCCESS ||
-        cufftMakePlanMany64(h->inv, desc->dim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, 1,
-                            &ws) != CUFFT_SUCCESS) {
-      set_error("cuFFT plan creation failed");
-      return fail(PF5D_ERR_CUFFT);
-    }
-    h->plans = true;
     if (desc->dim == 1 && npts <= kElastic1dMax32) {
       // 1D B(k) is one value for every k != 0 (checked exactly): closed form
       bool flat = true;
@@ -1312,6 +1300,24 @@ pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void
       h->closed1d = flat;
       h->bn = h->nk > 1 ? desc->bk[1] : 0.0;
       h->b0 = desc->bk[0];
+    }
+    if (desc->dim == 2 && colpass_fits(h->shape[0])) {
+      h->use_colpass = colpass_create(desc->dim, h->shape, &h->colp, true) == PF5D_OK;
+      if (!h->use_colpass) colpass_destroy(&h->colp);
+    }
+    if (!h->closed1d && !h->use_colpass) {
+      long long n[3];
+      for (int d = 0; d < desc->dim; ++d) n[d] = desc->shape[d];
+      size_t ws = 0;
+      if (cufftCreate(&h->fwd) != CUFFT_SUCCESS || cufftCreate(&h->inv) != CUFFT_SUCCESS ||
+          cufftMakePlanMany64(h->fwd, desc->dim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_R2C, 1,
+                              &ws) != CUFFT_SUCCESS ||
+          cufftMakePlanMany64(h->inv, desc->dim, n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_C2R, 1,
+                              &ws) != CUFFT_SUCCESS) {
+        set_error("cuFFT plan creation failed");
+        return fail(PF5D_ERR_CUFFT);
+      }
+      h->plans = true;
     }
     std::vector<float> b(h->nk);
     const double inv_n = 1.0 / (double)npts;
@@ -1322,10 +1328,6 @@ pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void
         cudaMemcpy(h->bk, b.data(), h->nk * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess) {
       set_error("device allocation failed");
       return fail(PF5D_ERR_CUDA);
-    }
-    if (desc->dim == 2 && colpass_fits(h->shape[0])) {
-      h->use_colpass = colpass_create(desc->dim, h->shape, &h->colp, true) == PF5D_OK;
-      if (!h->use_colpass) colpass_destroy(&h->colp);
     }
   }
   Rate32 &P = h->rp;

@@ -374,8 +374,10 @@ struct ChemTile {
   static constexpr int BZ = DIM == 3 ? PER : 1;
 };
 
-template <int DIM, bool VEC, int PER, int K>
+// FAST: double2-aligned nodes and a field on a 32-byte boundary.
+template <int DIM, bool FAST, int PER, int K>
 __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
+  constexpr int W = FAST ? 4 : 2;
   using G = ChemTile<DIM, PER>;
   constexpr int NT = kChemNT;
   __shared__ GatherSmem<NT, PER, K> g;
@@ -385,7 +387,6 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const int bx = blockIdx.x * G::BX, by = blockIdx.y * G::BY, bz = blockIdx.z * G::BZ;
   const int64_t plane = (int64_t)P.ny * P.nx;
-  const bool wide = ((uintptr_t)P.X & 31) == 0;
   // the point in slot q = j * NT + w * 32 + lane
   auto px = [&](int j, int l, int v) { return DIM == 1 ? bx + j * NT + v * 32 + l : bx + l; };
   auto py = [&](int j, int v) { return DIM == 1 ? 0 : (DIM == 2 ? by + PER * v + j : by + v); };
@@ -398,45 +399,45 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
     const int x = px(j, lane, w), y = py(j, w), z = pz(j);
     const bool valid = x < P.nx && y < P.ny && z < P.nz;
     double xc[S] = {0.0, 0.0, 0.0, 0.0};
-    if (valid) load_comp4(X + 4 * (z * plane + (int64_t)y * P.nx + x), wide, xc);
+    if (valid) load_comp4<W>(X + 4 * (z * plane + (int64_t)y * P.nx + x), xc);
     kr[j] = gather_add(g, P.T, valid, xc, j * NT + tid);
   }
   const int nitems = gather_sort(g, kr, tid);
-  gather_values<VEC>(g, P.T, nitems, tid);
+  gather_values<FAST>(g, P.T, nitems, tid);
   unsigned flags = 0;
-  gather_rest<VEC>(g, P.T, tid, &flags, [&](int q, double x[S]) {
+  gather_rest<FAST>(g, P.T, tid, &flags, [&](int q, double x[S]) {
     const int j = q / NT, v = (q / 32) % (NT / 32);
-    load_comp4(X + 4 * (pz(j) * plane + (int64_t)py(j, v) * P.nx + px(j, q & 31, v)), wide, x);
+    load_comp4<W>(X + 4 * (pz(j) * plane + (int64_t)py(j, v) * P.nx + px(j, q & 31, v)), x);
   });
   raise_rate_flags(P.st, flags);
   if (kr[0] == kNoKey) return;                  // none of this thread's points is in the field
   double below[S], xc[S], above[S];             // along the marching axis (y in 2D, z in 3D)
   const int x0 = px(0, lane, w), y0 = py(0, w), z0 = pz(0);
   auto at = [&](int z, int y, int x) { return X + 4 * (z * plane + (int64_t)y * P.nx + x); };
-  if (DIM == 2) load_comp4(at(0, y0 == 0 ? P.ny - 1 : y0 - 1, x0), wide, below);
-  if (DIM == 3) load_comp4(at(z0 == 0 ? P.nz - 1 : z0 - 1, y0, x0), wide, below);
-  load_comp4(at(z0, y0, x0), wide, xc);
+  if (DIM == 2) load_comp4<W>(at(0, y0 == 0 ? P.ny - 1 : y0 - 1, x0), below);
+  if (DIM == 3) load_comp4<W>(at(z0 == 0 ? P.nz - 1 : z0 - 1, y0, x0), below);
+  load_comp4<W>(at(z0, y0, x0), xc);
 #pragma unroll
   for (int j = 0; j < PER; ++j) {
     if (kr[j] == kNoKey) break;
     const int x = px(j, lane, w), y = py(j, w), z = pz(j);
     double lap[S], n0[S], n1[S];
     if (DIM == 1) {
-      if (j > 0) load_comp4(at(0, 0, x), wide, xc);
+      if (j > 0) load_comp4<W>(at(0, 0, x), xc);
     } else {
       const int yp = y + 1 == P.ny ? 0 : y + 1, zp = z + 1 == P.nz ? 0 : z + 1;
-      load_comp4(DIM == 2 ? at(0, yp, x) : at(zp, y, x), wide, above);
+      load_comp4<W>(DIM == 2 ? at(0, yp, x) : at(zp, y, x), above);
 #pragma unroll
       for (int c = 0; c < S; ++c) lap[c] = above[c] + below[c];
     }
     if (DIM == 3) {
-      load_comp4(at(z, y + 1 == P.ny ? 0 : y + 1, x), wide, n0);
-      load_comp4(at(z, y == 0 ? P.ny - 1 : y - 1, x), wide, n1);
+      load_comp4<W>(at(z, y + 1 == P.ny ? 0 : y + 1, x), n0);
+      load_comp4<W>(at(z, y == 0 ? P.ny - 1 : y - 1, x), n1);
 #pragma unroll
       for (int c = 0; c < S; ++c) lap[c] = (lap[c] + n0[c]) + n1[c];
     }
-    load_comp4(at(z, y, x + 1 == P.nx ? 0 : x + 1), wide, n0);
-    load_comp4(at(z, y, x == 0 ? P.nx - 1 : x - 1), wide, n1);
+    load_comp4<W>(at(z, y, x + 1 == P.nx ? 0 : x + 1), n0);
+    load_comp4<W>(at(z, y, x == 0 ? P.nx - 1 : x - 1), n1);
     const int64_t gi = z * plane + (int64_t)y * P.nx + x;
     const double spv = P.sp ? __ldg(P.sp + gi) : 0.0;
     double v[NP];
@@ -885,9 +886,9 @@ struct Pt64 {
   double x[S], mu[S], m[NM];
 };
 
-__device__ __forceinline__ void load_pt64(const RateParams &P, const double *X, int64_t g, bool wide,
-                                          Pt64 &q) {
-  load_comp4(X + 4 * g, wide, q.x);
+template <int W>
+__device__ __forceinline__ void load_pt64(const RateParams &P, const double *X, int64_t g, Pt64 &q) {
+  load_comp4<W>(X + 4 * g, q.x);
   const double2 *mm = reinterpret_cast<const double2 *>(P.mm) + g;
   const double2 a = __ldg(mm), b = __ldg(mm + P.npts), c = __ldg(mm + 2 * P.npts),
                 d = __ldg(mm + 3 * P.npts);
@@ -920,8 +921,9 @@ __device__ __forceinline__ void face_pts64(const Pt64 &lo, const Pt64 &hi, doubl
   face_flux8(lo.x, lo.m, hi.x, hi.m, g, J8);
 }
 
-template <int DIM, int R, int MINB>
+template <int DIM, bool FAST, int R, int MINB>
 __global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int rows) {
+  constexpr int W = FAST ? 4 : 2;
   static_assert(DIM == 3 || R == 1, "rows per thread are of axis 1");
   __shared__ double red[kFluxThreads / 32];
   pdl_wait();
@@ -934,7 +936,6 @@ __global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int r
   const int y = (blockIdx.y * 4 + w) * R;              // 3D
   const int first = (DIM == 3 ? blockIdx.z : y) * rows, last = min(first + rows, n0);
   const bool out_lane = lane > 0 && lane <= kFluxCols && col < P.nx;
-  const bool wide = ((uintptr_t)P.X & 31) == 0;
   double vmax = 0.0;
   if (first < n0 && (DIM == 2 || y < P.ny)) {          // whole warps
     auto at = [&](int i, int yy) {
@@ -948,8 +949,8 @@ __global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int r
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       Pt64 below;
-      load_pt64(P, X, at(first == 0 ? n0 - 1 : first - 1, row(r)), wide, below);
-      load_pt64(P, X, at(first, row(r)), wide, cur[r]);
+      load_pt64<W>(P, X, at(first == 0 ? n0 - 1 : first - 1, row(r)), below);
+      load_pt64<W>(P, X, at(first, row(r)), cur[r]);
       face_pts64(below, cur[r], P.inv_dx, Jm[r]);
     }
     for (int i = first; i < last; ++i) {
@@ -961,13 +962,13 @@ __global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int r
       double jym[S];
       if (DIM == 3) {
         Pt64 nb;
-        load_pt64(P, X, at(i, ym), wide, nb);
+        load_pt64<W>(P, X, at(i, ym), nb);
         face_pts64(nb, cur[0], P.inv_dx, jym);
       }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
         Pt64 up, nb;
-        load_pt64(P, X, at(ip, row(r)), wide, up);
+        load_pt64<W>(P, X, at(ip, row(r)), up);
         double jx[S], jl[S], jyp[S], jz[S], out[S];
 #pragma unroll
         for (int c = 0; c < S; ++c) {
@@ -982,7 +983,7 @@ __global__ void __launch_bounds__(kFluxThreads, MINB) k_flux(RateParams P, int r
         if (DIM == 3) {
           // the last row's upper neighbour (for a row that repeats: unused)
           if (r == R - 1 || y + r + 1 >= P.ny) {
-            load_pt64(P, X, at(i, yp), wide, nb);
+            load_pt64<W>(P, X, at(i, yp), nb);
             face_pts64(cur[r], nb, P.inv_dx, jyp);
           } else {
             face_pts64(cur[r], cur[r + 1 < R ? r + 1 : r], P.inv_dx, jyp);
@@ -1609,7 +1610,8 @@ struct pf5d_stepper {
   dim3 rate_grid, rate_block;
   size_t rate_smem = 0;
   int zc = 1;
-  bool vec = false;
+  bool vec = false;              // double2-aligned table nodes
+  bool fast = false;             // ... and X on a 32-byte boundary (split variants)
   int variant = 0;
   Stepper32 *s32 = nullptr;      // FP32C form (all calls delegate)
   double *mass_ws = nullptr;     // FP64 mean reduction workspace
@@ -1690,14 +1692,20 @@ RateVariant make_variant() {
   return v;
 }
 
-// The split form's mu/M kernel.
+// The split form's kernels (fast: see k_chem).
 template <int DIM, int PER, int K>
-void launch_chem(bool vec, cudaStream_t s, const RateParams &P) {
+void launch_chem(bool fast, cudaStream_t s, const RateParams &P) {
   using G = ChemTile<DIM, PER>;
   const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
                (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-  if (vec) launch_pdl(k_chem<DIM, true, PER, K>, g, dim3(kChemNT), 0, s, P);
+  if (fast) launch_pdl(k_chem<DIM, true, PER, K>, g, dim3(kChemNT), 0, s, P);
   else launch_pdl(k_chem<DIM, false, PER, K>, g, dim3(kChemNT), 0, s, P);
+}
+
+template <int DIM, int R, int MINB>
+void launch_flux(bool fast, dim3 g, cudaStream_t s, const RateParams &P, int rows) {
+  if (fast) launch_pdl(k_flux<DIM, true, R, MINB>, g, dim3(kFluxThreads), 0, s, P, rows);
+  else launch_pdl(k_flux<DIM, false, R, MINB>, g, dim3(kFluxThreads), 0, s, P, rows);
 }
 
 // Split variant: k_chem, then k_flux; in 2D a warp marches over ROWS rows (in
@@ -1714,16 +1722,17 @@ RateVariant make_split_variant() {
   v.split = true;
   v.smem2d = v.smem3d = 0;
   v.set_attrs = [](bool) {};
-  v.launch2d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P) {
-    launch_chem<2, PER, K>(vec, s, P);
-    launch_pdl(k_flux<2, 1, MINB>, g, dim3(kFluxThreads), 0, s, P, ROWS);
+  v.launch2d = [](bool fast, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P) {
+    launch_chem<2, PER, K>(fast, s, P);
+    launch_flux<2, 1, MINB>(fast, g, s, P, ROWS);
   };
-  v.launch3d = [](bool vec, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P, int zc) {
-    launch_chem<3, PER, K>(vec, s, P);
-    launch_pdl(k_flux<3, R, MINB>, g, dim3(kFluxThreads), 0, s, P, zc);
+  v.launch3d = [](bool fast, dim3 g, dim3, size_t, cudaStream_t s, const RateParams &P, int zc) {
+    launch_chem<3, PER, K>(fast, s, P);
+    launch_flux<3, R, MINB>(fast, g, s, P, zc);
   };
-  v.kernels = [](bool vec, int dim) {
-    return kname("k_chem", {dim, vec, PER, K}) + " + " + kname("k_flux", {dim, dim == 2 ? 1 : R, MINB});
+  v.kernels = [](bool fast, int dim) {
+    return kname("k_chem", {dim, fast, PER, K}) + " + " +
+           kname("k_flux", {dim, fast, dim == 2 ? 1 : R, MINB});
   };
   return v;
 }
@@ -1780,7 +1789,8 @@ int64_t max_rate_blocks(const pf5d_stepper *h) {
 pf5d_status configure_rate(pf5d_stepper *h, int variant) {
   const int dim = h->d.dim;
   const RateParams &P = h->rp;
-  h->vec = (P.T.stride % 2 == 0) && (((uintptr_t)P.T.grid & 15) == 0);
+  h->vec = (P.T.stride % 2 == 0) && aligned_to(P.T.grid, 16);
+  h->fast = h->vec && aligned_to(P.X, 32);
   if (dim == 1) {
     h->rate_block = dim3(kTX1);
     h->rate_grid = rate_grid_of(h, 0, &h->zc);
@@ -1801,6 +1811,11 @@ pf5d_status configure_rate(pf5d_stepper *h, int variant) {
   return PF5D_OK;
 }
 
+// What the variant's kernels want to know of the solve's alignment.
+bool variant_flag(const pf5d_stepper *h) {
+  return rate_variants()[h->variant].split ? h->fast : h->vec;
+}
+
 pf5d_status launch_rate(pf5d_stepper *h, cudaStream_t s) {
   const dim3 g = h->rate_grid, b = h->rate_block;
   const size_t sm = h->rate_smem;
@@ -1810,10 +1825,10 @@ pf5d_status launch_rate(pf5d_stepper *h, cudaStream_t s) {
       else launch_pdl(k_rate_1d<kTX1, false>, g, b, 0, s, h->rp);
       break;
     case 2:
-      rate_variants()[h->variant].launch2d(h->vec, g, b, sm, s, h->rp);
+      rate_variants()[h->variant].launch2d(variant_flag(h), g, b, sm, s, h->rp);
       break;
     default:
-      rate_variants()[h->variant].launch3d(h->vec, g, b, sm, s, h->rp, h->zc);
+      rate_variants()[h->variant].launch3d(variant_flag(h), g, b, sm, s, h->rp, h->zc);
   }
   PF5D_LAUNCHED();
   PF5D_CUDA(launch_pdl(k_dt_finish, dim3(1), dim3(kDtThreads), 0, s, h->rp,
@@ -2052,12 +2067,13 @@ pf5d_status pf5d_stepper_create(const pf5d_stepper_desc *desc, double *X, void *
     h->b0 = desc->bk[0];
   }
   if (desc->elastic) {
-    if ((st = fft_create(desc->dim, h->shape, &h->fft)) != PF5D_OK) return fail(st);
-    if ((st = upload_bk_scaled(desc->bk, h->fft.nk, npts, &h->bk)) != PF5D_OK) return fail(st);
     if (desc->dim >= 2 && colpass_fits(h->shape[0])) {
       h->use_colpass = colpass_create(desc->dim, h->shape, &h->colp, false) == PF5D_OK;
       if (!h->use_colpass) colpass_destroy(&h->colp);
     }
+    if ((st = fft_create(desc->dim, h->shape, &h->fft, !h->closed1d && !h->use_colpass)) != PF5D_OK)
+      return fail(st);
+    if ((st = upload_bk_scaled(desc->bk, h->fft.nk, npts, &h->bk)) != PF5D_OK) return fail(st);
     if (cudaMalloc(&h->s, npts * sizeof(double)) != cudaSuccess ||
         cudaMalloc(&h->k, h->fft.nk * sizeof(cufftDoubleComplex)) != cudaSuccess) {
       set_error("device allocation failed");
@@ -2294,9 +2310,9 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
     if ((st = launch_rate(h, s)) != PF5D_OK) return st;
     // mu and M of this step at every point, then the "before" reductions
     switch (dim) {
-      case 1: launch_chem<1, 4, 3>(h->vec, s, h->rp); break;
-      case 2: launch_chem<2, 4, 3>(h->vec, s, h->rp); break;
-      default: launch_chem<3, 4, 3>(h->vec, s, h->rp);
+      case 1: launch_chem<1, 4, 3>(h->fast, s, h->rp); break;
+      case 2: launch_chem<2, 4, 3>(h->fast, s, h->rp); break;
+      default: launch_chem<3, 4, 3>(h->fast, s, h->rp);
     }
     PF5D_LAUNCHED();
     Xpre = h->X;
@@ -2373,7 +2389,7 @@ const char *pf5d_stepper_rate_kernels(pf5d_stepper *h) {
   if (!h) return "";
   if (h->s32) return s32_rate_kernels(h->s32);
   if (h->d.dim == 1) h->kernels = kname("k_rate_1d", {kTX1, h->vec});
-  else h->kernels = rate_variants()[h->variant].kernels(h->vec, h->d.dim);
+  else h->kernels = rate_variants()[h->variant].kernels(variant_flag(h), h->d.dim);
   h->kernels += " + k_dt_finish";
   return h->kernels.c_str();
 }
