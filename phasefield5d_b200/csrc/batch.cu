@@ -7,9 +7,10 @@
 //     (batched plans; B(k) depends only on the direction of k, so a shape
 //     group shares one B(k)/N) and its B(k) multiply, the groups' chains on
 //     parallel graph branches;
-//   * one persistent rate launch: blocks loop over the lane's tiles
-//     (32x8-style plane tiles for 2D, runs of TX*TY points for 1D) and
-//     store each tile's max|dX/dt| in its own slot;
+//   * the rate launch: one persistent kernel whose blocks loop over the lane's
+//     tiles (32x8-style plane tiles for 2D, runs of TX*TY points for 1D), or,
+//     split, mu/M and then faces and divergence with a block per tile; each
+//     tile's max|dX/dt| goes into its own slot;
 //   * kb_dt: one warp per solve reduces its slots and runs its FP64 dt
 //     controller;
 //   * one persistent compensated-update launch over fixed 1024-point chunks.
@@ -28,6 +29,7 @@
 
 #include "pf5d_fp32c.cuh"
 #include "pf5d_host.h"
+#include "pf5d_split32.cuh"
 
 namespace pf5d {
 
@@ -39,6 +41,7 @@ struct BSolve {
   int dim;             // 1 or 2
   int ntx, nty;        // tile grid
   int tile0, ntiles;   // global tile range
+  int ctile0, nctx;    // split variants: first mu/M tile (2D solves only) and tiles per row
   int chunk0, nchunks; // global update-chunk range
   int emode;           // 0: elasticity off, 1: 1D constant-B form, 2: 2D cuFFT
   int oob_interval;
@@ -67,6 +70,18 @@ __device__ __forceinline__ int find_solve_chunk(const BSolve *solves, int n, int
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
     if (solves[mid].chunk0 <= c) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The same over the mu/M tiles (a solve without any shares its number with the
+// next one that has some).
+__device__ __forceinline__ int find_solve_ctile(const BSolve *solves, int n, int t) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (solves[mid].ctile0 <= t) lo = mid;
     else hi = mid - 1;
   }
   return lo;
@@ -177,6 +192,65 @@ __global__ void __launch_bounds__(TX * TY, MINB)
     __syncthreads();
     finish_slot32(vmax, red, tile_max + t);
   }
+}
+
+// The block's copy of a solve's rate parameters (a barrier follows).
+__device__ __forceinline__ void copy_rate32(Rate32 *dst, const Rate32 &src, int tid, int nt) {
+  const int *from = reinterpret_cast<const int *>(&src);
+  int *to = reinterpret_cast<int *>(dst);
+  for (int i = tid; i < (int)(sizeof(Rate32) / sizeof(int)); i += nt) to[i] = from[i];
+  __syncthreads();
+}
+
+// Split rate evaluation of a lane (pf5d_split32.cuh): mu/M of its 2D solves in
+// tiles of 32 columns by 4 * PER rows, then everybody's faces and divergence;
+// 1D solves, a few per cent of the points, go through their tile body in the
+// second kernel.  One block per tile: as blocks retire, the other lane's FFT
+// kernels (high priority) get their slots; with persistent blocks on the lane's
+// share of the slots, as kb_rate's, the rest stood idle while the other lane
+// was in its FFTs (251 us per step against 235).  kb_flux is bound by the
+// latency of its loads: 32 warps per SM instead of 16, 235 -> 212.
+// 64 uneven solves (2.4M points), us per step: 266 with the best fused kernel ->
+// 217, later in a run 260 -> 207; 8 solves of 128x128 keep the fused ones (31.5
+// against 34.8: two launches more latency), the tuner chooses.
+template <int PER, int K, int MINB>
+__global__ void __launch_bounds__(kChemNT32, MINB)
+    kb_chem(const BSolve *__restrict__ solves, int nsolves, int tile_begin) {
+  using G = ChemTile32<2, PER>;
+  __shared__ Rate32 Rs;
+  __shared__ GatherSmem32<kChemNT32, PER, K> g;
+  pdl_wait();
+  const int t = tile_begin + blockIdx.x;
+  const BSolve &B = solves[find_solve_ctile(solves, nsolves, t)];
+  copy_rate32(&Rs, B.R, threadIdx.x, kChemNT32);
+  if (Rs.st->halt) return;
+  const int local = t - B.ctile0;
+  chem32_body<2, PER, K>(Rs, g, local % B.nctx * G::BX, local / B.nctx * G::BY, 0);
+}
+
+template <int ROWS, int MINB>
+__global__ void __launch_bounds__(kFluxThreads32, MINB)
+    kb_flux(const BSolve *__restrict__ solves, int nsolves, int tile_begin, double *tile_max) {
+  constexpr int NT = kFluxThreads32;
+  __shared__ Rate32 Rs;
+  __shared__ __align__(16) unsigned char work[BatchSmem<32, 4>::s1d];
+  __shared__ double red[NT / 32];
+  const int tid = threadIdx.x;
+  pdl_wait();
+  const int t = tile_begin + blockIdx.x;
+  const BSolve &B = solves[find_solve_tile(solves, nsolves, t)];
+  copy_rate32(&Rs, B.R, tid, NT);
+  if (Rs.st->halt) return;
+  const int local = t - B.tile0;
+  float vmax;
+  if (B.dim == 2) {
+    vmax = flux32_body<2, 1>(Rs, local % B.ntx, local / B.ntx, 0, ROWS);
+  } else {
+    unsigned flags = 0;
+    vmax = tile1d32_body<NT>(B, Rs, local, reinterpret_cast<float *>(work), &flags, tid);
+    raise_rate_flags(Rs.st, flags);
+  }
+  finish_slot32(vmax, red, tile_max + t);
 }
 
 __global__ void __launch_bounds__(kUpdThreads)
@@ -374,14 +448,25 @@ __global__ void kb_dt(const BSolve *__restrict__ solves, int nsolves, const doub
   dt_from_slots32(B.R, tile_max + B.tile0, B.ntiles);
 }
 
+// A rate evaluation over tiles [tile_begin, tile_end) of `n` solves by at most
+// `grid` blocks (fused), and for the split variants over their mu/M tiles.
+struct BatchRate {
+  const BSolve *solves;
+  int n, tile_begin, tile_end, grid;
+  int ctile_begin, nctiles;
+  double *tile_max;
+};
+
 struct BatchVariant {
-  int tx, ty, minb;
+  int tx, ty, minb;                 // tile of a 2D solve
+  int nt;                           // points of a 1D solve's tile
   bool win;
+  bool split = false;
+  int cx = 0, cy = 0;               // mu/M tile (split)
   size_t smem;
   void (*set_attrs)();
-  void (*launch)(int grid, cudaStream_t s, const BSolve *solves, int n, int tile_begin,
-                 int tile_end, double *tile_max);
-  int (*occupancy)();
+  void (*launch)(cudaStream_t s, const BatchRate &r);
+  int (*occupancy)() = nullptr;     // resident blocks per SM (fused)
 };
 
 template <int TX, int TY, int MINB, bool WIN, int SORT = 0, bool PP = false>
@@ -391,22 +476,46 @@ BatchVariant make_bvariant() {
   v.tx = TX;
   v.ty = TY;
   v.minb = MINB;
+  v.nt = TX * TY;
   v.win = WIN;
   v.smem = SM::rate;
   v.set_attrs = []() {
     cudaFuncSetAttribute(kb_rate<TX, TY, MINB, WIN, SORT, PP>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM::rate);
   };
-  v.launch = [](int grid, cudaStream_t s, const BSolve *solves, int n, int tile_begin,
-                int tile_end, double *tile_max) {
-    launch_pdl(kb_rate<TX, TY, MINB, WIN, SORT, PP>, dim3(grid), dim3(TX, TY), SM::rate, s, solves, n,
-               tile_begin, tile_end, tile_max);
+  v.launch = [](cudaStream_t s, const BatchRate &r) {
+    launch_pdl(kb_rate<TX, TY, MINB, WIN, SORT, PP>, dim3(r.grid), dim3(TX, TY), SM::rate, s, r.solves,
+               r.n, r.tile_begin, r.tile_end, r.tile_max);
   };
   v.occupancy = []() {
     int nb = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kb_rate<TX, TY, MINB, WIN, SORT, PP>, TX * TY,
                                                   SM::rate);
     return nb;
+  };
+  return v;
+}
+
+template <int ROWS, int FMINB, int PER, int K, int CMINB>
+BatchVariant make_split_bvariant() {
+  using G = ChemTile32<2, PER>;
+  BatchVariant v;
+  v.tx = kFluxCols32;
+  v.ty = 4 * ROWS;
+  v.minb = FMINB;
+  v.nt = kFluxThreads32;
+  v.win = false;
+  v.split = true;
+  v.cx = G::BX;
+  v.cy = G::BY;
+  v.smem = 0;
+  v.set_attrs = []() {};
+  v.launch = [](cudaStream_t s, const BatchRate &r) {
+    if (r.nctiles > 0)
+      launch_pdl(kb_chem<PER, K, CMINB>, dim3(r.nctiles), dim3(kChemNT32), 0, s, r.solves, r.n,
+                 r.ctile_begin);
+    launch_pdl(kb_flux<ROWS, FMINB>, dim3(r.tile_end - r.tile_begin), dim3(kFluxThreads32), 0, s,
+               r.solves, r.n, r.tile_begin, r.tile_max);
   };
   return v;
 }
@@ -420,7 +529,9 @@ const std::vector<BatchVariant> &batch_variants() {
       make_bvariant<32, 16, 2, false, true>(), make_bvariant<32, 8, 3, false, false, true>(),
       make_bvariant<32, 16, 2, false, false, true>(), make_bvariant<32, 8, 3, false, true, true>(),
       make_bvariant<32, 16, 2, false, 2, true>(), make_bvariant<32, 8, 3, false, 2, true>(),
-      make_bvariant<32, 16, 2, false, 2, false>()};
+      make_bvariant<32, 16, 2, false, 2, false>(),
+      make_split_bvariant<8, 8, 4, 2, 6>(), make_split_bvariant<8, 8, 2, 2, 8>(),
+      make_split_bvariant<4, 8, 2, 2, 8>()};
   return v;
 }
 
@@ -437,6 +548,7 @@ constexpr int kLanes = 2;
 struct Lane {
   int s0 = 0, ns = 0;             // positions [s0, s0 + ns) of the lane order
   int tile0 = 0, ntiles = 0;      // the lane's tiles (current variant)
+  int ctile0 = 0, nctiles = 0;    // the lane's mu/M tiles (split variants)
   int chunk0 = 0, nchunks = 0;    // the lane's update chunks
   std::vector<int> order;         // the lane's shape groups, largest first
   int aux0 = 0, naux = 0;         // its FFT branch streams aux[aux0, aux0 + naux)
@@ -466,7 +578,9 @@ struct pf5d_batch {
   std::vector<ShapeGroup> groups;
   int total_tiles = 0, total_chunks = 0;
   int variant = 0, upd_grid = 1;
-  int lane_grid = 1;                // persistent rate blocks of one lane
+  int lane_grid = 1;                // most rate blocks of one lane
+  int total_ctiles = 0;
+  float *mm = nullptr;              // split variants: mu, M, (M_Fe, X_Fe) per point
   cudaStream_t cap = nullptr;
   double *tile_max = nullptr;       // per-tile max |dX/dt| of the last rate launch
   // Shape groups' FFT chains run as parallel branches of the step graph:
@@ -491,11 +605,10 @@ namespace {
 // Tiles of all solves under `variant` (configure_batch's tiling).
 int batch_tiles_of(const pf5d_batch *h, int variant) {
   const BatchVariant &v = batch_variants()[variant];
-  const int nt = v.tx * v.ty;
   int tiles = 0;
   for (const auto &b : h->solves)
     tiles += b.dim == 2 ? ((b.R.nx + v.tx - 1) / v.tx) * ((b.R.ny + v.ty - 1) / v.ty)
-                        : (b.R.nx + nt - 1) / nt;
+                        : (b.R.nx + v.nt - 1) / v.nt;
   return tiles;
 }
 
@@ -503,39 +616,49 @@ pf5d_status configure_batch(pf5d_batch *h, int variant) {
   const auto &vars = batch_variants();
   PF5D_REQUIRE(variant >= 0 && variant < (int)vars.size(), PF5D_ERR_ARG, "bad variant %d", variant);
   const BatchVariant &v = vars[variant];
+  const bool any2d = std::any_of(h->solves.begin(), h->solves.end(),
+                                 [](const BSolve &b) { return b.dim == 2; });
+  PF5D_REQUIRE(!v.split || h->mm || !any2d, PF5D_ERR_CUDA, "no memory for variant %d's mu/M buffer",
+               variant);
   v.set_attrs();
   PF5D_LAUNCHED();
   // Tile grid of every solve for this variant, numbered in lane order.
-  const int nt = v.tx * v.ty;
-  int tiles = 0;
+  int tiles = 0, ctiles = 0;
   for (auto &ln : h->lanes) {
     ln.tile0 = tiles;
+    ln.ctile0 = ctiles;
     for (int k = ln.s0; k < ln.s0 + ln.ns; ++k) {
       BSolve &b = h->solves[h->lane_order[k]];
       if (b.dim == 2) {
         b.ntx = (b.R.nx + v.tx - 1) / v.tx;
         b.nty = (b.R.ny + v.ty - 1) / v.ty;
       } else {
-        b.ntx = (b.R.nx + nt - 1) / nt;
+        b.ntx = (b.R.nx + v.nt - 1) / v.nt;
         b.nty = 1;
       }
+      b.ctile0 = ctiles;
+      b.nctx = v.split ? (b.R.nx + v.cx - 1) / v.cx : 0;
+      if (v.split && b.dim == 2) ctiles += b.nctx * ((b.R.ny + v.cy - 1) / v.cy);
       b.tile0 = tiles;
       b.ntiles = b.ntx * b.nty;
       tiles += b.ntiles;
     }
     ln.ntiles = tiles - ln.tile0;
+    ln.nctiles = ctiles - ln.ctile0;
   }
   h->total_tiles = tiles;
+  h->total_ctiles = ctiles;
   std::vector<BSolve> lane(h->lane_order.size());
   for (size_t k = 0; k < lane.size(); ++k) lane[k] = h->solves[h->lane_order[k]];
   PF5D_CUDA(cudaMemcpy(h->d_solves, h->solves.data(), h->solves.size() * sizeof(BSolve),
                        cudaMemcpyHostToDevice));
   PF5D_CUDA(cudaMemcpy(h->d_lane, lane.data(), lane.size() * sizeof(BSolve),
                        cudaMemcpyHostToDevice));
-  // each lane's rate kernel holds at most its share of the resident block
-  // slots, so the other lane's FFT kernels find free slots
-  const int per_sm = std::max(1, v.occupancy());
-  h->lane_grid = std::max(1, sm_count() * per_sm / (int)std::max<size_t>(h->lanes.size(), 1));
+  // fused: each lane's rate kernel holds at most its share of the resident
+  // block slots, so the other lane's FFT kernels find free slots (split: kb_chem)
+  if (!v.split)
+    h->lane_grid = std::max(1, sm_count() * std::max(1, v.occupancy()) /
+                                   (int)std::max<size_t>(h->lanes.size(), 1));
   h->variant = variant;
   return PF5D_OK;
 }
@@ -572,8 +695,10 @@ pf5d_status enqueue_lane_step(pf5d_batch *h, int L, cudaStream_t s, cudaEvent_t 
   }
   if (offset) PF5D_CUDA(cudaEventRecord(offset, s));
   const BSolve *ls = h->d_lane + ln.s0;
-  batch_variants()[h->variant].launch(std::max(1, std::min(ln.ntiles, h->lane_grid)), s, ls, ln.ns,
-                                      ln.tile0, ln.tile0 + ln.ntiles, h->tile_max);
+  const BatchRate rate{ls, ln.ns, ln.tile0, ln.tile0 + ln.ntiles,
+                       std::max(1, std::min(ln.ntiles, h->lane_grid)), ln.ctile0, ln.nctiles,
+                       h->tile_max};
+  batch_variants()[h->variant].launch(s, rate);
   PF5D_LAUNCHED();
   PF5D_CUDA(launch_pdl(kb_dt, dim3((unsigned)((ln.ns + 7) / 8)), dim3(256), 0, s, ls, ln.ns,
                        (const double *)h->tile_max));
@@ -907,6 +1032,24 @@ pf5d_status pf5d_batch_create(const pf5d_batch_solve *solves, int32_t nsolves,
     set_error("device allocation failed");
     return fail(PF5D_ERR_CUDA);
   }
+  // The split variants' buffer, after all that the fused ones need: without it
+  // (no memory, no 2D solve) the batch runs those.
+  const bool any2d = std::any_of(h->solves.begin(), h->solves.end(),
+                                 [](const BSolve &b) { return b.dim == 2; });
+  if (any2d) {
+    if (cudaMalloc(&h->mm, npts_total * (2 * sizeof(float4) + sizeof(float2))) == cudaSuccess) {
+      float4 *mu = reinterpret_cast<float4 *>(h->mm);
+      for (int i = 0; i < nsolves; ++i) {
+        Rate32 &P = h->solves[i].R;
+        P.mm_mu = mu + h->pt_off[i];
+        P.mm_m = mu + npts_total + h->pt_off[i];
+        P.mm_f = reinterpret_cast<float2 *>(mu + 2 * npts_total) + h->pt_off[i];
+      }
+    } else {
+      h->mm = nullptr;
+      cudaGetLastError();
+    }
+  }
   pf5d_status st = configure_batch(h, 0);
   if (st != PF5D_OK) return fail(st);
   for (int i = 0; i < nsolves; ++i) {
@@ -1004,12 +1147,13 @@ pf5d_status pf5d_batch_autotune(pf5d_batch *h, int32_t *variant, float *best_ms,
   float best_t = 1e30f;
   for (int v = 0; v < (int)batch_variants().size(); ++v) {
     if (configure_batch(h, v) != PF5D_OK) continue;
-    const int grid = std::max(h->total_tiles, 1);
-    batch_variants()[v].launch(grid, s, h->d_lane, (int)n, 0, h->total_tiles, h->tile_max);
+    const BatchRate rate{h->d_lane, (int)n, 0, h->total_tiles, std::max(h->total_tiles, 1), 0,
+                         h->total_ctiles, h->tile_max};
+    batch_variants()[v].launch(s, rate);
     if (cudaGetLastError() != cudaSuccess) continue;
     PF5D_CUDA(cudaEventRecord(e0, s));
     for (int r = 0; r < 3; ++r)
-      batch_variants()[v].launch(grid, s, h->d_lane, (int)n, 0, h->total_tiles, h->tile_max);
+      batch_variants()[v].launch(s, rate);
     PF5D_CUDA(cudaEventRecord(e1, s));
     PF5D_CUDA(cudaEventSynchronize(e1));
     float ms = 0.f;
@@ -1049,6 +1193,7 @@ pf5d_status pf5d_batch_destroy(pf5d_batch *h) {
   cudaFree(h->d_solves);
   cudaFree(h->d_lane);
   cudaFree(h->tile_max);
+  cudaFree(h->mm);
   if (h->cap) cudaStreamDestroy(h->cap);
   for (auto as : h->aux) cudaStreamDestroy(as);
   for (auto ev : h->join) cudaEventDestroy(ev);
