@@ -144,7 +144,19 @@ cudaError_t launch_cluster(void (*kernel)(KArgs...), const Loop1dShape &L, size_
 // Whether this device can hold the cluster (once per solve, at its creation).
 template <typename... KArgs>
 bool cluster_fits(void (*kernel)(KArgs...), const Loop1dShape &L, size_t smem) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the kernel, not to the solve: the device's, so that a
+  // smaller solve created later leaves a larger one's launches valid
+  int dev = 0, most = 0;
+  cudaFuncAttributes fa;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+      cudaFuncGetAttributes(&fa, kernel) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  most -= (int)fa.sharedSizeBytes;
+  if ((int64_t)smem > most) return false;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(L.blocks);
