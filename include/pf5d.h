@@ -292,9 +292,9 @@ pf5d_status pf5d_stepper_reset(pf5d_stepper *h, double dt, double time, void *st
 pf5d_status pf5d_stepper_destroy(pf5d_stepper *h);
 
 /* ------------------------------------------------------- batched form -----
- * Many independent FP32-compensated 1D/2D solves advanced together: one
- * persistent rate launch over the tiles of all solves, one compensated-update
- * launch, cuFFT plans batched per 2D shape; each solve keeps its own
+ * Many independent FP32-compensated 1D/2D solves advanced together: one rate
+ * evaluation over the tiles of all solves, one compensated-update launch, cuFFT
+ * plans batched per 2D shape; each solve keeps its own
  * adaptive dt.  This replaces the reference's one-process-per-solve sweeps
  * (run/launch.py:119-150) with one device-resident batch. */
 typedef struct {
