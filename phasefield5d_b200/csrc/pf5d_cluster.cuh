@@ -1,23 +1,17 @@
 // pf5d_cluster.cuh -- what the 1D step loops share (one thread-block cluster
-// advances a whole solve, many steps per launch): the split of the points over
-// the cluster's blocks, the sum behind the closed-form elastic term, and the
-// launch.
+// advances a whole solve, many steps per launch): the sum behind the closed-form
+// elastic term, the messages between the blocks, and the launch.  The split of
+// the points over the blocks is in pf5d_loop1d.h.
 #pragma once
 
-#include <algorithm>
 #include <cstdint>
 
 #include <cooperative_groups.h>
 
 #include "pf5d_host.h"
+#include "pf5d_loop1d.h"
 
 namespace pf5d {
-
-constexpr int64_t kLoop1dMax = 16384;        // points of a 1D solve that a cluster advances
-constexpr int kLoop1dThreads = 512;          // most threads of a block (128 registers each)
-constexpr int kLoop1dBlocks = 16;            // most blocks of a cluster
-constexpr int kLoop1dSteps = 2000;           // most steps of a launch
-constexpr int kLoop1dGroups = (int)(kLoop1dMax / 32);
 
 // Sum of n values in groups of 32 consecutive ones: a fixed tree within each
 // group (group_sum); then each lane adds every 32nd group's sum in order and a
@@ -100,26 +94,6 @@ __device__ __forceinline__ double warp_max_nonneg(double v) {
   const unsigned mh = __reduce_max_sync(0xffffffffu, hi);
   const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? lo : 0u);
   return __hiloint2double((int)mh, (int)ml);
-}
-
-// Blocks of the cluster, points per block (a multiple of 32) and threads per
-// block for n points.  A block evaluates mu/M at its points and one halo
-// position on each side: all warps but the last (which sums the misfit
-// meanwhile) cover chunk + 2 positions in as few passes as kLoop1dThreads
-// allows.
-struct Loop1dShape {
-  int blocks, chunk, threads;
-};
-inline Loop1dShape loop1d_shape(int64_t n, int max_blocks) {
-  Loop1dShape L;
-  const int groups = (int)((n + 31) / 32);
-  L.blocks = 1;
-  while (L.blocks < max_blocks && L.blocks < groups) L.blocks *= 2;
-  L.chunk = 32 * ((groups + L.blocks - 1) / L.blocks);
-  const int most = kLoop1dThreads - 32;
-  const int passes = (L.chunk + 2 + most - 1) / most;
-  L.threads = 32 + 32 * (((L.chunk + 2 + passes - 1) / passes + 31) / 32);
-  return L;
 }
 
 // One cluster of L.blocks blocks.

@@ -484,10 +484,10 @@ __global__ void __launch_bounds__(MAXT, 1)
   const int nw = (int)blockDim.x >> 5, nt = (int)blockDim.x - 32;   // the last warp sums
   const bool worker = t < nt;
   const int rank = (int)cluster.block_rank(), nb = (int)cluster.num_blocks();
-  const int i0 = rank * chunk, m = max(0, min(chunk, n - i0));
+  const int i0 = rank * chunk, m = min(chunk, n - i0);     // m > 0 (loop1d_shape)
   const int ng = (n + 31) / 32;
   const unsigned bar_a = shared_addr(&sm.bar_a), bar_b = shared_addr(&sm.bar_b);
-  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + (m > 0 ? sizeof(sm.halo) : 0u);
+  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + sizeof(sm.halo);
   double dt = st->dt, time = st->time, xdotmax = st->xdotmax;
   long long step = st->step;
   int to_check = U.oob_interval > 0 ? U.oob_interval - (int)(step % U.oob_interval) : -1;
@@ -506,8 +506,8 @@ __global__ void __launch_bounds__(MAXT, 1)
   unsigned hdst = 0, hbar = 0;
   {
     const int b = t >> 2, h = t & 3;
-    const int bm = b < nb ? max(0, min(chunk, n - b * chunk)) : 0;
-    if (bm > 0 && m > 0) {
+    if (b < nb) {
+      const int bm = min(chunk, n - b * chunk);
       const int src = wrap_any(b * chunk + (h < 2 ? h - 2 : bm + h - 2), n) - i0;
       if (src >= 0 && src < m) {
         hsrc = src + 2;
@@ -581,7 +581,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   for (int k = 0; k <= nsteps; ++k) {
     // B of the step before (k = 0: the state at the launch)
     stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
-    if (t < 4 && m > 0) {                // halo entries into the chunk's rows
+    if (t < 4) {                         // halo entries into the chunk's rows
       const int p = t < 2 ? t : m + t;
       *reinterpret_cast<ulonglong2 *>(Hs + p) = sm.halo[t][0];
       if (t == 1 || t == 2) Qs[p - 1] = __uint_as_float((unsigned)sm.halo[t][1].x);
@@ -595,29 +595,28 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     if (__syncthreads_or(stalled)) stalled = true;
     if (halt || stalled || k == nsteps) break;
-    if (m > 0 && k % kLoop1dResort32 == 0) sort_cells();
+    if (k % kLoop1dResort32 == 0) sort_cells();
     unsigned nn = 0;
     if (worker) {
-      if (m > 0)
-        for (int w = t; w < m + 2; w += nt) {
-          const int pos = order[w];
-          const float4 h = Hs[pos + 1], hp = Hs[pos + 2], hm = Hs[pos];
-          const float d[S] = {h.x, h.y, h.z, h.w};
-          const double sd = dsum32(d);
-          float v[NP];
-          interp32(P, d, sd, nullptr, nullptr, v, &nn);
-          const float np[S] = {hp.x, hp.y, hp.z, hp.w}, nm[S] = {hm.x, hm.y, hm.z, hm.w};
-          float lk[S];
+      for (int w = t; w < m + 2; w += nt) {
+        const int pos = order[w];
+        const float4 h = Hs[pos + 1], hp = Hs[pos + 2], hm = Hs[pos];
+        const float d[S] = {h.x, h.y, h.z, h.w};
+        const double sd = dsum32(d);
+        float v[NP];
+        interp32(P, d, sd, nullptr, nullptr, v, &nn);
+        const float np[S] = {hp.x, hp.y, hp.z, hp.w}, nm[S] = {hm.x, hm.y, hm.z, hm.w};
+        float lk[S];
 #pragma unroll
-          for (int c = 0; c < S; ++c) {
-            const float nb2[2] = {np[c], nm[c]};
-            lk[c] = -lap32<2>(nb2, d[c], P.inv_dx2) * P.kappa[c];
-          }
-          Vs[pos] = make_float4(v[0], v[1], v[2], v[3]);
-          Ks[pos] = make_float4(lk[0], lk[1], lk[2], lk[3]);
-          Ms[pos] = make_float4(v[5], v[6], v[7], v[8]);
-          Es[pos] = make_float2(v[4], (float)(P.c_fe - sd));
+        for (int c = 0; c < S; ++c) {
+          const float nb2[2] = {np[c], nm[c]};
+          lk[c] = -lap32<2>(nb2, d[c], P.inv_dx2) * P.kappa[c];
         }
+        Vs[pos] = make_float4(v[0], v[1], v[2], v[3]);
+        Ks[pos] = make_float4(lk[0], lk[1], lk[2], lk[3]);
+        Ms[pos] = make_float4(v[5], v[6], v[7], v[8]);
+        Es[pos] = make_float2(v[4], (float)(P.c_fe - sd));
+      }
     } else {
       if (lane == 0) {
         mbar_expect(bar_a, bytes_a);
@@ -633,18 +632,16 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     __syncthreads();
     // face i lies between mu/M positions i and i+1 (hi positions i+1, i+2)
-    if (m > 0) {
-      const double mean = P.sp ? sm.mean : 0.0;
-      auto mu_at = [&](int q) {
-        const float spv = P.sp ? (float)(bn * ((double)Qs[q] - mean) + b0 * mean) : 0.f;
-        const float4 v = Vs[q], k4 = Ks[q];
-        return make_float4(v.x + fmaf(spv, P.lvec[0], k4.x), v.y + fmaf(spv, P.lvec[1], k4.y),
-                           v.z + fmaf(spv, P.lvec[2], k4.z), v.w + fmaf(spv, P.lvec[3], k4.w));
-      };
-      for (int i = t; i < m + 1; i += (int)blockDim.x)
-        Fs[i] = face_flux32(P, Hs[i + 1], mu_at(i), Ms[i], Es[i], Hs[i + 2], mu_at(i + 1), Ms[i + 1],
-                            Es[i + 1]);
-    }
+    const double mean = P.sp ? sm.mean : 0.0;
+    auto mu_at = [&](int q) {
+      const float spv = P.sp ? (float)(bn * ((double)Qs[q] - mean) + b0 * mean) : 0.f;
+      const float4 v = Vs[q], k4 = Ks[q];
+      return make_float4(v.x + fmaf(spv, P.lvec[0], k4.x), v.y + fmaf(spv, P.lvec[1], k4.y),
+                         v.z + fmaf(spv, P.lvec[2], k4.z), v.w + fmaf(spv, P.lvec[3], k4.w));
+    };
+    for (int i = t; i < m + 1; i += (int)blockDim.x)
+      Fs[i] = face_flux32(P, Hs[i + 1], mu_at(i), Ms[i], Es[i], Hs[i + 2], mu_at(i + 1), Ms[i + 1],
+                          Es[i + 1]);
     __syncthreads();
     float vmax32 = 0.f;
     for (int p = t; p < m; p += (int)blockDim.x) {

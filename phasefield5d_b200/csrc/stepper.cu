@@ -1270,10 +1270,11 @@ __global__ void __launch_bounds__(kElastic1dThreads)
 //     thread then forms the same dt; update and clamp;
 //   B, to every block: each 32 points' misfit sum and out-of-bounds flags; to
 //     the neighbours: the points of their halos.
-// One copy of each message is enough: a block sends A of a step only when it
-// has all of B of the step before, and every warp has read that by then; it
-// sends B only when it has all of A, and B leaves after the block's barrier
-// that follows the reads of A.
+// One copy of each message is enough.  A block sends A of a step only when it
+// has all of B of the step before, and every block sends B (loop1d_shape leaves
+// none without points) after its barrier that follows its reads of A.  A block
+// sends B only when it has all of A, which every warp sends after its reads of
+// B.
 // Values are formed as k_elastic1d, k_rate_1d, k_dt_finish and k_update_step
 // form them.  The positions are taken in the order of their table cells, so
 // that the lanes of a warp read few nodes; the cells hardly change from step to
@@ -1321,10 +1322,10 @@ __global__ void __launch_bounds__(MAXT, 1)
   const int nw = (int)blockDim.x >> 5, nt = (int)blockDim.x - 32;   // the last warp sums
   const bool worker = t < nt;
   const int rank = (int)cluster.block_rank(), nb = (int)cluster.num_blocks();
-  const int i0 = rank * chunk, m = max(0, min(chunk, n - i0));
+  const int i0 = rank * chunk, m = min(chunk, n - i0);     // m > 0 (loop1d_shape)
   const int ng = (n + 31) / 32;
   const unsigned bar_a = shared_addr(&sm.bar_a), bar_b = shared_addr(&sm.bar_b);
-  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + (m > 0 ? sizeof(sm.halo) : 0u);
+  const unsigned bytes_a = 16u * nb * nw, bytes_b = 16u * ng + sizeof(sm.halo);
   double dt = st->dt, time = st->time, xdotmax = st->xdotmax;
   long long step = st->step;
   // steps until the next out-of-bounds test (the one after which step is a multiple)
@@ -1344,8 +1345,8 @@ __global__ void __launch_bounds__(MAXT, 1)
   unsigned hdst = 0, hbar = 0;
   {
     const int b = t >> 2, h = t & 3;
-    const int bm = b < nb ? max(0, min(chunk, n - b * chunk)) : 0;
-    if (bm > 0 && m > 0) {
+    if (b < nb) {
+      const int bm = min(chunk, n - b * chunk);
       const int src = wrap_any(b * chunk + (h < 2 ? h - 2 : bm + h - 2), n) - i0;
       if (src >= 0 && src < m) {
         hsrc = src + 2;
@@ -1421,7 +1422,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   for (int k = 0; k <= nsteps; ++k) {
     // B of the step before (k = 0: the state at the launch)
     stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
-    if (t < 8 && m > 0) {                // halo entries into the chunk's rows
+    if (t < 8) {                         // halo entries into the chunk's rows
       const int h = t >> 1, c = 2 * (t & 1), p = h < 2 ? h : m + h;
       const ulonglong2 v = sm.halo[h][t & 1];
       Xs[c * HX + p] = __longlong_as_double((long long)v.x);
@@ -1436,27 +1437,26 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     if (__syncthreads_or(stalled)) stalled = true;
     if (halt || stalled || k == nsteps) break;
-    if (m > 0 && k % kLoop1dResort == 0) sort_cells();
+    if (k % kLoop1dResort == 0) sort_cells();
     unsigned nn = 0;
     if (worker) {
-      if (m > 0)
-        for (int w = t; w < m + 2; w += nt) {
-          const int pos = order[w];
-          double x[S], v[NP];
+      for (int w = t; w < m + 2; w += nt) {
+        const int pos = order[w];
+        double x[S], v[NP];
 #pragma unroll
-          for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + pos + 1];
-          interp_point<VEC>(P.T, x, v, &nn);
+        for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + pos + 1];
+        interp_point<VEC>(P.T, x, v, &nn);
 #pragma unroll
-          for (int c = 0; c < S; ++c) {
-            const double *q = Xs + c * HX + pos + 1;
-            const double lap = (q[1] + q[-1] - 2.0 * x[c]) * P.inv_dx2;
-            const double lk = lap * P.kappa.v[c];
-            Ms[c * MX + pos] = v[c] - lk;
-          }
-#pragma unroll
-          for (int c = 0; c < NM; ++c) Ms[(S + c) * MX + pos] = v[S + c];
-          if (P.sp) Qs[pos] = misfit(x);
+        for (int c = 0; c < S; ++c) {
+          const double *q = Xs + c * HX + pos + 1;
+          const double lap = (q[1] + q[-1] - 2.0 * x[c]) * P.inv_dx2;
+          const double lk = lap * P.kappa.v[c];
+          Ms[c * MX + pos] = v[c] - lk;
         }
+#pragma unroll
+        for (int c = 0; c < NM; ++c) Ms[(S + c) * MX + pos] = v[S + c];
+        if (P.sp) Qs[pos] = misfit(x);
+      }
     } else {
       if (lane == 0) {
         mbar_expect(bar_a, bytes_a);
@@ -1472,32 +1472,30 @@ __global__ void __launch_bounds__(MAXT, 1)
     }
     __syncthreads();
     // face i lies between mu/M positions i and i+1 (X positions i+1, i+2)
-    if (m > 0) {
-      const double mean = sm.mean;
-      for (int i = t; i < m + 1; i += (int)blockDim.x) {
-        double Xc[S], Xn[S], Mc[NM], Mn[NM], g[S], J[S];
-        const double sc = P.sp ? bn * (Qs[i] - mean) + b0 * mean : 0.0;
-        const double sn = P.sp ? bn * (Qs[i + 1] - mean) + b0 * mean : 0.0;
+    const double mean = sm.mean;
+    for (int i = t; i < m + 1; i += (int)blockDim.x) {
+      double Xc[S], Xn[S], Mc[NM], Mn[NM], g[S], J[S];
+      const double sc = P.sp ? bn * (Qs[i] - mean) + b0 * mean : 0.0;
+      const double sn = P.sp ? bn * (Qs[i + 1] - mean) + b0 * mean : 0.0;
 #pragma unroll
-        for (int c = 0; c < S; ++c) {
-          Xc[c] = Xs[c * HX + i + 1];
-          Xn[c] = Xs[c * HX + i + 2];
-          double muc = Ms[c * MX + i], mun = Ms[c * MX + i + 1];
-          if (P.sp) {
-            muc = muc + sc * P.lvec.v[c];
-            mun = mun + sn * P.lvec.v[c];
-          }
-          g[c] = (mun - muc) * P.inv_dx;
+      for (int c = 0; c < S; ++c) {
+        Xc[c] = Xs[c * HX + i + 1];
+        Xn[c] = Xs[c * HX + i + 2];
+        double muc = Ms[c * MX + i], mun = Ms[c * MX + i + 1];
+        if (P.sp) {
+          muc = muc + sc * P.lvec.v[c];
+          mun = mun + sn * P.lvec.v[c];
         }
-#pragma unroll
-        for (int c = 0; c < NM; ++c) {
-          Mc[c] = Ms[(S + c) * MX + i];
-          Mn[c] = Ms[(S + c) * MX + i + 1];
-        }
-        face_flux8(Xc, Mc, Xn, Mn, g, J);
-#pragma unroll
-        for (int c = 0; c < S; ++c) Fs[c * FX + i] = J[c];
+        g[c] = (mun - muc) * P.inv_dx;
       }
+#pragma unroll
+      for (int c = 0; c < NM; ++c) {
+        Mc[c] = Ms[(S + c) * MX + i];
+        Mn[c] = Ms[(S + c) * MX + i + 1];
+      }
+      face_flux8(Xc, Mc, Xn, Mn, g, J);
+#pragma unroll
+      for (int c = 0; c < S; ++c) Fs[c * FX + i] = J[c];
     }
     __syncthreads();
     double vmax = 0.0;
