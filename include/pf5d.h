@@ -55,7 +55,9 @@ typedef enum {
 #define PF5D_FLAG_HALTED       0x40u  /* step loop stopped (OOB check or an NN error) */
 #define PF5D_FLAG_NN_NONFINITE 0x80u  /* a fallback point had a NaN/inf component   */
 #define PF5D_FLAG_STALLED      0x100u /* the 1D step loop's blocks lost each other: a
-                                         wait gave up; halted, field as before the call */
+                                         wait gave up (an error, not a halt of the solve).
+                                         Field, dt, time and step are those after the
+                                         launches before it, of up to 2000 steps each */
 /* The nearest-row search is exact for every finite point (it widens its
  * window until the nearest present node is proven).  NN_FAR, NN_TRUNCATED and
  * NN_NONFINITE are errors where the reference raises (RuntimeError for the
@@ -212,6 +214,10 @@ pf5d_status pf5d_stepper_create(const pf5d_stepper_desc *desc, double *X, void *
                                 pf5d_stepper **out);
 /* Enqueue n steps on `stream` (no host synchronisation). */
 pf5d_status pf5d_stepper_advance(pf5d_stepper *h, int64_t nsteps, void *stream);
+/* Longest wait of the 1D step loop's blocks for one another (2 s at creation),
+ * after which the launch ends with PF5D_FLAG_STALLED; 0: one look.  At most an
+ * hour. */
+pf5d_status pf5d_stepper_set_wait_limit(pf5d_stepper *h, double seconds);
 /* Synchronise `stream` and copy the device step state to *out. */
 pf5d_status pf5d_stepper_state(pf5d_stepper *h, pf5d_step_state *out, void *stream);
 /* Device pointer to the last dX/dt buffer ((*shape, 4); float64 for FP64,

@@ -106,6 +106,7 @@ _SIGS = {
     "pf5d_adaptive_dt": (_f64, [_f64, _f64, _f64, _f64, _f64, _f64, _f64]),
     "pf5d_stepper_create": (_i32, [ctypes.POINTER(StepperDesc), _vp, _vp, ctypes.POINTER(_vp)]),
     "pf5d_stepper_advance": (_i32, [_vp, _i64, _vp]),
+    "pf5d_stepper_set_wait_limit": (_i32, [_vp, _f64]),
     "pf5d_stepper_state": (_i32, [_vp, ctypes.POINTER(StepState), _vp]),
     "pf5d_stepper_rate": (_vp, [_vp]),
     "pf5d_stepper_field": (_i32, [_vp, _vp, _vp]),
@@ -183,6 +184,15 @@ def check(status, what=""):
 
 NN_NONFINITE_MSG = "'x' must be finite, check for nan or inf values"
 NN_FAR_MSG = "Some compositions are outside the CALPHAD domain (KD-tree)."
+
+STALLED_MSG = ("the 1D step loop stalled: its blocks lost each other; field, dt, time and step are "
+               "those of the last launch that ended well")
+
+
+def raise_stalled(flags):
+    """Raise where a launch of the 1D step loop gave up (not a halt of the solve)."""
+    if flags & FLAG_STALLED:
+        raise RuntimeError(STALLED_MSG)
 
 
 def nn_flags(flags):

@@ -74,16 +74,50 @@ __device__ __forceinline__ void mbar_init(unsigned bar) {
 __device__ __forceinline__ void mbar_expect(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
 }
-constexpr int kMbarTries = 1 << 22;          // then the wait gives up
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// Waits of a warp for a phase; false, for all its lanes, when `limit` ns have
+// passed (0: one look) or, whatever the clock says, after kMbarTries tries.
+constexpr int kMbarTries = 1 << 24;
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, unsigned long long limit) {
+  unsigned ok;
+  asm volatile("{\n.reg .pred p;\n"
+               "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+               "selp.b32 %0, 1, 0, p;\n}"
+               : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  if (__all_sync(0xffffffffu, ok)) return true;
+  if (limit == 0) return false;
+  unsigned long long start = 0;
   for (int i = 0; i < kMbarTries; ++i) {
-    unsigned ok;
     asm volatile("{\n.reg .pred p;\n"
                  "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
                  "selp.b32 %0, 1, 0, p;\n}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    if (ok) return true;
+    if (__all_sync(0xffffffffu, ok)) return true;
+    const unsigned long long now = __shfl_sync(0xffffffffu, now_ns(), 0);
+    if (i == 0) start = now;
+    else if (now - start > limit) break;
   }
+  return false;
+}
+
+// The blocks' common verdict after the last step, before any of them stores:
+// true where no block gave up.  After a wait that gave up, messages may still be
+// on their way to a block that has stopped waiting for them; no block leaves
+// before they have come (a few us; kDrainNs, or kMbarTries looks at the clock).
+// `failed` in shared memory is 0 since before the first cluster barrier.
+constexpr unsigned long long kDrainNs = 1000000;
+__device__ __forceinline__ bool cluster_agrees(cooperative_groups::cluster_group &cluster,
+                                               unsigned *failed, bool stalled) {
+  if (stalled && threadIdx.x < cluster.num_blocks())
+    *cluster.map_shared_rank(failed, threadIdx.x) = 1u;
+  cluster.sync();
+  if (!*reinterpret_cast<volatile unsigned *>(failed)) return true;
+  const unsigned long long start = now_ns();
+  for (int i = 0; i < kMbarTries && now_ns() - start < kDrainNs; ++i) __nanosleep(1000);
   return false;
 }
 

@@ -19,6 +19,7 @@ struct Stepper32;
 pf5d_status s32_create(const pf5d_stepper_desc *desc, const double *X_init, void *stream,
                        Stepper32 **out);
 pf5d_status s32_advance(Stepper32 *h, int64_t nsteps, void *stream);
+void s32_set_wait_limit(Stepper32 *h, unsigned long long ns);
 pf5d_status s32_state(Stepper32 *h, pf5d_step_state *out, void *stream);
 pf5d_status s32_field(Stepper32 *h, double *X_out, void *stream);
 pf5d_status s32_mass(Stepper32 *h, double *mean_out, void *stream);

@@ -10,6 +10,7 @@ constexpr int64_t kLoop1dMax = 16384;        // points of a 1D solve that a clus
 constexpr int kLoop1dThreads = 512;          // most threads of a block (128 registers each)
 constexpr int kLoop1dBlocks = 16;            // most blocks of a cluster
 constexpr int kLoop1dSteps = 2000;           // most steps of a launch
+constexpr unsigned long long kLoop1dWaitNs = 2000000000;   // longest wait of a block for the others
 constexpr int kLoop1dGroups = (int)(kLoop1dMax / 32);
 
 // Blocks of the cluster, points per block (a multiple of 32) and threads per

@@ -451,7 +451,8 @@ struct Loop1dSmem32 {
   ulonglong2 halo[4][2];                 // B: positions -2, -1, m, m + 1: hi; misfit
   double own[kLoop1dGroups];             // this block's groups, before they are sent
   unsigned own_flags[kLoop1dGroups];
-  double mean, pad;
+  double mean;
+  unsigned failed, pad;                  // a block gave up
   unsigned long long bar_a, bar_b;
   int bins[256];                         // of the cell sort
 };
@@ -467,7 +468,8 @@ constexpr int kLoop1dResort32 = 128;
 
 template <int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
-    k32_loop1d(Rate32 P, Update32 U, double bn, double b0, int chunk, int nsteps) {
+    k32_loop1d(Rate32 P, Update32 U, double bn, double b0, int chunk, int nsteps,
+               unsigned long long limit) {
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   extern __shared__ __align__(16) unsigned char lraw[];
   Loop1dSmem32 &sm = *reinterpret_cast<Loop1dSmem32 *>(lraw);
@@ -558,6 +560,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   };
 
   if (t == 0) {
+    sm.failed = 0;
     mbar_init(bar_a);
     mbar_init(bar_b);
   }
@@ -580,7 +583,7 @@ __global__ void __launch_bounds__(MAXT, 1)
 
   for (int k = 0; k <= nsteps; ++k) {
     // B of the step before (k = 0: the state at the launch)
-    stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
+    if (!stalled && !halt) stalled = !mbar_wait(bar_b, (unsigned)k & 1u, limit);
     if (t < 4) {                         // halo entries into the chunk's rows
       const int p = t < 2 ? t : m + t;
       *reinterpret_cast<ulonglong2 *>(Hs + p) = sm.halo[t][0];
@@ -593,7 +596,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       flags |= f;
       if (f & (PF5D_FLAG_NONFINITE | PF5D_FLAG_OOB_HARD)) halt = true;
     }
-    if (__syncthreads_or(stalled)) stalled = true;
+    stalled = __syncthreads_or(stalled);
     if (halt || stalled || k == nsteps) break;
     if (k % kLoop1dResort32 == 0) sort_cells();
     unsigned nn = 0;
@@ -660,7 +663,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (lane < nb)
       send2(rank_addr(shared_addr(&sm.max[rank * nw + warp]), lane), rank_addr(bar_a, lane),
             __float_as_uint(vmax32), nn);
-    stalled = stalled || !mbar_wait(bar_a, (unsigned)k & 1u);       // A
+    stalled = !mbar_wait(bar_a, (unsigned)k & 1u, limit);           // A
     unsigned gbits = 0;
     nn = 0;
     for (int i = lane; i < nb * nw; i += 32) {
@@ -670,64 +673,65 @@ __global__ void __launch_bounds__(MAXT, 1)
     const double gmax = (double)__uint_as_float(__reduce_max_sync(0xffffffffu, gbits));
     nn = __reduce_or_sync(0xffffffffu, nn);
     flags |= nn;
-    if (nn & kNNErrorFlags) {            // the same in every block: stop before the update
-      halt = true;
-      break;
-    }
-    if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
-    time = time + dt;
-    xdotmax = gmax;
-    step = step + 1;
-    checked = --to_check == 0;
-    if (checked) to_check = U.oob_interval;
-    const float dtf = (float)dt;
-    for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
-      const int p = p0 + lane;
-      unsigned fo = 0;
-      float s = 0.f;
-      if (p < m) {
-        const float4 H = Hs[p + 2], L = Ls[p], R = Ds[p];
-        float h[S] = {H.x, H.y, H.z, H.w}, l[S] = {L.x, L.y, L.z, L.w};
-        const float r[S] = {R.x, R.y, R.z, R.w};
-        double dd[S];
-        update_point32(U, dtf, r, h, l, dd);
-        const float4 hn = make_float4(h[0], h[1], h[2], h[3]), ln = make_float4(l[0], l[1], l[2], l[3]);
-        Hs[p + 2] = hn;
-        Ls[p] = ln;
-        s = misfit(hn, ln);
-        Qs[p + 1] = s;
-        if (checked) {
-          double x[S];
+    // an error of the fallback, the same in every block: stop before the update
+    halt = !stalled && (nn & kNNErrorFlags);
+    if (!stalled && !halt) {
+      if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
+      time = time + dt;
+      xdotmax = gmax;
+      step = step + 1;
+      checked = --to_check == 0;
+      if (checked) to_check = U.oob_interval;
+      const float dtf = (float)dt;
+      for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+        const int p = p0 + lane;
+        unsigned fo = 0;
+        float s = 0.f;
+        if (p < m) {
+          const float4 H = Hs[p + 2], L = Ls[p], R = Ds[p];
+          float h[S] = {H.x, H.y, H.z, H.w}, l[S] = {L.x, L.y, L.z, L.w};
+          const float r[S] = {R.x, R.y, R.z, R.w};
+          double dd[S];
+          update_point32(U, dtf, r, h, l, dd);
+          const float4 hn = make_float4(h[0], h[1], h[2], h[3]), ln = make_float4(l[0], l[1], l[2], l[3]);
+          Hs[p + 2] = hn;
+          Ls[p] = ln;
+          s = misfit(hn, ln);
+          Qs[p + 1] = s;
+          if (checked) {
+            double x[S];
 #pragma unroll
-          for (int c = 0; c < S; ++c) x[c] = U.x0[c] + dd[c];
-          fo = oob_flags_x(x);
+            for (int c = 0; c < S; ++c) x[c] = U.x0[c] + dd[c];
+            fo = oob_flags_x(x);
+          }
         }
+        keep_group(s, p0, fo);
       }
-      keep_group(s, p0, fo);
     }
     __syncthreads();
-    send_b();
+    // a warp that gave up leaves with its block, after the next barrier
+    if (!stalled && !halt) send_b();
   }
 
-  if (!stalled)
+  if (cluster_agrees(cluster, &sm.failed, stalled)) {
     for (int p = t; p < m; p += (int)blockDim.x) {
       U.hi[i0 + p] = Hs[p + 2];
       U.lo[i0 + p] = Ls[p];
       P.dX[i0 + p] = Ds[p];
       if (U.s) U.s[i0 + p] = Qs[p + 1];
     }
-  if (stalled && t == 0) {
+    if (rank == 0 && t == 0) {
+      st->dt = dt;
+      st->time = time;
+      st->xdotmax = xdotmax;
+      st->step = step;
+      if (flags) atomicOr(&st->flags, flags);
+      if (halt) atomicExch(&st->halt, 1u);
+    }
+  } else if (rank == 0 && t == 0) {
     atomicOr(&st->flags, PF5D_FLAG_STALLED);
     atomicExch(&st->halt, 1u);
-  } else if (rank == 0 && t == 0) {
-    st->dt = dt;
-    st->time = time;
-    st->xdotmax = xdotmax;
-    st->step = step;
-    if (flags) atomicOr(&st->flags, flags);
-    if (halt) atomicExch(&st->halt, 1u);
   }
-  cluster.sync();                        // no block leaves while another may still send to it
 }
 
 __global__ void k32_bmul(cufftComplex *__restrict__ k, const float *__restrict__ bk, int64_t nk,
@@ -841,6 +845,7 @@ struct Stepper32 {
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
   bool use_loop1d = false;       // 1D steps by k32_loop1d
   Loop1dShape loop;
+  unsigned long long wait_ns = kLoop1dWaitNs;   // its blocks' longest wait
   int64_t shape[3] = {1, 1, 1};
   int64_t npts = 0, nk = 0;
   float4 *hi = nullptr, *lo = nullptr, *dX = nullptr;
@@ -995,7 +1000,7 @@ static pf5d_status graph32(Stepper32 *h, int64_t n, cudaGraphExec_t *out) {
 }
 
 // The step loop of a 1D solve (255 registers a thread in small blocks).
-using Loop1dKernel32 = void (*)(Rate32, Update32, double, double, int, int);
+using Loop1dKernel32 = void (*)(Rate32, Update32, double, double, int, int, unsigned long long);
 static Loop1dKernel32 loop1d_kernel32(const Stepper32 *h) {
   return h->loop.threads <= kLoop1dThreads / 2 ? k32_loop1d<kLoop1dThreads / 2>
                                                : k32_loop1d<kLoop1dThreads>;
@@ -1175,7 +1180,7 @@ pf5d_status s32_advance(Stepper32 *h, int64_t nsteps, void *stream) {
     for (; nsteps > 0; nsteps -= kLoop1dSteps) {
       const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);
       PF5D_CUDA(launch_cluster(loop1d_kernel32(h), h->loop, sm, s, h->rp, h->up, h->bn, h->b0,
-                               h->loop.chunk, n));
+                               h->loop.chunk, n, h->wait_ns));
     }
     return PF5D_OK;
   }
@@ -1189,6 +1194,8 @@ pf5d_status s32_advance(Stepper32 *h, int64_t nsteps, void *stream) {
   }
   return PF5D_OK;
 }
+
+void s32_set_wait_limit(Stepper32 *h, unsigned long long ns) { h->wait_ns = ns; }
 
 pf5d_status s32_state(Stepper32 *h, pf5d_step_state *out, void *stream) {
   StepState32 hs;

@@ -1293,7 +1293,8 @@ struct Loop1dSmem {
   ulonglong2 halo[4][2];                 // B: positions -2, -1, m, m + 1
   double own[kLoop1dGroups];             // this block's groups, before they are sent
   unsigned own_flags[kLoop1dGroups];
-  double mean, pad;
+  double mean;
+  unsigned failed, pad;                  // a block gave up
   unsigned long long bar_a, bar_b;
   int bins[256];                         // of the cell sort
 };
@@ -1308,7 +1309,8 @@ constexpr int kLoop1dResort = 128;
 
 template <bool VEC, int MAXT>
 __global__ void __launch_bounds__(MAXT, 1)
-    k_loop1d(RateParams P, UpdateParams U, double bn, double b0, int chunk, int nsteps) {
+    k_loop1d(RateParams P, UpdateParams U, double bn, double b0, int chunk, int nsteps,
+             unsigned long long limit) {
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   extern __shared__ __align__(16) unsigned char lraw[];
   Loop1dSmem &sm = *reinterpret_cast<Loop1dSmem *>(lraw);
@@ -1397,6 +1399,7 @@ __global__ void __launch_bounds__(MAXT, 1)
   };
 
   if (t == 0) {
+    sm.failed = 0;
     mbar_init(bar_a);
     mbar_init(bar_b);
   }
@@ -1421,7 +1424,7 @@ __global__ void __launch_bounds__(MAXT, 1)
 
   for (int k = 0; k <= nsteps; ++k) {
     // B of the step before (k = 0: the state at the launch)
-    stalled = stalled || !mbar_wait(bar_b, (unsigned)k & 1u);
+    if (!stalled && !halt) stalled = !mbar_wait(bar_b, (unsigned)k & 1u, limit);
     if (t < 8) {                         // halo entries into the chunk's rows
       const int h = t >> 1, c = 2 * (t & 1), p = h < 2 ? h : m + h;
       const ulonglong2 v = sm.halo[h][t & 1];
@@ -1435,7 +1438,7 @@ __global__ void __launch_bounds__(MAXT, 1)
       flags |= f;
       if (f & (PF5D_FLAG_NONFINITE | PF5D_FLAG_OOB_HARD)) halt = true;
     }
-    if (__syncthreads_or(stalled)) stalled = true;
+    stalled = __syncthreads_or(stalled);
     if (halt || stalled || k == nsteps) break;
     if (k % kLoop1dResort == 0) sort_cells();
     unsigned nn = 0;
@@ -1512,7 +1515,7 @@ __global__ void __launch_bounds__(MAXT, 1)
     if (lane < nb)
       send2(rank_addr(shared_addr(&sm.max[rank * nw + warp]), lane), rank_addr(bar_a, lane),
             (unsigned long long)__double_as_longlong(vmax), nn);
-    stalled = stalled || !mbar_wait(bar_a, (unsigned)k & 1u);       // A
+    stalled = !mbar_wait(bar_a, (unsigned)k & 1u, limit);           // A
     double gmax = 0.0;
     nn = 0;
     for (int i = lane; i < nb * nw; i += 32) {
@@ -1522,42 +1525,43 @@ __global__ void __launch_bounds__(MAXT, 1)
     gmax = warp_max_nonneg(gmax);
     nn = __reduce_or_sync(0xffffffffu, nn);
     flags |= nn;
-    if (nn & kNNErrorFlags) {            // the same in every block: stop before the update
-      halt = true;
-      break;
-    }
-    if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
-    time = time + dt;
-    xdotmax = gmax;
-    step = step + 1;
-    checked = --to_check == 0;
-    if (checked) to_check = U.oob_interval;
-    for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
-      const int p = p0 + lane;
-      double x[S] = {0.0, 0.0, 0.0, 0.0};
-      unsigned fo = 0;
-      if (p < m) {
+    // an error of the fallback, the same in every block: stop before the update
+    halt = !stalled && (nn & kNNErrorFlags);
+    if (!stalled && !halt) {
+      if (P.adaptive) dt = adaptive_dt(dt, gmax, P.ctld, P.t_cfl, P.lower, P.upper, P.factor);
+      time = time + dt;
+      xdotmax = gmax;
+      step = step + 1;
+      checked = --to_check == 0;
+      if (checked) to_check = U.oob_interval;
+      for (int p0 = 32 * warp; p0 < m; p0 += 32 * nw) {
+        const int p = p0 + lane;
+        double x[S] = {0.0, 0.0, 0.0, 0.0};
+        unsigned fo = 0;
+        if (p < m) {
 #pragma unroll
-        for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + p + 2] + Ds[c * chunk + p] * dt;
-        double sum = 0.0;
+          for (int c = 0; c < S; ++c) x[c] = Xs[c * HX + p + 2] + Ds[c * chunk + p] * dt;
+          double sum = 0.0;
 #pragma unroll
-        for (int c = 0; c < S; ++c) sum = sum + x[c];
-        if (sum > 1.0) {
-          const double inv = 1.0 / sum;
+          for (int c = 0; c < S; ++c) sum = sum + x[c];
+          if (sum > 1.0) {
+            const double inv = 1.0 / sum;
 #pragma unroll
-          for (int c = 0; c < S; ++c) x[c] = x[c] * inv;
+            for (int c = 0; c < S; ++c) x[c] = x[c] * inv;
+          }
+#pragma unroll
+          for (int c = 0; c < S; ++c) Xs[c * HX + p + 2] = x[c];
+          if (checked) fo = oob_flags(x);
         }
-#pragma unroll
-        for (int c = 0; c < S; ++c) Xs[c * HX + p + 2] = x[c];
-        if (checked) fo = oob_flags(x);
+        keep_group(x, p0, fo);
       }
-      keep_group(x, p0, fo);
     }
     __syncthreads();
-    send_b();
+    // a warp that gave up leaves with its block, after the next barrier
+    if (!stalled && !halt) send_b();
   }
 
-  if (!stalled)
+  if (cluster_agrees(cluster, &sm.failed, stalled)) {
     for (int p = t; p < m; p += (int)blockDim.x) {
       double x[S], d[S];
 #pragma unroll
@@ -1574,18 +1578,18 @@ __global__ void __launch_bounds__(MAXT, 1)
       o[1] = make_double2(d[2], d[3]);
       if (U.s) U.s[g] = misfit(x);
     }
-  if (stalled && t == 0) {
+    if (rank == 0 && t == 0) {
+      st->dt = dt;
+      st->time = time;
+      st->xdotmax = xdotmax;
+      st->step = step;
+      if (flags) atomicOr(&st->flags, flags);
+      if (halt) atomicExch(&st->halt, 1u);
+    }
+  } else if (rank == 0 && t == 0) {
     atomicOr(&st->flags, PF5D_FLAG_STALLED);
     atomicExch(&st->halt, 1u);
-  } else if (rank == 0 && t == 0) {
-    st->dt = dt;
-    st->time = time;
-    st->xdotmax = xdotmax;
-    st->step = step;
-    if (flags) atomicOr(&st->flags, flags);
-    if (halt) atomicExch(&st->halt, 1u);
   }
-  cluster.sync();                        // no block leaves while another may still send to it
 }
 
 }  // namespace pf5d
@@ -1622,6 +1626,7 @@ struct pf5d_stepper {
   double bn = 0.0, b0 = 0.0;     // its B(k): bn for every k != 0, b0 at k = 0
   bool use_loop1d = false;       // 1D steps by k_loop1d
   Loop1dShape loop;
+  unsigned long long wait_ns = kLoop1dWaitNs;   // its blocks' longest wait
   double *save_x = nullptr;      // FP32C save steps: FP64 field, dX/dt, mu/M
   std::string kernels;           // text returned by pf5d_stepper_rate_kernels
 };
@@ -1958,7 +1963,7 @@ pf5d_status enqueue_step(pf5d_stepper *h, cudaStream_t s) {
 
 // The step loop of a 1D solve.  Blocks of up to 256 threads may take 255
 // registers each, which lets the table loads run ahead of the sums.
-using Loop1dKernel = void (*)(RateParams, UpdateParams, double, double, int, int);
+using Loop1dKernel = void (*)(RateParams, UpdateParams, double, double, int, int, unsigned long long);
 Loop1dKernel loop1d_kernel(const pf5d_stepper *h) {
   const bool few = h->loop.threads <= kLoop1dThreads / 2;
   if (h->vec) return few ? k_loop1d<true, kLoop1dThreads / 2> : k_loop1d<true, kLoop1dThreads>;
@@ -2175,7 +2180,7 @@ pf5d_status pf5d_stepper_advance(pf5d_stepper *h, int64_t nsteps, void *stream) 
     for (; nsteps > 0; nsteps -= kLoop1dSteps) {
       const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);
       PF5D_CUDA(launch_cluster(loop1d_kernel(h), h->loop, sm, s, h->rp, h->up, h->bn, h->b0,
-                               h->loop.chunk, n));
+                               h->loop.chunk, n, h->wait_ns));
     }
     return PF5D_OK;
   }
@@ -2187,6 +2192,14 @@ pf5d_status pf5d_stepper_advance(pf5d_stepper *h, int64_t nsteps, void *stream) 
     PF5D_CUDA(cudaGraphLaunch(g, s));
     nsteps -= n;
   }
+  return PF5D_OK;
+}
+
+pf5d_status pf5d_stepper_set_wait_limit(pf5d_stepper *h, double seconds) {
+  PF5D_REQUIRE(h && seconds >= 0.0 && seconds <= 3600.0, PF5D_ERR_ARG, "bad arguments");
+  const auto ns = (unsigned long long)(seconds * 1e9);
+  if (h->s32) s32_set_wait_limit(h->s32, ns);
+  else h->wait_ns = ns;
   return PF5D_OK;
 }
 

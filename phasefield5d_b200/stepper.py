@@ -138,15 +138,21 @@ class Stepper:
         _lib.check(self.L.pf5d_stepper_advance(self.h, int(n_steps), self._s()), "advance")
         self.steps_enqueued += int(n_steps)
 
+    def set_wait_limit(self, seconds):
+        """Longest wait of the 1D step loop's blocks for one another."""
+        _lib.check(self.L.pf5d_stepper_set_wait_limit(self.h, float(seconds)), "set_wait_limit")
+
     def state(self):
         """Synchronise and return {dt, time, xdotmax, step, flags, halted}
         plus the decoded nearest-row fallback bits: ``nn_used`` (some point
         took the fallback), ``nn_far`` (a row farther than max_nn_dist),
         ``nn_nonfinite`` (a non-finite composition reached the fallback) and
         ``nn_no_row``.  The last three halt the loop before that step's
-        update, where the reference's loop raises."""
+        update, where the reference's loop raises.  RuntimeError: the 1D step
+        loop gave up (``reset`` starts it again)."""
         st = _lib.StepState()
         _lib.check(self.L.pf5d_stepper_state(self.h, ctypes.byref(st), self._s()), "state")
+        _lib.raise_stalled(int(st.flags))
         out = dict(dt=st.dt, time=st.time, xdotmax=st.xdotmax, step=int(st.step),
                    flags=int(st.flags), halted=bool(st.halted))
         out.update(_lib.nn_flags(int(st.flags)))
