@@ -132,6 +132,16 @@ __global__ void __launch_bounds__(256) k_laplacian4(int n0, int n1, int n2,
   o[1] = make_double2(lap[2], lap[3]);
 }
 
+// Whether k_laplacian4's 32x8 tiles are full enough: a quarter of the lanes
+// along the last axis and 20 points a block.  us, k_laplacian -> k_laplacian4:
+// 512x512x2 (2 lanes of 32) 21 -> 62, 5000x50x8 (8 lanes) 69 -> 62, 25000x1x8
+// (8 points a block) 11 -> 17, 12500x2x8 (16) 10.5 -> 10.5.  1D tiles are one
+// row of 32 points: 22 -> 19 at 10^6.
+static bool laplacian4_pays(int dim, int64_t nx, int64_t ny, int64_t nz) {
+  const int64_t tx = (nx + 31) / 32, ty = (ny + 7) / 8;
+  return dim == 1 || (nx >= 8 * tx && nx * ny * nz >= 20 * tx * ty * nz);
+}
+
 struct Kappa {
   double k[8];
 };
@@ -159,6 +169,48 @@ __device__ __forceinline__ void load5(const double *p, double v[NM]) {
   for (int s = 0; s < NM; ++s) v[s] = p[s];
 }
 
+// One point per thread, both faces of every axis: any shape.
+__global__ void k_divergence_points(int dim, int64_t n0, int64_t n1, int64_t n2,
+                                    const double *__restrict__ X, const double *__restrict__ M,
+                                    int64_t ms, const double *__restrict__ mu, int64_t mus,
+                                    double inv_dx, double *__restrict__ out) {
+  const int64_t npts = n0 * n1 * n2;
+  for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < npts;
+       p += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = p % n2, j = (p / n2) % n1, i = p / (n2 * n1);
+    int64_t nb[6];
+    nb[0] = (wrap_p(i, n0) * n1 + j) * n2 + k;
+    nb[1] = (wrap_m(i, n0) * n1 + j) * n2 + k;
+    nb[2] = (i * n1 + wrap_p(j, n1)) * n2 + k;
+    nb[3] = (i * n1 + wrap_m(j, n1)) * n2 + k;
+    nb[4] = (i * n1 + j) * n2 + wrap_p(k, n2);
+    nb[5] = (i * n1 + j) * n2 + wrap_m(k, n2);
+    double Xc[S], Mc[NM], muc[S];
+    load4(X + p * S, Xc);
+    load5(M + p * ms, Mc);
+    load4(mu + p * mus, muc);
+    double acc[S];
+    for (int f = 0; f < 2 * dim; ++f) {
+      const int64_t q = nb[f];
+      double Xn[S], Mn[NM], mun[S], g[S], J[S];
+      load4(X + q * S, Xn);
+      load5(M + q * ms, Mn);
+      load4(mu + q * mus, mun);
+#pragma unroll
+      for (int s = 0; s < S; ++s) g[s] = (f & 1) ? (muc[s] - mun[s]) * inv_dx : (mun[s] - muc[s]) * inv_dx;
+      face_flux(Xc, Mc, Xn, Mn, g, J);
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+        if (f == 0) acc[s] = J[s];
+        else if (f & 1) acc[s] = acc[s] - J[s];
+        else acc[s] = acc[s] + J[s];
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) out[p * S + s] = acc[s] * inv_dx;
+  }
+}
+
 // A warp takes 32 neighbouring columns of the last axis and marches along the
 // first, as the split rate stage's k_flux: the face along the march is carried,
 // the face between columns handed on by shuffles (30 columns are finished), and
@@ -168,8 +220,8 @@ __device__ __forceinline__ void load5(const double *p, double v[NM]) {
 // interp[..., 4:]); a warp then reads its 32 rows, one run of 2304 bytes, in
 // memory order and turns them in shared memory, where loads of a column of the
 // rows would touch 18 lines each.
-// Bound by the latency of the loads.  128^3, rows of nine: 212 us with a
-// point and its six neighbours per thread -> 162.
+// Bound by the latency of the loads.  128^3, rows of nine: 212 us with
+// k_divergence_points -> 162.
 constexpr int kDivThreads = 128, kDivCols = 30;
 
 struct DivView {
@@ -297,6 +349,33 @@ __global__ void __launch_bounds__(kDivThreads, 4)
   }
 }
 
+// Whether the march is the faster form: it spends a warp on 30 columns and, in
+// 3D, a block on four rows, full or not; reading rows of nine through shared
+// memory costs it more.  Measured from 16,000 to 3,000,000 points; us, a point
+// per thread -> march:
+//   2D, rows of nine: 12 columns of 32 lanes 4.7 -> 6.2 (16,000 points), 14
+//     columns 8.1 -> 8.1; apart: 8 columns 16.5 -> 18.7, 9 columns 74 -> 61;
+//   3D, rows of nine: 24 columns (0.75) 170 -> 165, 20 (0.62) 12.4 -> 14.4;
+//     2 or 3 rows of 4 still 258 -> 178, 6 rows of 8 12.4 -> 14.4, 1 row of 4
+//     18.7 -> 25; few blocks do not hide its longer steps: 16,000 points 6.3 ->
+//     8.3, 40,000 8.3 -> 8.3, 160,000 18.5 -> 14.5; apart: 31 columns in two
+//     warps (0.48) 22.8 -> 22.8, 12 (0.37) 20.8 -> 22.8; with rows to spare from
+//     0.68 on.
+static bool march_pays(int dim, int64_t npts, int64_t n1, int64_t nx, bool rows9) {
+  const int64_t lanes = 32 * ((nx + kDivCols - 1) / kDivCols);
+  if (dim == 1) return true;
+  if (dim == 2) return 100 * nx >= (rows9 ? 43 : 27) * lanes;
+  const bool full = 8 * n1 >= 28 * ((n1 + 3) / 4);                 // 7 of 8 rows
+  if (rows9)
+    return 100 * nx >= 68 * lanes && ((full && npts >= 32768) || n1 == 2 || n1 == 3);
+  return 100 * nx >= (full ? 45 : 68) * lanes && n1 >= 2;
+}
+
+static bool rows_of_nine(const DivView &V, int64_t nx) {
+  return V.M == V.mu + S && V.mus == NP && V.ms == NP &&
+         nx < (1 << 27);                               // 32-bit offsets in a row of rows
+}
+
 template <int DIM>
 static void launch_divergence(int n0, int n1, int n2, const DivView &V, double inv_dx, double *out,
                               cudaStream_t s) {
@@ -313,8 +392,7 @@ static void launch_divergence(int n0, int n1, int n2, const DivView &V, double i
                                     : tiles * chunks * ((n1 + 3) / 4);
   const dim3 grid((unsigned)blocks);
   const bool wide = aligned_to(V.X, 32);
-  const bool rows9 = V.M == V.mu + S && V.mus == NP && V.ms == NP &&
-                     nx < (1 << 27);                   // 32-bit offsets in a row of rows
+  const bool rows9 = rows_of_nine(V, nx);
   auto kernel = rows9 ? (wide ? k_divergence<DIM, true, 4> : k_divergence<DIM, true, 1>)
                       : (wide ? k_divergence<DIM, false, 4> : k_divergence<DIM, false, 1>);
   kernel<<<grid, kDivThreads, 0, s>>>(n0, n1, n2, V, inv_dx, out, rows);
@@ -612,7 +690,7 @@ pf5d_status pf5d_laplacian(int32_t dim, const int64_t *shape, int32_t ncomp, con
   const int64_t npts = n0 * n1 * n2;
   const int64_t ny = dim == 1 ? 1 : shape[dim - 2], nx = shape[dim - 1], nz = dim == 3 ? n0 : 1;
   if (ncomp == S && (((uintptr_t)c | (uintptr_t)out) & 15) == 0 && nx < (1 << 30) &&
-      ny <= 8 * 65535 && nz <= 65535) {
+      ny <= 8 * 65535 && nz <= 65535 && laplacian4_pays(dim, nx, ny, nz)) {
     const dim3 grid((unsigned)((nx + 31) / 32), (unsigned)((ny + 7) / 8), (unsigned)nz), block(32, 8);
     const bool wide = aligned_to(c, 32);
     auto kernel = dim == 1   ? (wide ? k_laplacian4<1, 4> : k_laplacian4<1, 2>)
@@ -653,7 +731,11 @@ pf5d_status pf5d_divergence_from_mu(int32_t dim, const int64_t *shape, int32_t n
   const DivView V{X, mu, M, mu_stride, m_stride};
   const int a = (int)n0, b = (int)n1, c = (int)n2;
   cudaStream_t s = as_stream(stream);
-  if (dim == 1) launch_divergence<1>(a, b, c, V, inv_dx, out, s);
+  const int64_t nx = dim == 1 ? n0 : (dim == 2 ? n1 : n2), npts = n0 * n1 * n2;
+  if (!march_pays(dim, npts, n1, nx, rows_of_nine(V, nx)))
+    k_divergence_points<<<grid_for(npts, 128), 128, 0, s>>>(dim, n0, n1, n2, X, M, m_stride, mu,
+                                                            mu_stride, inv_dx, out);
+  else if (dim == 1) launch_divergence<1>(a, b, c, V, inv_dx, out, s);
   else if (dim == 2) launch_divergence<2>(a, b, c, V, inv_dx, out, s);
   else launch_divergence<3>(a, b, c, V, inv_dx, out, s);
   PF5D_LAUNCHED();
