@@ -285,8 +285,10 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
 int32_t pf5d_stepper_variant_count(const pf5d_stepper *h);
 /* Kernels of this library that one step launches with the current variant
  * (rate kernel(s), dt controller, update, and when elasticity is on the B(k)
- * multiply or the column kernel in its place; cuFFT's own kernels not counted); 1 for a 1D solve that the step loop advances (one
- * launch for up to 2000 steps); 0 for a null stepper. */
+ * multiply or the column kernel in its place; cuFFT's own kernels not
+ * counted); 1 for a 1D solve that the step loop advances (one launch for up to
+ * 2000 steps; above 10240 points a call of a single step runs the kernels apart);
+ * 0 for a null stepper. */
 int32_t pf5d_stepper_launches_per_step(const pf5d_stepper *h);
 /* The kernel instances one rate stage of the current variant launches, as
  * profilers name them ("k_rate_tile2d<32, 8, 2, 1, 1, 0, 352, 1, 0> +

@@ -28,6 +28,54 @@ __device__ __forceinline__ double sum_groups(const double *sums, int n) {
   return group_sum(v);
 }
 
+// group_sum of 16 groups, a lane's value of group j in v[j], with a fifth of the
+// shuffles: at each of the first four levels a lane keeps half of its groups and
+// hands its values of the other half to the lane that keeps those.  The same
+// pairs are added as in group_sum, in either order, so the same bits.  Returns
+// the sum of group 8 l4 + 4 l3 + 2 l2 + l1 (the lane's bits).
+__device__ __forceinline__ double group_sums16(double v[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int o = 16, n = 8; n > 0; o >>= 1, n >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < n; ++j) {
+      const double got = __shfl_xor_sync(0xffffffffu, up ? v[j] : v[j + n], o);
+      v[j] = (up ? v[j + n] : v[j]) + got;
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
+// Sums of all groups of s (n values, s(i) reads one) into sums[], by a block of
+// 1024 threads: warp w takes the groups 16 w to 16 w + 15, or every 32nd where
+// they are few.
+constexpr int kGroupThreads = 1024;
+static_assert(kLoop1dGroups == 16 * (kGroupThreads / 32), "16 groups a warp");
+template <typename Read>
+__device__ __forceinline__ void block_group_sums(double *sums, int64_t n, Read s) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, ng = (int)((n + 31) / 32);
+  if (ng > 64) {
+    double v[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int64_t i = 32 * (int64_t)(16 * w + j) + lane;
+      v[j] = i < n ? s(i) : 0.0;
+    }
+    if (16 * w < ng) {
+      const double sum = group_sums16(v);
+      if ((lane & 1) == 0) sums[16 * w + (lane >> 1)] = sum;
+    }
+  } else {
+    for (int g = w; g < ng; g += kGroupThreads / 32) {
+      const int64_t i = 32 * (int64_t)g + lane;
+      const double v = group_sum(i < n ? s(i) : 0.0);
+      if (lane == 0) sums[g] = v;
+    }
+  }
+  __syncthreads();
+}
+
 // Exclusive prefix sum of 256 shared counters by one warp.
 __device__ __forceinline__ void scan_bins256(int *bins, int lane) {
   int v[8], sum = 0;

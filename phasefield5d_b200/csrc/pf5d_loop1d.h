@@ -38,4 +38,11 @@ inline Loop1dShape loop1d_shape(int64_t n, int max_blocks) {
   return L;
 }
 
+// Whether the loop is the faster form for a call of nsteps steps.  A launch first
+// loads and sorts the solve, on 16 SMs; a single step of a long solve costs more
+// that way than as separate kernels.  us, kernels -> loop, FP64 and FP32c: 8192
+// points 22.5 -> 20.6 and 18.5 -> 17.3, 12000 22.6 -> 23.4 and 18.4 -> 18.4, 16384
+// 22.5 -> 28.7 and 18.4 -> 21.4; two steps of 16384 are even.
+inline bool loop1d_pays(int64_t n, int64_t nsteps) { return n <= 10240 || nsteps > 1; }
+
 }  // namespace pf5d

@@ -416,7 +416,7 @@ __global__ void __launch_bounds__(kDt32Threads) k32_dt(Rate32 P, int nparts) {
 // exactly (elastic.py:250-263); the mean and the product in FP64, s' rounded
 // once to FP32.  One block; the mean is summed in the order of
 // pf5d_cluster.cuh, as k32_loop1d sums it.
-constexpr int kElastic1dThreads32 = 1024;
+constexpr int kElastic1dThreads32 = kGroupThreads;
 constexpr int64_t kElastic1dMax32 = kLoop1dMax;
 __global__ void __launch_bounds__(kElastic1dThreads32)
     k32_elastic1d(float *s, int64_t n, double bn, double b0, const unsigned *halt) {
@@ -424,12 +424,7 @@ __global__ void __launch_bounds__(kElastic1dThreads32)
   pdl_wait();
   if (*halt) return;
   const int t = threadIdx.x, ng = (int)((n + 31) / 32);
-  for (int g = t >> 5; g < ng; g += kElastic1dThreads32 / 32) {
-    const int64_t i = 32 * (int64_t)g + (t & 31);
-    const double v = group_sum(i < n ? (double)s[i] : 0.0);
-    if ((t & 31) == 0) sums[g] = v;
-  }
-  __syncthreads();
+  block_group_sums(sums, n, [&](int64_t i) { return (double)s[i]; });
   const double mean = sum_groups(sums, ng) / (double)n;
   for (int64_t i = t; i < n; i += kElastic1dThreads32)
     s[i] = (float)(bn * ((double)s[i] - mean) + b0 * mean);
@@ -1175,7 +1170,7 @@ pf5d_status s32_reset(Stepper32 *h, const double *X, double dt, double time, voi
 
 pf5d_status s32_advance(Stepper32 *h, int64_t nsteps, void *stream) {
   cudaStream_t s = as_stream(stream);
-  if (h->use_loop1d) {
+  if (h->use_loop1d && loop1d_pays(h->npts, nsteps)) {
     const size_t sm = loop1d_smem32(h->loop.chunk);
     for (; nsteps > 0; nsteps -= kLoop1dSteps) {
       const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);

@@ -1236,8 +1236,10 @@ namespace pf5d {
 // b0 is B(0).  That is irfft(B rfft(s)) (elastic.py:250-263) exactly, for a
 // B(k) that depends on k only through its sign, as every 1D B(k) does.  One
 // block; the mean is summed in the order of pf5d_cluster.cuh, as k_loop1d
-// sums it, so a step has the same bits either way.
-constexpr int kElastic1dThreads = 1024;
+// sums it, so a step has the same bits either way.  Bound by its loads and
+// shuffles: a shuffle tree per group of 32 made a single step of 16384 points
+// 4 us longer than with 16 groups at a time (26.6 -> 22.5).
+constexpr int kElastic1dThreads = kGroupThreads;
 constexpr int64_t kElastic1dMax = kLoop1dMax;     // points of a 1D solve that use it
 __global__ void __launch_bounds__(kElastic1dThreads)
     k_elastic1d(double *s, int64_t n, double bn, double b0, const unsigned *halt) {
@@ -1245,12 +1247,7 @@ __global__ void __launch_bounds__(kElastic1dThreads)
   pdl_wait();
   if (*halt) return;
   const int t = threadIdx.x, ng = (int)((n + 31) / 32);
-  for (int g = t >> 5; g < ng; g += kElastic1dThreads / 32) {
-    const int64_t i = 32 * (int64_t)g + (t & 31);
-    const double v = group_sum(i < n ? s[i] : 0.0);
-    if ((t & 31) == 0) sums[g] = v;
-  }
-  __syncthreads();
+  block_group_sums(sums, n, [&](int64_t i) { return s[i]; });
   const double mean = sum_groups(sums, ng) / (double)n;
   for (int64_t i = t; i < n; i += kElastic1dThreads) s[i] = bn * (s[i] - mean) + b0 * mean;
 }
@@ -2175,7 +2172,7 @@ pf5d_status pf5d_stepper_advance(pf5d_stepper *h, int64_t nsteps, void *stream) 
   PF5D_REQUIRE(h && nsteps >= 0, PF5D_ERR_ARG, "bad arguments");
   if (h->s32) return s32_advance(h->s32, nsteps, stream);
   cudaStream_t s = as_stream(stream);
-  if (h->use_loop1d) {
+  if (h->use_loop1d && loop1d_pays(h->npts, nsteps)) {
     const size_t sm = loop1d_smem(h->loop.chunk);
     for (; nsteps > 0; nsteps -= kLoop1dSteps) {
       const int n = (int)std::min<int64_t>(nsteps, kLoop1dSteps);
