@@ -377,6 +377,14 @@ void launch_chem32(cudaStream_t s, const Rate32 &P) {
   launch_pdl(k32_chem<DIM, PER, K, MINB>, g, dim3(kChemNT32), 0, s, P);
 }
 
+// A save step's, for any size (the FP64 form's launch_chem_save): 24x24 156 ->
+// 148 us, 8192 points 141 -> 138.
+template <int DIM>
+void launch_chem32_save(cudaStream_t s, const Rate32 &P) {
+  if (P.npts < 65536) launch_chem32<DIM, 1, 2, 6>(s, P);
+  else launch_chem32<DIM, 4, 4, 4>(s, P);
+}
+
 template <int DIM, int R, int MINB>
 __global__ void __launch_bounds__(kFluxThreads32, MINB) k32_flux(Rate32 P, int rows) {
   __shared__ double red[kFluxThreads32 / 32];
@@ -1237,9 +1245,9 @@ pf5d_status s32_step_save_inputs(Stepper32 *h, double *X_out, double *dX_out, do
   pf5d_status st = launch_rate32(h, s);
   if (st != PF5D_OK) return st;
   switch (h->d.dim) {
-    case 1: launch_chem32<1, 4, 4, 4>(s, h->rp); break;
-    case 2: launch_chem32<2, 4, 4, 4>(s, h->rp); break;
-    default: launch_chem32<3, 4, 4, 4>(s, h->rp);
+    case 1: launch_chem32_save<1>(s, h->rp); break;
+    case 2: launch_chem32_save<2>(s, h->rp); break;
+    default: launch_chem32_save<3>(s, h->rp);
   }
   PF5D_LAUNCHED();
   k32_join<<<grid_for(h->npts, 256, 4), 256, 0, s>>>(h->hi, h->lo, h->npts, h->up, X_out);

@@ -1702,6 +1702,15 @@ void launch_chem(bool fast, cudaStream_t s, const RateParams &P) {
   else launch_pdl(k_chem<DIM, false, PER, K>, g, dim3(kChemNT), 0, s, P);
 }
 
+// A save step's, for any size: fields below 2^16 points would leave SMs idle
+// with 512 points a block.  Whole save steps, us, PER = 4 -> 1 (FP64): 24x24
+// 142 -> 134, 200x200 168 -> 160, 16384 points 132 -> 128.
+template <int DIM>
+void launch_chem_save(bool fast, cudaStream_t s, const RateParams &P) {
+  if (P.npts < 65536) launch_chem<DIM, 1, 2>(fast, s, P);
+  else launch_chem<DIM, 4, 3>(fast, s, P);
+}
+
 template <int DIM, int R, int MINB>
 void launch_flux(bool fast, dim3 g, cudaStream_t s, const RateParams &P, int rows) {
   if (fast) launch_pdl(k_flux<DIM, true, R, MINB>, g, dim3(kFluxThreads), 0, s, P, rows);
@@ -2318,9 +2327,9 @@ pf5d_status pf5d_stepper_step_save(pf5d_stepper *h, pf5d_save_diag *out, void *s
     if ((st = launch_rate(h, s)) != PF5D_OK) return st;
     // mu and M of this step at every point, then the "before" reductions
     switch (dim) {
-      case 1: launch_chem<1, 4, 3>(h->fast, s, h->rp); break;
-      case 2: launch_chem<2, 4, 3>(h->fast, s, h->rp); break;
-      default: launch_chem<3, 4, 3>(h->fast, s, h->rp);
+      case 1: launch_chem_save<1>(h->fast, s, h->rp); break;
+      case 2: launch_chem_save<2>(h->fast, s, h->rp); break;
+      default: launch_chem_save<3>(h->fast, s, h->rp);
     }
     PF5D_LAUNCHED();
     Xpre = h->X;
