@@ -360,28 +360,31 @@ __global__ void k32_mass_final(const double *partial, int nparts, double *out) {
 
 // Split rate evaluation (pf5d_split32.cuh): mu/M of a 1D/2D/3D field, then
 // the faces and the divergence of a 2D or 3D one.
-template <int DIM, int PER, int K, int MINB>
+// LONGY: as k_chem's.
+template <int DIM, int PER, int K, int MINB, bool LONGY = false>
 __global__ void __launch_bounds__(kChemNT32, MINB) k32_chem(Rate32 P) {
   using G = ChemTile32<DIM, PER>;
   __shared__ GatherSmem32<kChemNT32, PER, K> g;
   pdl_wait();
   if (P.st->halt) return;
-  chem32_body<DIM, PER, K>(P, g, blockIdx.x * G::BX, blockIdx.y * G::BY, blockIdx.z * G::BZ);
+  chem32_body<DIM, PER, K>(P, g, (LONGY ? blockIdx.y : blockIdx.x) * G::BX,
+                           (LONGY ? blockIdx.x : blockIdx.y) * G::BY, blockIdx.z * G::BZ);
 }
 
-template <int DIM, int PER, int K, int MINB>
+template <int DIM, int PER, int K, int MINB, bool LONGY = false>
 void launch_chem32(cudaStream_t s, const Rate32 &P) {
   using G = ChemTile32<DIM, PER>;
-  const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
-               (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-  launch_pdl(k32_chem<DIM, PER, K, MINB>, g, dim3(kChemNT32), 0, s, P);
+  const unsigned gx = (unsigned)((P.nx + G::BX - 1) / G::BX), gy = (unsigned)((P.ny + G::BY - 1) / G::BY);
+  const dim3 g(LONGY ? gy : gx, LONGY ? gx : gy, (unsigned)((P.nz + G::BZ - 1) / G::BZ));
+  launch_pdl(k32_chem<DIM, PER, K, MINB, LONGY>, g, dim3(kChemNT32), 0, s, P);
 }
 
 // A save step's, for any size (the FP64 form's launch_chem_save): 24x24 156 ->
 // 148 us, 8192 points 141 -> 138.
 template <int DIM>
 void launch_chem32_save(cudaStream_t s, const Rate32 &P) {
-  if (P.npts < 65536) launch_chem32<DIM, 1, 2, 6>(s, P);
+  if (DIM == 3 && P.ny > 65535 * ChemTile32<3, 4>::BY) launch_chem32<3, 4, 2, 6, true>(s, P);
+  else if (P.npts < 65536) launch_chem32<DIM, 1, 2, 6>(s, P);
   else launch_chem32<DIM, 4, 4, 4>(s, P);
 }
 

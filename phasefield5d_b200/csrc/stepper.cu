@@ -374,8 +374,11 @@ struct ChemTile {
   static constexpr int BZ = DIM == 3 ? PER : 1;
 };
 
-// FAST: double2-aligned nodes and a field on a 32-byte boundary.
-template <int DIM, bool FAST, int PER, int K>
+// FAST: double2-aligned nodes and a field on a 32-byte boundary.  LONGY: the
+// grid's x counts the tiles along axis y and its y those along x, for fields with
+// more than 65535 of the former (both in the grid's x, told apart by a division,
+// cost two registers: 1.62 -> 1.72 ms of the rate stage at 256^3 with K = 3).
+template <int DIM, bool FAST, int PER, int K, bool LONGY = false>
 __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
   constexpr int W = FAST ? 4 : 2;
   using G = ChemTile<DIM, PER>;
@@ -385,7 +388,8 @@ __global__ void __launch_bounds__(kChemNT, kChemMinB) k_chem(RateParams P) {
   if (P.st->halt) return;
   const double *X = after_wait(P.X);
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int bx = blockIdx.x * G::BX, by = blockIdx.y * G::BY, bz = blockIdx.z * G::BZ;
+  const int bx = (LONGY ? blockIdx.y : blockIdx.x) * G::BX;
+  const int by = (LONGY ? blockIdx.x : blockIdx.y) * G::BY, bz = blockIdx.z * G::BZ;
   const int64_t plane = (int64_t)P.ny * P.nx;
   // the point in slot q = j * NT + w * 32 + lane
   auto px = [&](int j, int l, int v) { return DIM == 1 ? bx + j * NT + v * 32 + l : bx + l; };
@@ -1693,13 +1697,13 @@ RateVariant make_variant() {
 }
 
 // The split form's kernels (fast: see k_chem).
-template <int DIM, int PER, int K>
+template <int DIM, int PER, int K, bool LONGY = false>
 void launch_chem(bool fast, cudaStream_t s, const RateParams &P) {
   using G = ChemTile<DIM, PER>;
-  const dim3 g((unsigned)((P.nx + G::BX - 1) / G::BX), (unsigned)((P.ny + G::BY - 1) / G::BY),
-               (unsigned)((P.nz + G::BZ - 1) / G::BZ));
-  if (fast) launch_pdl(k_chem<DIM, true, PER, K>, g, dim3(kChemNT), 0, s, P);
-  else launch_pdl(k_chem<DIM, false, PER, K>, g, dim3(kChemNT), 0, s, P);
+  const unsigned gx = (unsigned)((P.nx + G::BX - 1) / G::BX), gy = (unsigned)((P.ny + G::BY - 1) / G::BY);
+  const dim3 g(LONGY ? gy : gx, LONGY ? gx : gy, (unsigned)((P.nz + G::BZ - 1) / G::BZ));
+  if (fast) launch_pdl(k_chem<DIM, true, PER, K, LONGY>, g, dim3(kChemNT), 0, s, P);
+  else launch_pdl(k_chem<DIM, false, PER, K, LONGY>, g, dim3(kChemNT), 0, s, P);
 }
 
 // A save step's, for any size: fields below 2^16 points would leave SMs idle
@@ -1707,7 +1711,8 @@ void launch_chem(bool fast, cudaStream_t s, const RateParams &P) {
 // 142 -> 134, 200x200 168 -> 160, 16384 points 132 -> 128.
 template <int DIM>
 void launch_chem_save(bool fast, cudaStream_t s, const RateParams &P) {
-  if (P.npts < 65536) launch_chem<DIM, 1, 2>(fast, s, P);
+  if (DIM == 3 && P.ny > 65535 * ChemTile<3, 4>::BY) launch_chem<3, 4, 2, true>(fast, s, P);
+  else if (P.npts < 65536) launch_chem<DIM, 1, 2>(fast, s, P);
   else launch_chem<DIM, 4, 3>(fast, s, P);
 }
 
