@@ -807,6 +807,7 @@ pf5d_status pf5d_batch_create(const pf5d_batch_solve *solves, int32_t nsolves,
     g.ny = kv.first.first;
     g.nx = kv.first.second;
     g.count = (int)kv.second.size();
+    s_total += s_total & 1;                  // the plans want complex alignment (8 bytes)
     g.s_off = s_total;
     g.nk = (int64_t)g.ny * (g.nx / 2 + 1);
     g.k_off = k_total;
