@@ -446,7 +446,9 @@ __host__ __device__ inline double adaptive_dt(double dt, double xdotmax, double 
   if (t_cfl < most) most = t_cfl;
   // Both change limits lie past those bounds (by far more than a rounding), so
   // the clip cannot fall below them: no division (a few hundred cycles each).
-  if (xdotmax > 0.0 && most * xdotmax < (lower < upper ? lower : upper) * (1.0 - 1e-9)) return most;
+  // A NaN fails one of the comparisons.
+  const double change = most * xdotmax;
+  if (xdotmax > 0.0 && change < lower * (1.0 - 1e-9) && change < upper * (1.0 - 1e-9)) return most;
   double dt_raw;
   if (xdotmax <= 0.0) {
     dt_raw = dt;
