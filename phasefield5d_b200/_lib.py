@@ -7,6 +7,7 @@ phasefield5d_b200/csrc``).
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 
@@ -219,6 +220,21 @@ def stream_handle(stream=None):
     import torch
     s = stream if stream is not None else torch.cuda.current_stream()
     return ctypes.c_void_p(s.cuda_stream)
+
+
+@contextlib.contextmanager
+def ordered(stream):
+    """Work enqueued on ``stream`` inside comes after what the current stream
+    holds (whose freed memory a new tensor may reuse) and before what it is
+    given next (which may read the result)."""
+    import torch
+    cur = torch.cuda.current_stream()
+    if stream is None or stream.cuda_stream == cur.cuda_stream:
+        yield
+        return
+    stream.wait_stream(cur)
+    yield
+    cur.wait_stream(stream)
 
 
 def ptr(t):
