@@ -612,13 +612,42 @@ int batch_tiles_of(const pf5d_batch *h, int variant) {
   return tiles;
 }
 
+bool any_2d(const pf5d_batch *h) {
+  return std::any_of(h->solves.begin(), h->solves.end(), [](const BSolve &b) { return b.dim == 2; });
+}
+
+// The split variants' mu/M buffer (40 bytes per point), held only while one of
+// them is configured; without memory for it the batch runs the fused ones.
+bool need_mm(pf5d_batch *h) {
+  if (h->mm || !any_2d(h)) return true;
+  const int64_t npts = h->total_points;
+  if (cudaMalloc(&h->mm, npts * (2 * sizeof(float4) + sizeof(float2))) != cudaSuccess) {
+    h->mm = nullptr;
+    cudaGetLastError();
+    return false;
+  }
+  float4 *mu = reinterpret_cast<float4 *>(h->mm);
+  for (size_t i = 0; i < h->solves.size(); ++i) {
+    Rate32 &P = h->solves[i].R;
+    P.mm_mu = mu + h->pt_off[i];
+    P.mm_m = mu + npts + h->pt_off[i];
+    P.mm_f = reinterpret_cast<float2 *>(mu + 2 * npts) + h->pt_off[i];
+  }
+  return true;
+}
+
+// After the captured graphs of a split variant are gone.
+void drop_unused_mm(pf5d_batch *h) {
+  if (batch_variants()[h->variant].split) return;
+  cudaFree(h->mm);
+  h->mm = nullptr;
+}
+
 pf5d_status configure_batch(pf5d_batch *h, int variant) {
   const auto &vars = batch_variants();
   PF5D_REQUIRE(variant >= 0 && variant < (int)vars.size(), PF5D_ERR_ARG, "bad variant %d", variant);
   const BatchVariant &v = vars[variant];
-  const bool any2d = std::any_of(h->solves.begin(), h->solves.end(),
-                                 [](const BSolve &b) { return b.dim == 2; });
-  PF5D_REQUIRE(!v.split || h->mm || !any2d, PF5D_ERR_CUDA, "no memory for variant %d's mu/M buffer",
+  PF5D_REQUIRE(!v.split || need_mm(h), PF5D_ERR_CUDA, "no memory for variant %d's mu/M buffer",
                variant);
   v.set_attrs();
   PF5D_LAUNCHED();
@@ -1033,24 +1062,6 @@ pf5d_status pf5d_batch_create(const pf5d_batch_solve *solves, int32_t nsolves,
     set_error("device allocation failed");
     return fail(PF5D_ERR_CUDA);
   }
-  // The split variants' buffer, after all that the fused ones need: without it
-  // (no memory, no 2D solve) the batch runs those.
-  const bool any2d = std::any_of(h->solves.begin(), h->solves.end(),
-                                 [](const BSolve &b) { return b.dim == 2; });
-  if (any2d) {
-    if (cudaMalloc(&h->mm, npts_total * (2 * sizeof(float4) + sizeof(float2))) == cudaSuccess) {
-      float4 *mu = reinterpret_cast<float4 *>(h->mm);
-      for (int i = 0; i < nsolves; ++i) {
-        Rate32 &P = h->solves[i].R;
-        P.mm_mu = mu + h->pt_off[i];
-        P.mm_m = mu + npts_total + h->pt_off[i];
-        P.mm_f = reinterpret_cast<float2 *>(mu + 2 * npts_total) + h->pt_off[i];
-      }
-    } else {
-      h->mm = nullptr;
-      cudaGetLastError();
-    }
-  }
   pf5d_status st = configure_batch(h, 0);
   if (st != PF5D_OK) return fail(st);
   for (int i = 0; i < nsolves; ++i) {
@@ -1128,8 +1139,10 @@ pf5d_status pf5d_batch_export(pf5d_batch *h, int32_t i, float *hi_out, float *lo
 pf5d_status pf5d_batch_set_variant(pf5d_batch *h, int32_t variant) {
   PF5D_REQUIRE(h, PF5D_ERR_ARG, "null batch");
   pf5d_status st = configure_batch(h, variant);
-  if (st == PF5D_OK) drop_graphs(h);
-  return st;
+  if (st != PF5D_OK) return st;
+  drop_graphs(h);
+  drop_unused_mm(h);
+  return PF5D_OK;
 }
 
 int32_t pf5d_batch_variant_count(void) { return (int32_t)batch_variants().size(); }
@@ -1169,6 +1182,7 @@ pf5d_status pf5d_batch_autotune(pf5d_batch *h, int32_t *variant, float *best_ms,
   pf5d_status st = configure_batch(h, best);
   if (st != PF5D_OK) return st;
   drop_graphs(h);
+  drop_unused_mm(h);
   PF5D_CUDA(cudaMemcpyAsync(h->st, saved.data(), n * sizeof(StepState32), cudaMemcpyHostToDevice, s));
   PF5D_CUDA(cudaStreamSynchronize(s));
   if (variant) *variant = best;
