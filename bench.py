@@ -115,16 +115,38 @@ def measured_peak():
         return FALLBACK_HBM_GBS, "fallback"
 
 
-def committed_traffic(kernel, workload, precision):
+def committed_traffic(kernel, workload, precision, kernels):
     """DRAM bytes of one step's ``kernel`` stage (all its launches) on this
     workload from the committed ncu capture (profiles/traffic.json), or None
-    when none was taken."""
+    when none was taken of ``kernels`` (Stepper.rate_kernels): the autotuner's
+    pick may be another variant than the captured one."""
     try:
         with open(os.path.join(HERE, "profiles", "traffic.json")) as f:
             ent = json.load(f)[kernel][f"{workload}_{precision}"]
-        return float(ent["dram_bytes_per_launch"])
+        # profiler names "void pf5d::k_x<1, 2>(args)"; the dt controller is not among them
+        captured = {k.split("pf5d::", 1)[1].split("(", 1)[0] for k in ent["kernels"]}
+        ran = {k for k in kernels.split(" + ") if k not in ("k_dt_finish", "k32_dt")}
+        return float(ent["dram_bytes_per_launch"]) if ran == captured else None
     except Exception:
         return None
+
+
+def rate_roofline(kernels, workload, precision, dim, launches_per_step, rate_ms, step_ms,
+                  rate_bytes, step_bytes):
+    """Roofline entry of the kernel(s) a step spends its time in: the rate
+    stage launched alone, or, where one launch is the whole step (the 1D step
+    loop, which the stage's kernels are not part of), that step."""
+    if dim == 1 and launches_per_step == 1:
+        kernels = "k32_loop1d" if precision == "fp32c" else "k_loop1d"
+        ms, nbytes, traffic = step_ms, step_bytes, None
+    else:
+        ms, nbytes = rate_ms, rate_bytes
+        traffic = committed_traffic("rate", workload, precision, kernels)
+    peak, peak_kind = measured_peak()
+    achieved = nbytes / (ms * 1e-3) / 1e9
+    return {"bound": "hbm", "kernel": kernels, "ms_per_launch": ms, "achieved": achieved,
+            "peak": peak, "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak,
+            "algorithmic_bytes_per_launch": nbytes, "traffic": traffic}
 
 
 class ClockSampler:
@@ -272,7 +294,8 @@ def _events(torch):
 
 def _stepper_timing(prob, precision, args, flush, torch):
     """Device-resident one-step timing with L2 flushed between steps, and the
-    fused rate kernel launched alone: (ms per step, rate ms, variant)."""
+    rate stage launched alone: (ms per step, rate ms, variant, the stage's
+    kernels, launches per step)."""
     from phasefield5d_b200 import _lib
     from phasefield5d_b200.stepper import Stepper
     stream = torch.cuda.current_stream()
@@ -303,9 +326,9 @@ def _stepper_timing(prob, precision, args, flush, torch):
         rate.append((a, b))
     torch.cuda.synchronize()
     rate_ms = sum(a.elapsed_time(b) for a, b in rate) / len(rate)
-    variant, kernels = st.variant, st.rate_kernels
+    info = st.variant, st.rate_kernels, st.launches_per_step
     st.close()
-    return step_ms, rate_ms, variant, kernels
+    return (step_ms, rate_ms, *info)
 
 
 def form_workload(prob, workload, precision, args, flush, torch, accuracy_steps=0):
@@ -316,10 +339,10 @@ def form_workload(prob, workload, precision, args, flush, torch, accuracy_steps=
     ``accuracy_steps`` (FP32c only) the accuracy report against the plain
     FP64 form over that many steps."""
     from phasefield5d_b200.precision import compare_forms
-    peak, peak_kind = measured_peak()
+    peak = measured_peak()[0]
     P = prob.n_points
     fp32c = precision == "fp32c"
-    step_ms, rate_ms, variant, kernels = _stepper_timing(prob, precision, args, flush, torch)
+    step_ms, rate_ms, variant, kernels, launches = _stepper_timing(prob, precision, args, flush, torch)
     per_rate = RATE_BYTES_FP32C if fp32c else RATE_BYTES_FP64
     per_step = STEP_BYTES_FP32C if fp32c else STEP_BYTES_FP64
     if prob.lvec is None:
@@ -327,15 +350,11 @@ def form_workload(prob, workload, precision, args, flush, torch, accuracy_steps=
         per_step -= 24 if fp32c else 48
     rate_bytes = per_rate * P
     value = P / (step_ms * 1e-3)
-    achieved = rate_bytes / (rate_ms * 1e-3) / 1e9
     out = {"value": value, "unit": "grid-point steps/s", "ms_per_step": step_ms,
            "shape": list(prob.shape), "precision": precision,
            "l2": "flushed (256 MiB write) between timed steps", "rate_variant": variant,
-           "roofline": {"bound": "hbm", "kernel": kernels, "ms_per_launch": rate_ms,
-                        "achieved": achieved, "peak": peak, "peak_kind": peak_kind,
-                        "unit": "GB/s", "frac": achieved / peak,
-                        "algorithmic_bytes_per_launch": rate_bytes,
-                        "traffic": committed_traffic("rate", workload, precision)},
+           "roofline": rate_roofline(kernels, workload, precision, prob.dim, launches, rate_ms, step_ms,
+                                     rate_bytes, per_step * P),
            "step_roofline": {"bytes_per_grid_point_step": per_step,
                              "achieved_gbs": per_step * value / 1e9,
                              "frac": per_step * value / 1e9 / peak}}
@@ -559,8 +578,9 @@ def run_ours(args, rank, world, local_rank):
     torch.cuda.synchronize()
     resident_ms = w0.elapsed_time(w1) / 200
 
-    # ---- dominant kernel (fused rate) alone, L2 flushed, same stream -------
-    probe = Stepper.from_problem(prob, precision=args.precision)
+    # ---- the stages alone, L2 flushed, same stream, the variant timed above --
+    probe = Stepper.from_problem(prob, precision=args.precision, autotune=False)
+    probe.set_variant(st.variant)
     stage_ms = {}
     stages = [("rate", _lib.STAGE_RATE), ("update", _lib.STAGE_UPDATE)]
     if prob.lvec is not None:
@@ -619,11 +639,10 @@ def run_ours(args, rank, world, local_rank):
         return
 
     value = replica_throughput(P, args.steps, world, total_ms)
-    peak, peak_kind = measured_peak()
+    peak = measured_peak()[0]
     per_rate = RATE_BYTES_FP32C if fp32c else RATE_BYTES_FP64
     per_step = STEP_BYTES_FP32C if fp32c else STEP_BYTES_FP64
     rate_bytes = per_rate * P if prob.lvec is not None else (per_rate - (4 if fp32c else 8)) * P
-    achieved = rate_bytes / (stage_ms["rate"] * 1e-3) / 1e9
     cpu = None
     if not args.no_cpu_baseline and world == 1:        # the CPU baseline: N = 1 only
         cpu = cpu_baseline(prob, args, WORKLOADS[args.workload][0])
@@ -638,11 +657,9 @@ def run_ours(args, rank, world, local_rank):
                    "table_nodes_per_axis": int(prob.grid.shape[0]), "omega_seed": prob.omega_seed,
                    "l2": "flushed (256 MiB write) between timed steps",
                    "parallelism": f"replicas x{world}" if world > 1 else "single solve"},
-        "roofline": {"bound": "hbm", "kernel": rate_kernels,
-                     "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
-                     "frac": achieved / peak, "traffic": committed_traffic("rate", args.workload, args.precision),
-                     "algorithmic_bytes_per_launch": rate_bytes,
-                     "ms_per_launch": stage_ms["rate"]},
+        "roofline": rate_roofline(rate_kernels, args.workload, args.precision, prob.dim,
+                                  launches_per_step, stage_ms["rate"], total_ms / args.steps,
+                                  rate_bytes, per_step * P),
         "step_roofline": {"bytes_per_grid_point_step": per_step,
                           "achieved_gbs": per_step * value / world / 1e9,
                           "frac": per_step * value / world / 1e9 / peak},

@@ -820,7 +820,7 @@ Variant32 make_split_variant32() {
     launch_pdl(k32_flux<3, R, MINB>, g, dim3(kFluxThreads32), 0, s, P, zc);
   };
   v.kernels = [](int dim) {
-    return kname("k32_chem", {dim, PER, K, KMINB}) + " + " +
+    return kname("k32_chem", {dim, PER, K, KMINB, 0}) + " + " +
            kname("k32_flux", {dim, dim == 2 ? 1 : R, MINB});
   };
   return v;

@@ -1745,7 +1745,7 @@ RateVariant make_split_variant() {
     launch_flux<3, R, MINB>(fast, g, s, P, zc);
   };
   v.kernels = [](bool fast, int dim) {
-    return kname("k_chem", {dim, fast, PER, K}) + " + " +
+    return kname("k_chem", {dim, fast, PER, K, 0}) + " + " +
            kname("k_flux", {dim, fast, dim == 2 ? 1 : R, MINB});
   };
   return v;
