@@ -7,7 +7,6 @@ phasefield5d_b200/csrc``).
 """
 from __future__ import annotations
 
-import contextlib
 import ctypes
 import os
 
@@ -222,19 +221,24 @@ def stream_handle(stream=None):
     return ctypes.c_void_p(s.cuda_stream)
 
 
-@contextlib.contextmanager
-def ordered(stream):
-    """Work enqueued on ``stream`` inside comes after what the current stream
-    holds (whose freed memory a new tensor may reuse) and before what it is
-    given next (which may read the result)."""
-    import torch
-    cur = torch.cuda.current_stream()
-    if stream is None or stream.cuda_stream == cur.cuda_stream:
-        yield
-        return
-    stream.wait_stream(cur)
-    yield
-    cur.wait_stream(stream)
+def wait_for_caller(stream):
+    """Work enqueued on ``stream`` from here on comes after what the current
+    stream holds (whose freed memory a new tensor may reuse)."""
+    if stream is not None:
+        import torch
+        cur = torch.cuda.current_stream()
+        if stream.cuda_stream != cur.cuda_stream:
+            stream.wait_stream(cur)
+
+
+def caller_waits(stream):
+    """What the current stream is given from here on comes after the work
+    enqueued on ``stream`` so far."""
+    if stream is not None:
+        import torch
+        cur = torch.cuda.current_stream()
+        if stream.cuda_stream != cur.cuda_stream:
+            cur.wait_stream(stream)
 
 
 def ptr(t):

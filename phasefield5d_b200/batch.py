@@ -142,8 +142,9 @@ class BatchStepper:
     def field(self, i):
         p = self.problems[i]
         out = self._torch.empty((*p.shape, 4), dtype=self._torch.float64, device="cuda")
-        with _lib.ordered(self.stream):
-            _lib.check(self.L.pf5d_batch_field(self.h, int(i), _lib.ptr(out), self._s()), "field")
+        _lib.wait_for_caller(self.stream)
+        _lib.check(self.L.pf5d_batch_field(self.h, int(i), _lib.ptr(out), self._s()), "field")
+        _lib.caller_waits(self.stream)
         return out
 
     def export(self, i):
@@ -151,9 +152,10 @@ class BatchStepper:
         p = self.problems[i]
         hi = self._torch.empty((p.n_points, 4), dtype=self._torch.float32, device="cuda")
         lo = self._torch.empty_like(hi)
-        with _lib.ordered(self.stream):
-            _lib.check(self.L.pf5d_batch_export(self.h, int(i), _lib.ptr(hi), _lib.ptr(lo), self._s()),
-                       "export")
+        _lib.wait_for_caller(self.stream)
+        _lib.check(self.L.pf5d_batch_export(self.h, int(i), _lib.ptr(hi), _lib.ptr(lo), self._s()),
+                   "export")
+        _lib.caller_waits(self.stream)
         st = self.states()[i]
         return hi, lo, st["dt"], st["time"], st["step"]
 

@@ -173,8 +173,7 @@ class Stepper:
     def rate(self):
         """dX/dt of the last step as a (*shape, 4) CUDA tensor (a view)."""
         ptr = self.L.pf5d_stepper_rate(self.h)
-        with _lib.ordered(self.stream):
-            pass                          # what reads it next waits for the steps so far
+        _lib.caller_waits(self.stream)
         return _tensor_from_ptr(ptr, self.n_points * 4, self._torch).view(*self.shape, 4)
 
     def autotune(self):
@@ -223,8 +222,9 @@ class Stepper:
     def field(self):
         """Current field X as a (*shape, 4) float64 CUDA tensor (a copy)."""
         out = self._torch.empty((*self.shape, 4), dtype=self._torch.float64, device="cuda")
-        with _lib.ordered(self.stream):
-            _lib.check(self.L.pf5d_stepper_field(self.h, _lib.ptr(out), self._s()), "field")
+        _lib.wait_for_caller(self.stream)
+        _lib.check(self.L.pf5d_stepper_field(self.h, _lib.ptr(out), self._s()), "field")
+        _lib.caller_waits(self.stream)
         return out
 
     def mass(self):
