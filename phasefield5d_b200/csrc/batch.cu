@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(kUpdThreads)
   for (int cidx = chunk_begin + blockIdx.x; cidx < chunk_end; cidx += gridDim.x) {
     const BSolve &B = solves[find_solve_chunk(solves, nsolves, cidx)];
     StepState32 *st = B.R.st;
-    if (st->halt) continue;
+    if (st->hold) continue;
     const int local = cidx - B.chunk0;
     const float dtf = (float)st->dt;
     const bool check = B.oob_interval > 0 && (st->step % B.oob_interval) == 0;
@@ -444,7 +444,7 @@ __global__ void kb_dt(const BSolve *__restrict__ solves, int nsolves, const doub
   const int i = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (i >= nsolves) return;
   const BSolve &B = solves[i];
-  if (B.R.st->halt) return;
+  if (halted_before_dt(B.R.st)) return;
   dt_from_slots32(B.R, tile_max + B.tile0, B.ntiles);
 }
 

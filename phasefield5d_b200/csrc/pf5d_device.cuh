@@ -147,13 +147,28 @@ struct NearestNode {
 // table without rows.
 constexpr unsigned kNNErrorFlags = PF5D_FLAG_NN_FAR | PF5D_FLAG_NN_TRUNCATED | PF5D_FLAG_NN_NONFINITE;
 
-// Record a rate kernel's flags in its step state (flags, halt); the
-// fallback's error flags halt the loop before the step's update.
+// How a step loop ends.  No kernel tests at its entry what it may set itself: a
+// block of it could start while another one sets it, some of its warps would
+// leave, and the others would go on with shared memory that nobody prepared (the
+// cell order's counters among it), or a field would be updated in part.  So
+//   * a rate kernel records its flags and sets nothing else;
+//   * the dt kernel after it, for one solve, turns the fallback's errors into
+//     `halt` and any halt into `hold`, and leaves dt, time and step;
+//   * the update tests `hold`, and sets `halt` where it finds the field out of
+//     bounds, which the next step's kernels and dt kernel see.
 template <typename St>
 __device__ __forceinline__ void raise_rate_flags(St *st, unsigned f) {
-  if (!f) return;
-  atomicOr(&st->flags, f);
-  if (f & kNNErrorFlags) atomicExch(&st->halt, 1u);
+  if (f) atomicOr(&st->flags, f);
+}
+
+// In the dt kernel: whether the loop is halted (then every thread of the solve
+// may write the same words).
+template <typename St>
+__device__ __forceinline__ bool halted_before_dt(St *st) {
+  if (!(st->flags & kNNErrorFlags) && !st->halt) return false;
+  st->halt = 1u;
+  st->hold = 1u;
+  return true;
 }
 
 // The search needs only the node coordinates and a presence probe, so it

@@ -20,6 +20,7 @@ struct StepState32 {
   double xdotmax;
   unsigned flags;
   unsigned halt;
+  unsigned hold, pad;
   long long step;
 };
 

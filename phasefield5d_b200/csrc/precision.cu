@@ -255,7 +255,7 @@ __device__ __forceinline__ void update_point32(const Update32 &U, float dtf, con
 __global__ void k32_update(Update32 U) {
   pdl_wait();
   StepState32 *st = U.st;
-  if (st->halt) return;
+  if (st->hold) return;
   const float dtf = (float)st->dt;
   const bool check = U.oob_interval > 0 && (st->step % U.oob_interval) == 0;
   unsigned f = 0;
@@ -404,7 +404,7 @@ __global__ void __launch_bounds__(kDt32Threads) k32_dt(Rate32 P, int nparts) {
   __shared__ double red[kDt32Threads / 32];
   pdl_wait();
   StepState32 *st = P.st;
-  if (st->halt) return;
+  if (halted_before_dt(st)) return;
   double m = 0.0;
   for (int i = threadIdx.x; i < nparts; i += kDt32Threads) m = fmax(m, P.partial[i]);
 #pragma unroll

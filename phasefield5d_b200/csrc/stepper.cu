@@ -51,7 +51,8 @@ struct StepState {
   double time;
   double xdotmax;      // max |dX/dt| of the last rate evaluation
   unsigned flags;      // PF5D_FLAG_* accumulated
-  unsigned halt;       // non-zero: every step kernel returns at entry
+  unsigned halt;       // non-zero: a step's kernels up to the dt kernel return at entry
+  unsigned hold, pad;  // non-zero: so does the update (halted_before_dt)
   long long step;      // completed steps
 };
 
@@ -494,7 +495,7 @@ __global__ void __launch_bounds__(kDtThreads) k_dt_finish(RateParams P, int npar
   __shared__ double red[kDtThreads / 32];
   pdl_wait();
   StepState *st = P.st;
-  if (st->halt) return;
+  if (halted_before_dt(st)) return;
   double m = 0.0;
   for (int i = threadIdx.x; i < nparts; i += kDtThreads) m = fmax(m, P.partial[i]);
 #pragma unroll
@@ -1150,7 +1151,7 @@ __device__ __forceinline__ void raise_flags(StepState *st, unsigned f) {
 __global__ void k_update_step(UpdateParams U) {
   pdl_wait();
   StepState *st = U.st;
-  if (st->halt) return;
+  if (st->hold) return;
   const double dt = st->dt;
   const bool check = U.oob_interval > 0 && (st->step % U.oob_interval) == 0;
   unsigned f = 0;
