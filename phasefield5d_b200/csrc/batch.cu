@@ -1138,6 +1138,8 @@ pf5d_status pf5d_batch_export(pf5d_batch *h, int32_t i, float *hi_out, float *lo
 
 pf5d_status pf5d_batch_set_variant(pf5d_batch *h, int32_t variant) {
   PF5D_REQUIRE(h, PF5D_ERR_ARG, "null batch");
+  // steps in flight, on whichever stream, read the descriptors and the buffer
+  PF5D_CUDA(cudaDeviceSynchronize());
   pf5d_status st = configure_batch(h, variant);
   if (st != PF5D_OK) return st;
   drop_graphs(h);
