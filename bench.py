@@ -92,6 +92,9 @@ def parse():
     ap.add_argument("--serve-requests", type=int, default=12)
     ap.add_argument("--serve-rates", default="1,10,50", help="Poisson arrival rates, req/s")
     ap.add_argument("--serve-steps", type=int, default=2000)
+    ap.add_argument("--rate-variant", type=int, default=None,
+                    help="rate-kernel variant of the timed solve (default: the autotuner's pick; "
+                         "its timings, and with them the pick, are off under a profiler)")
     ap.add_argument("--ncu-range", action="store_true",
                     help="after warm-up, run one extra step (untimed) between cudaProfilerStart/"
                          "Stop, for ncu --profile-from-start off")
@@ -542,7 +545,9 @@ def run_ours(args, rank, world, local_rank):
 
     fp32c = args.precision == "fp32c"
     # ---- device-resident steps, L2 flushed between timed steps -------------
-    st = Stepper.from_problem(prob, precision=args.precision)
+    st = Stepper.from_problem(prob, precision=args.precision, autotune=args.rate_variant is None)
+    if args.rate_variant is not None:
+        st.set_variant(args.rate_variant)
     st.advance(1)                       # captures the one-step graph
     for _ in range(args.warmup):
         flush.zero_()

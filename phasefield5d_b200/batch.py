@@ -173,6 +173,7 @@ class BatchStepper:
 
     def set_variant(self, v):
         _lib.check(self.L.pf5d_batch_set_variant(self.h, int(v)), "set_variant")
+        self.variant, self.tuned_ms = int(v), None
 
     def close(self):
         if getattr(self, "h", None):

@@ -218,6 +218,7 @@ class Stepper:
 
     def set_variant(self, variant):
         _lib.check(self.L.pf5d_stepper_set_variant(self.h, int(variant)), "set_variant")
+        self.variant, self.tuned_ms = int(variant), None
 
     def field(self):
         """Current field X as a (*shape, 4) float64 CUDA tensor (a copy)."""
