@@ -357,12 +357,14 @@ __device__ __forceinline__ void mu_plane64(const RateParams &P, const double *Xm
 // and a thread's PER are consecutive along y (2D) or z (3D), so it loads each
 // point of that axis once.
 //
-// Bound by the L1 data path (67% of its wavefronts' rate at 128x256x256, FP64
-// pipe 38%).  One point per thread (1.21 ms at 256^3, on-node composition)
-// moved every node into registers once per point; with K = 3 points of a cell
-// per load it is 0.99 ms.  K = 4 needs 168 registers, and the 12 warps per SM
-// that leaves lose more (1.18) than the fewer loads give; K = 2 with the same
-// 16 warps is 1.01.  PER = 4 keeps a cell's run longer than K in fields that
+// Bound by the L1 data path and the latency behind it (at 128^3 64% of its
+// wavefronts' rate, FP64 pipe 36%, DRAM 16%).  One point per thread (1.21 ms at
+// 256^3, on-node composition) moved every node into registers once per point;
+// with K = 2 points of a cell per load it is 1.03 ms.  K = 3 loads less, but
+// spills 180 bytes per thread at the same 16 warps per SM: even at 128^3 (144
+// against 146 us), behind at 256^3 and 512^2 (rate stage 31.0 against 30.2), so
+// both are variants.  K = 4 needs 168 registers, and the 12 warps per SM that
+// leaves lose more (1.18) than the fewer loads give.  PER = 4 keeps a cell's run longer than K in fields that
 // spread over many cells (rate stage with two phases: 1.97 ms, PER = 2 2.11);
 // below about 400^2 points its blocks leave SMs idle, and PER = 2 takes over:
 // 389x250 rate stage 22.0 -> 17.6 us (27.4 -> 22.1 with two phases).
@@ -874,11 +876,13 @@ __global__ void __launch_bounds__(TX * TY, MINB) k_rate_march3d(RateParams P, in
 // Divergence in the reference's order: axis 0, then 1, then 2
 // (fluxes.py:349-395).
 //
-// Three-dimensional fields: bound by FP64 issue (52% of the pipe) and by the
-// latency of the loads that 12 warps per SM leave (DRAM 45%); the next plane
-// but one is prefetched into L2.  256^3: 0.76 ms as a 32x4 tile with a shared
-// cp.async ring and five faces per point, 0.63 here.  R = 2 rows per thread
-// take 3.5 faces per point instead of 4 but 204 registers (8 warps): 0.67.
+// Three-dimensional fields: bound by FP64 issue (at 128^3 54% of the pipe) and
+// by the latency of the loads that 12 warps per SM leave (DRAM 38%); the next
+// plane but one is prefetched into L2.  256^3: 0.76 ms as a 32x4 tile with a
+// shared cp.async ring and five faces per point, 0.60 here.  R = 2 rows per
+// thread take 3.5 faces per point instead of 4 but 210 registers (8 warps, 47%
+// of the pipe): 93 against 88 us at 128^3, but the fastest stage at 256^3 (with
+// K = 2 1.59 ms against 1.62 with R = 1 and K = 3).
 // Two-dimensional: 512^2 rate stage 39.1 us as one fused tile kernel (31%
 // halo recomputation, four faces per point), 29.8 split; 4 rows per warp keep
 // 16 warps per SM there, 2 rows are better below about 400^2, where they are
@@ -1288,7 +1292,9 @@ __global__ void __launch_bounds__(kElastic1dThreads)
 // kernels -> here: 203 points 14.4 -> 3.3 us, 1280 14.7 -> 3.6, 4112 16.1 ->
 // 5.7, 16384 18.0 -> 14.1 -- so every solve with the closed-form elastic term
 // (or none) takes it.  With cluster barriers in place of the messages a step
-// of 1280 points was 6.0 us, without the cell order 5.0.
+// of 1280 points was 6.0 us, without the cell order 5.0.  That a block leaves
+// the loop as a whole, and the blocks agree before they store, costs 0.1 us of
+// these (16384 points 0.4).
 struct Loop1dSmem {
   ulonglong2 sums[kLoop1dGroups];        // B: misfit sum (bits) and flags of every group
   ulonglong2 max[kLoop1dBlocks * (kLoop1dThreads / 32)];   // A: max |dX/dt| (bits), flags
